@@ -8,17 +8,18 @@
 //
 // A block takes 32 columns of one head of one request, and what bounds it is the chain from chunk to chunk, so its warps share a
 // chunk's work.  Eight computing warps hold S^T in registers, a warp 16 columns and a quarter of the rows, as accumulators of
-// mma.m16n8k8: the layout of an accumulator is that of an A operand with the contraction index permuted (column 2t for index t,
-// 2t + 1 for t + 4), so S never passes through memory, and B operands are read in the permuted order.  The four warps of 16 columns
-// add their shares of S^T q through shared memory, once a chunk; two of them finish 8 tokens each.  Eight loader warps prepare the
-// next chunk meanwhile in the other of two buffers, its rows and D put (q . k), and one warp the decays and the normaliser.
-// (B200, 16 heads of 128 x 128, a portion of 1,501 beside 24 single tokens: 143 us with exponential gates, 736 by the walk;
-// vob_matrix_scan_by_chunks has more of both.)
+// mma.m16n8k16: two neighbouring accumulators lie like an A operand, so S never passes through memory.  The four warps of 16
+// columns add their shares of S^T q through shared memory, once a chunk; two of them finish 8 tokens each.  Eight loader warps
+// prepare the next chunk meanwhile in the other of two buffers, its rows and D put (q . k), and one warp the decays and the normaliser.
 //
-// Everything is held in float.  A product runs as three of 11-bit parts (x = hi + lo, both exact in the tensor cores' 32-bit
-// format; hi hi + lo hi + hi lo), as two where an operand is a bfloat16 number: some 2^-22 a term.  The tensor cores' own sums cut
-// off instead of rounding, so a chunk's share of S is summed from zero and added to S by one rounded multiply-add: over a long text
-// nothing drifts.
+// Bits.  Everything is held in float, and no result is further from the recurrence in 64 bits than the walk's:
+//   * a float enters a product as three bfloat16 slices that add up to it, x = hi + mid + lo.  A product of two slices has 16
+//     bits, so the tensor cores' sums, which cut off instead of rounding, are exact for hi hi while the terms lie within some
+//     8 bits of each other; the other pairs of slices (down to 2^-25) are summed apart, where what is cut off is 2^-8 of that;
+//   * what goes into the state, and the scores, are cut on a grid (hi: multiples of 2^-7 of the largest that is summed): numbers
+//     far below that one then leave nothing to cut off;
+//   * products of decays carry their rounding errors along (hi + lo), and b_15 multiplies S as such a pair: over a long text
+//     nothing drifts.
 #pragma once
 #include "common.cuh"
 
@@ -26,61 +27,87 @@ namespace vob {
 
 constexpr int CS_C = 16, CS_COLS = 32;                 // tokens of a chunk, columns of a block
 constexpr int CS_COMPUTE = 256, CS_LOADERS = 256, CS_DECAYS = 32, CS_THREADS = CS_COMPUTE + CS_LOADERS + CS_DECAYS;
-constexpr int CS_VS = CS_COLS + 8, CS_TS = CS_C + 4;   // rows in shared memory: a fragment's reads fall into different banks
+constexpr int CS_VS = CS_COLS + 4, CS_TS = CS_C + 4;   // rows in shared memory: a fragment's reads fall into different banks
 // named barriers: a buffer is full (everyone), a buffer is empty (computing warps and loaders; computing warps and decays), a chunk's
 // rows and decays are there (loaders, decays), the shares of 16 columns are there (their computing warps)
 enum { CS_FULL = 1, CS_EMPTY = 3, CS_ROWS = 5, CS_SHARES = 6, CS_EMPTY_DECAYS = 8 };
 
-// Offsets (floats) in a buffer, for heads of up to KP rows.  EXACT: q and k are bfloat16 numbers, else each lies as (hi, lo).
+// Offsets (32-bit words) in a buffer, for heads of up to KP rows.  EXACT: q and k are bfloat16 numbers, one slice, else three.
 template <int KP, bool EXACT> struct ChunkLayout {
-  static constexpr int WORDS = EXACT ? 1 : 2, KS = WORDS * (KP + 8);
-  static constexpr int Q = 0, K = Q + CS_C * KS, V = K + CS_C * KS;
+  static constexpr int SLICES = EXACT ? 1 : 3, KS = KP / 2 + 4, SLICE = CS_C * KS;      // a slice: [token][row], two rows a word
+  static constexpr int Q = 0, K = Q + SLICES * SLICE, V = K + SLICES * SLICE;            // v: floats
   static constexpr int A = V + CS_C * CS_VS;           // scores D_ij put_j (q_i . k_j), zeros above the diagonal: two halves of the sum over the rows
-  static constexpr int D = A + 2 * CS_C * CS_TS;
-  static constexpr int PRE = D + CS_C;                 // b_i (times the read-out's scale): column 16 of the rows of D
-  static constexpr int END = D + CS_C * CS_TS;         // D_15,j put_j
-  static constexpr int PUT = END + CS_C;
-  static constexpr int ALL = PUT + CS_C;               // b_15
+  static constexpr int D = A + 2 * CS_C * CS_TS;       // D_ij put_j, times the read-out's scale
+  static constexpr int PRE = D + CS_C;                 // b_i, times the read-out's scale: column 16 of the rows of D
+  static constexpr int END = D + CS_C * CS_TS;         // D_15,j put_j, behind them what is missing from each
+  static constexpr int ALL = END + 2 * CS_C;           // b_15, and what is missing from it
   static constexpr int FLOATS = ALL + 4;
   // behind the two buffers: the shares of S^T q, by the chunk's parity, 16 columns, 8 tokens and quarter of the rows
   static constexpr int SHARES = 2 * FLOATS, SHARE = 4 * 32;
   static constexpr int TOTAL = SHARES + 2 * 2 * 2 * 4 * SHARE;
+  static_assert(KS % 4 == 0 && FLOATS % 4 == 0 && END % 4 == 0 && D % 4 == 0, "rows and vectors start on 16 bytes");
 };
 
-// x = hi + lo, both with at most 11 significant bits (hi rounded to nearest; lo loses at most the last bit of x).
-__device__ __forceinline__ void split_tf32(float x, float& hi, float& lo) {
-  hi = __uint_as_float((__float_as_uint(x) + 0x1000u) & 0xffffe000u);
-  lo = __uint_as_float(__float_as_uint(x - hi) & 0xffffe000u);
+__device__ __forceinline__ void cs_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
+  asm("mma.sync.aligned.m16n8k16.row.col.f32.bf16.bf16.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
+      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3]) : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
-__device__ __forceinline__ void mma_tf32(float (&d)[4], const float (&a)[4], float b0, float b1) {
-  asm("mma.sync.aligned.m16n8k8.row.col.f32.tf32.tf32.f32 {%0,%1,%2,%3}, {%4,%5,%6,%7}, {%8,%9}, {%0,%1,%2,%3};\n"
-      : "+f"(d[0]), "+f"(d[1]), "+f"(d[2]), "+f"(d[3])
-      : "r"(__float_as_uint(a[0])), "r"(__float_as_uint(a[1])), "r"(__float_as_uint(a[2])), "r"(__float_as_uint(a[3])),
-        "r"(__float_as_uint(b0)), "r"(__float_as_uint(b1)));
+// Four 8 x 8 matrices of 16-bit elements; lane l names row l % 8 of matrix l / 8.
+__device__ __forceinline__ void cs_ldmatrix(uint32_t (&r)[4], const float* row) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(row)));
 }
-// An accumulator as an A operand: parts of (row g, 2t), (row g + 8, 2t), (row g, 2t + 1), (row g + 8, 2t + 1).
-__device__ __forceinline__ void split_operand(const float (&c)[4], float (&hi)[4], float (&lo)[4]) {
-  split_tf32(c[0], hi[0], lo[0]);
-  split_tf32(c[2], hi[1], lo[1]);
-  split_tf32(c[1], hi[2], lo[2]);
-  split_tf32(c[3], hi[3], lo[3]);
+__device__ __forceinline__ void cs_ldmatrix_trans(uint32_t (&r)[4], const float* row) {
+  asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(row)));
 }
-// d += A B, its small parts into x; an exact operand has no low part.
-template <bool A_EXACT, bool B_EXACT>
-__device__ __forceinline__ void mma_parts(float (&d)[4], float (&x)[4], const float (&hi)[4], const float (&lo)[4], float h0, float h1,
-                                          float l0, float l1) {
-  mma_tf32(d, hi, h0, h1);
-  if (!A_EXACT) mma_tf32(x, lo, h0, h1);
-  if (!B_EXACT) mma_tf32(x, hi, l0, l1);
+// Two bfloat16 numbers in a word, the first in the low half.
+__device__ __forceinline__ uint32_t cs_pack(float x, float y) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(x, y);
+  return *reinterpret_cast<const uint32_t*>(&v);
 }
-// The parts of elements d and d + 1 of a row, (h0, l0, h1, l1), and of element d, (h, l).
-template <bool EXACT> __device__ __forceinline__ float4 parts_of_two(const float* row, int d) {
-  if (!EXACT) return *reinterpret_cast<const float4*>(row + 2 * d);
-  const float2 x = *reinterpret_cast<const float2*>(row + d);
-  return make_float4(x.x, 0.f, x.y, 0.f);
+__device__ __forceinline__ float2 cs_unpack(uint32_t w) { return make_float2(__uint_as_float(w << 16), __uint_as_float(w & 0xffff0000u)); }
+// (x, y) = hi + mid + lo, exactly: 24 bits are 8 + 8 + 8.
+__device__ __forceinline__ void cs_slices(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  hi = cs_pack(x, y);
+  const float2 h = cs_unpack(hi);
+  x -= h.x;
+  y -= h.y;
+  mid = cs_pack(x, y);
+  const float2 m = cs_unpack(mid);
+  lo = cs_pack(x - m.x, y - m.y);
 }
-template <bool EXACT> __device__ __forceinline__ float2 parts_of_one(const float* row, int d) {
-  return EXACT ? make_float2(row[d], 0.f) : *reinterpret_cast<const float2*>(row + 2 * d);
+// (x + rx, y + ry) as slices of which hi lies on the grid of 2^-7 of the power of two in `most` (the largest |x| of those that are summed).
+__device__ __forceinline__ void cs_grid_slices(float x, float y, float rx, float ry, float most, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const float shift = __uint_as_float(__float_as_uint(most) & 0x7f800000u) * 98304.f;       // 1.5 * 2^23 steps of 2^-7
+  const float hx = (x + shift) - shift, hy = (y + shift) - shift;
+  x = (x - hx) + rx;
+  y = (y - hy) + ry;
+  hi = cs_pack(hx, hy);
+  mid = cs_pack(x, y);
+  const float2 m = cs_unpack(mid);
+  lo = cs_pack(x - m.x, y - m.y);
+}
+__device__ __forceinline__ float cs_most_of_four(float x) {        // over the lanes of a row of a fragment
+  x = fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 1));
+  return fmaxf(x, __shfl_xor_sync(0xffffffffu, x, 2));
+}
+// Slices of A times slices of B: hi hi into d, all others that matter into x.  A_EXACT, B_EXACT: that operand is its hi slice.  GRID: one
+// of the two lies on a grid, its mid slice is up to 2^-8 of its largest, and mid lo counts too.
+template <bool A_EXACT, bool B_EXACT, bool GRID>
+__device__ __forceinline__ void cs_products(float (&d)[4], float (&x)[4], const uint32_t (&a)[3][4], const uint32_t (&b)[3][2]) {
+  cs_mma(d, a[0], b[0][0], b[0][1]);
+  if (!A_EXACT) cs_mma(x, a[1], b[0][0], b[0][1]);
+  if (!B_EXACT) cs_mma(x, a[0], b[1][0], b[1][1]);
+  if (!A_EXACT) cs_mma(x, a[2], b[0][0], b[0][1]);
+  if (!B_EXACT) cs_mma(x, a[0], b[2][0], b[2][1]);
+  if (!A_EXACT && !B_EXACT) {
+    cs_mma(x, a[1], b[1][0], b[1][1]);
+    if (GRID) {
+      cs_mma(x, a[2], b[1][0], b[1][1]);
+      cs_mma(x, a[1], b[2][0], b[2][1]);
+    }
+  }
 }
 
 // A SOURCE gives, for token t of the step and head h: q_raw, k_raw (row d) and v_raw (column c) as stored, act (what becomes of
@@ -92,7 +119,7 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
                   float* raw, int heads, int dk, int dv, long num_slots, int* err) {
   constexpr bool EXACT = SRC::EXACT;
   using LO = ChunkLayout<KP, EXACT>;
-  constexpr int KS = LO::KS, HK = KP / 4, NT = HK / 8, NV = KP / 32;
+  constexpr int KS = LO::KS, SLICES = LO::SLICES, HK = KP / 4, NT = HK / 8, NV = KP / 32;
   static_assert(EXACT || !SRC::NORMALISER, "the normaliser's walk reads rows that lie as they are");
   extern __shared__ float4 sm4[];
   float* sm = reinterpret_cast<float*>(sm4);
@@ -177,20 +204,27 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
       float* bf = sm + (c & 1) * LO::FLOATS;
       const typename SRC::GateRaw next = src.gate_raw((size_t)min(t0 + (c + 1) * CS_C + lane, t1 - 1), h);
       if (c >= 2) named_sync(CS_EMPTY_DECAYS + (c & 1), CS_COMPUTE + CS_DECAYS);
-      // lane j < 16: D_ij down its column; lane 16: the products b_i
-      float run = 1.f;
-      const float factor = lane == CS_C ? scale : 1.f;
+      // lane j < 16: D_ij down its column; lane 16: the products b_i; both with their rounding errors beside them
+      float run = 1.f, rest = 0.f;
+      const float factor = lane == CS_C ? scale : gt.y * scale;
 #pragma unroll
       for (int i = 0; i < CS_C; ++i) {
-        const float keep = __shfl_sync(0xffffffffu, gt.x, i);
-        run *= lane < i || lane == CS_C ? keep : 1.f;
-        if (lane <= CS_C) bf[LO::D + i * CS_TS + lane] = run * factor;
+        const float keep = __shfl_sync(0xffffffffu, gt.x, i), mine_too = lane < i || lane == CS_C ? keep : 1.f;
+        const float next_run = run * mine_too;
+        rest = fmaf(rest, mine_too, fmaf(run, mine_too, -next_run));
+        run = next_run;
+        if (lane <= CS_C) bf[LO::D + i * CS_TS + lane] = fmaf(run, factor, rest * factor);
       }
       if (lane < CS_C) {
-        bf[LO::END + lane] = run * gt.y;
-        bf[LO::PUT + lane] = gt.y;
+        const float end = run * gt.y;
+        bf[LO::END + lane] = end;
+        bf[LO::END + CS_C + lane] = fmaf(rest, gt.y, fmaf(run, gt.y, -end));
       }
-      if (lane == CS_C) bf[LO::ALL] = run;
+      if (lane == CS_C) {
+        const float all = run + rest;
+        bf[LO::ALL] = all;
+        bf[LO::ALL + 1] = rest - (all - run);
+      }
       __threadfence_block();
       named_sync(CS_ROWS, CS_LOADERS + CS_DECAYS);      // (waited for, not only told: two chunks' arrivals must not meet)
       named_arrive(CS_FULL + (c & 1), CS_THREADS);
@@ -204,8 +238,8 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
             float q[NE], k[NE];
 #pragma unroll
             for (int e = 0; e < NE; e += 2) {
-              const float2 q2 = *reinterpret_cast<const float2*>(bf + LO::Q + i * KS + 64 * (e / 2) + 2 * lane);
-              const float2 k2 = *reinterpret_cast<const float2*>(bf + LO::K + i * KS + 64 * (e / 2) + 2 * lane);
+              const float2 q2 = cs_unpack(__float_as_uint(bf[LO::Q + i * KS + 32 * (e / 2) + lane]));
+              const float2 k2 = cs_unpack(__float_as_uint(bf[LO::K + i * KS + 32 * (e / 2) + lane]));
               q[e] = q2.x; q[e + 1] = q2.y; k[e] = k2.x; k[e + 1] = k2.y;
             }
             dots[i] = 0.f;
@@ -254,7 +288,7 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
         const size_t at = (size_t)(base + min(lw + STEP * tt, n - 1));
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
-          const int d = min(lane + 32 * j, dk - 1);
+          const int d = min(2 * lane + 64 * (j >> 1) + (j & 1), dk - 1);      // neighbouring rows share a word
           qv[tt][j] = src.q_raw(at, h, d);
           kv[tt][j] = src.k_raw(at, h, d);
         }
@@ -270,21 +304,21 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
 #pragma unroll
       for (int tt = 0; tt < TPW; ++tt) {
         const int i = lw + STEP * tt;
-        float* qd = bf + LO::Q + i * KS + LO::WORDS * lane;
-        float* kd = bf + LO::K + i * KS + LO::WORDS * lane;
+        uint32_t* qd = reinterpret_cast<uint32_t*>(bf) + LO::Q + i * KS + lane;
+        uint32_t* kd = reinterpret_cast<uint32_t*>(bf) + LO::K + i * KS + lane;
 #pragma unroll
-        for (int j = 0; j < NV; ++j) {
-          const bool live = i < n && lane + 32 * j < dk;
-          const float q = live ? src.act(to_f(qv[tt][j])) : 0.f, k = live ? src.act(to_f(kv[tt][j])) : 0.f;
-          if (EXACT) {
-            qd[32 * j] = q;
-            kd[32 * j] = k;
-          } else {
-            float2 x, y;
-            split_tf32(q, x.x, x.y);
-            split_tf32(k, y.x, y.y);
-            *reinterpret_cast<float2*>(qd + 64 * j) = x;
-            *reinterpret_cast<float2*>(kd + 64 * j) = y;
+        for (int j = 0; j < NV; j += 2) {
+          const int d = 2 * lane + 32 * j;
+          float x[4] = {to_f(qv[tt][j]), to_f(qv[tt][j + 1]), to_f(kv[tt][j]), to_f(kv[tt][j + 1])};
+#pragma unroll
+          for (int e = 0; e < 4; ++e) x[e] = i < n && d + (e & 1) < dk ? src.act(x[e]) : 0.f;
+#pragma unroll
+          for (int e = 0; e < 4; e += 2) {
+            uint32_t s[3];
+            if (EXACT) s[0] = cs_pack(x[e], x[e + 1]);
+            else cs_slices(x[e], x[e + 1], s[0], s[1], s[2]);
+#pragma unroll
+            for (int p = 0; p < SLICES; ++p) (e ? kd : qd)[p * LO::SLICE + 16 * j] = s[p];
           }
         }
         bf[LO::V + i * CS_VS + lane] = i < n && v_live ? src.act(to_f(vv[tt])) : 0.f;
@@ -294,20 +328,34 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
       // scores: a warp of the first four takes 8 of the chunk's k and half of the rows
       if (lw < 4) {
         const int nt = lw >> 1, kh = lw & 1;
-        float acc[2][4] = {}, small[2][4] = {};
+        constexpr int NK = KP / 32;                       // steps of 16 rows
+        float acc[NK][4] = {}, small[4] = {};
+        const float* qr = bf + LO::Q + ((lane & 7) + ((lane >> 3) & 1) * 8) * KS + kh * (KP / 4) + (lane >> 4) * 4;
+        const float* kr = bf + LO::K + (nt * 8 + (lane & 7)) * KS + kh * (KP / 4) + (lane >> 3) * 4;
 #pragma unroll
-        for (int ks = 0; ks < KP / 16; ++ks) {
-          const int at = kh * (KP / 2) + ks * 8 + 2 * t;
-          const float4 a0 = parts_of_two<EXACT>(bf + LO::Q + g * KS, at), a1 = parts_of_two<EXACT>(bf + LO::Q + (g + 8) * KS, at);
-          const float4 k2 = parts_of_two<EXACT>(bf + LO::K + (nt * 8 + g) * KS, at);
-          const float hi[4] = {a0.x, a1.x, a0.z, a1.z}, lo[4] = {a0.y, a1.y, a0.w, a1.w};
-          mma_parts<EXACT, EXACT>(acc[ks & 1], small[ks & 1], hi, lo, k2.x, k2.z, k2.y, k2.w);
+        for (int ks = 0; ks < NK; ks += 2) {
+          uint32_t b4[3][4];
+#pragma unroll
+          for (int p = 0; p < SLICES; ++p) cs_ldmatrix(b4[p], kr + p * LO::SLICE + ks * 8);
+#pragma unroll
+          for (int two = 0; two < 2; ++two) {
+            uint32_t a[3][4], b[3][2];
+#pragma unroll
+            for (int p = 0; p < SLICES; ++p) {
+              cs_ldmatrix(a[p], qr + p * LO::SLICE + (ks + two) * 8);
+              b[p][0] = b4[p][2 * two];
+              b[p][1] = b4[p][2 * two + 1];
+            }
+            cs_products<EXACT, EXACT, false>(acc[ks + two], small, a, b);
+          }
         }
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
           const int i = g + (e >> 1) * 8, j = nt * 8 + 2 * t + (e & 1);
-          const float dot = (acc[0][e] + acc[1][e]) + (small[0][e] + small[1][e]);
-          bf[LO::A + (kh * CS_C + i) * CS_TS + j] = j <= i ? dot * bf[LO::D + i * CS_TS + j] * (bf[LO::PUT + j] * scale) : 0.f;
+          float dot = acc[0][e] + acc[1][e];
+          if constexpr (NK == 4) dot += acc[2][e] + acc[3][e];
+          if (!EXACT) dot += small[e];
+          bf[LO::A + (kh * CS_C + i) * CS_TS + j] = j <= i ? dot * bf[LO::D + i * CS_TS + j] : 0.f;
         }
       }
       __threadfence_block();
@@ -331,55 +379,86 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
     const int base = t0 + c * CS_C, n = min(CS_C, t1 - base);
     float* shares = sm + LO::SHARES + ((c & 1) * 2 + ct) * (2 * 4 * LO::SHARE) + lane;
     named_sync(CS_FULL + (c & 1), CS_THREADS);
-    // S^T q over this warp's rows: [16 columns] x [16 tokens]
-    {
-      float O[2][2][4] = {}, Ox[2][2][4] = {};
+    // v^T as an A operand: tokens 2t, 2t + 1 of columns col and col + 8, then tokens 2t + 8, 2t + 9
+    const float* vs = bf + LO::V + col;
+    float U[4][2];
 #pragma unroll
-      for (int k = 0; k < NT; ++k) {
-        float hi[4], lo[4];
-        split_operand(S[k], hi, lo);
+    for (int r = 0; r < 4; ++r)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) U[r][e] = vs[(2 * t + e + (r >> 1) * 8) * CS_VS + (r & 1) * 8];
+    {
+      // S^T q over this warp's rows: [16 columns] x [16 tokens]
+      float O[2][NT / 2][4] = {}, Ox[2][4] = {};
+      const float* qr = bf + LO::Q + ((lane & 7) + (lane >> 4) * 8) * KS + d0 / 2 + ((lane >> 3) & 1) * 4;
+#pragma unroll
+      for (int ks = 0; ks < NT / 2; ++ks) {
+        uint32_t a[3][4], b4[3][4];
+#pragma unroll
+        for (int r = 0; r < 4; ++r) cs_slices(S[2 * ks + (r >> 1)][2 * (r & 1)], S[2 * ks + (r >> 1)][2 * (r & 1) + 1], a[0][r], a[1][r], a[2][r]);
+#pragma unroll
+        for (int p = 0; p < SLICES; ++p) cs_ldmatrix(b4[p], qr + p * LO::SLICE + ks * 8);
 #pragma unroll
         for (int m = 0; m < 2; ++m) {
-          const float4 q2 = parts_of_two<EXACT>(bf + LO::Q + (m * 8 + g) * KS, d0 + k * 8 + 2 * t);
-          mma_parts<false, EXACT>(O[m][k & 1], Ox[m][k & 1], hi, lo, q2.x, q2.z, q2.y, q2.w);
+          uint32_t b[3][2];
+#pragma unroll
+          for (int p = 0; p < SLICES; ++p) {
+            b[p][0] = b4[p][2 * m];
+            b[p][1] = b4[p][2 * m + 1];
+          }
+          cs_products<false, EXACT, false>(O[m][ks], Ox[m], a, b);
         }
       }
 #pragma unroll
       for (int m = 0; m < 2; ++m)
 #pragma unroll
-        for (int e = 0; e < 4; ++e)
-          shares[(m * 4 + part) * LO::SHARE + e * 32] = (O[m][0][e] + O[m][1][e]) + (Ox[m][0][e] + Ox[m][1][e]);
+        for (int e = 0; e < 4; ++e) {
+          float o = O[m][0][e] + Ox[m][e];
+          if (NT == 4) o += O[m][NT / 2 - 1][e];
+          shares[(m * 4 + part) * LO::SHARE + e * 32] = o;
+        }
     }
-    // v^T as an A operand: elements (column, token 8m + t), (column, 8m + t + 4), then the same of column + 8
-    const float* vs = bf + LO::V + col;
-    float U[2][4];
-#pragma unroll
-    for (int m = 0; m < 2; ++m)
-#pragma unroll
-      for (int e = 0; e < 4; ++e) U[m][e] = vs[(m * 8 + t + (e & 1) * 4) * CS_VS + (e >> 1) * 8];
     // S = b_15 S + sum_j D_15,j put_j k_j v_j^T
     {
-      float uh[2][4], ul[2][4];
+      uint32_t u[3][4];
+      {
+        const float* end = bf + LO::END + 2 * t;
+        const float2 e[2] = {*reinterpret_cast<const float2*>(end), *reinterpret_cast<const float2*>(end + 8)};
+        const float2 r[2] = {*reinterpret_cast<const float2*>(end + CS_C), *reinterpret_cast<const float2*>(end + CS_C + 8)};
+        float w[4][2], rest[4][2], most[2];
 #pragma unroll
-      for (int m = 0; m < 2; ++m) {
-        const float e0 = bf[LO::END + m * 8 + t], e1 = bf[LO::END + m * 8 + t + 4];
-        const float u[4] = {U[m][0] * e0, U[m][1] * e1, U[m][2] * e0, U[m][3] * e1};
-        split_operand(u, uh[m], ul[m]);
-      }
-      const float all = bf[LO::ALL];
-      float acc[NT][4] = {}, x[NT][4] = {};
-#pragma unroll
-      for (int m = 0; m < 2; ++m)
-#pragma unroll
-        for (int k = 0; k < NT; ++k) {
-          const float* row = bf + LO::K + (m * 8 + t) * KS;
-          const float2 k0 = parts_of_one<EXACT>(row, d0 + k * 8 + g), k1 = parts_of_one<EXACT>(row + 4 * KS, d0 + k * 8 + g);
-          mma_parts<false, EXACT>(acc[k], x[k], uh[m], ul[m], k0.x, k1.x, k0.y, k1.y);
+        for (int k = 0; k < 4; ++k) {
+          w[k][0] = U[k][0] * e[k >> 1].x;
+          w[k][1] = U[k][1] * e[k >> 1].y;
+          rest[k][0] = fmaf(U[k][0], r[k >> 1].x, fmaf(U[k][0], e[k >> 1].x, -w[k][0]));
+          rest[k][1] = fmaf(U[k][1], r[k >> 1].y, fmaf(U[k][1], e[k >> 1].y, -w[k][1]));
         }
 #pragma unroll
-      for (int k = 0; k < NT; ++k)
+        for (int half = 0; half < 2; ++half)
+          most[half] = cs_most_of_four(fmaxf(fmaxf(fabsf(w[half][0]), fabsf(w[half][1])), fmaxf(fabsf(w[half + 2][0]), fabsf(w[half + 2][1]))));
 #pragma unroll
-        for (int e = 0; e < 4; ++e) S[k][e] = fmaf(all, S[k][e], acc[k][e] + x[k][e]);
+        for (int k = 0; k < 4; ++k) cs_grid_slices(w[k][0], w[k][1], rest[k][0], rest[k][1], most[k & 1], u[0][k], u[1][k], u[2][k]);
+      }
+      const float all = bf[LO::ALL], all_rest = bf[LO::ALL + 1];
+      const float* kr = bf + LO::K + ((lane & 7) + ((lane >> 3) & 1) * 8) * KS + d0 / 2 + (lane >> 4) * 4;
+#pragma unroll
+      for (int k = 0; k < NT; k += 2) {
+        uint32_t b4[3][4];
+#pragma unroll
+        for (int p = 0; p < SLICES; ++p) cs_ldmatrix_trans(b4[p], kr + p * LO::SLICE + k * 4);
+#pragma unroll
+        for (int two = 0; two < 2; ++two) {
+          uint32_t b[3][2];
+#pragma unroll
+          for (int p = 0; p < SLICES; ++p) {
+            b[p][0] = b4[p][2 * two];
+            b[p][1] = b4[p][2 * two + 1];
+          }
+          float acc[4] = {}, x[4] = {};
+          cs_products<false, EXACT, true>(acc, x, u, b);
+#pragma unroll
+          for (int e = 0; e < 4; ++e) S[k + two][e] = acc[e] + fmaf(all, S[k + two][e], fmaf(all_rest, S[k + two][e], x[e]));
+        }
+      }
     }
     // o = b S^T q + sum_j A_ij v_j: warps 0 and 1 of the four finish tokens 8 part + 2t, + 1, the others only hand their shares in
     if (part >= 2) {
@@ -388,19 +467,25 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
     } else {
       named_sync(CS_SHARES + ct, 128);
       float acc[4] = {}, x[4] = {};
+      {
+        uint32_t a[3][4], b[3][2];
+        float w[2][2];
 #pragma unroll
-      for (int kk = 0; kk < 2; ++kk) {
-        if (kk == 1 && part == 0) break;                  // (the same for the warp)
-        const float* a = bf + LO::A + (part * 8 + g) * CS_TS + kk * 8 + t;
-        float hi[4], lo[4], h0, l0, h1, l1;
-        if (EXACT) {
-          hi[0] = U[kk][0]; hi[1] = U[kk][2]; hi[2] = U[kk][1]; hi[3] = U[kk][3];
-        } else {
-          split_operand(U[kk], hi, lo);
+        for (int r = 0; r < 4; ++r) {
+          if (EXACT) a[0][r] = cs_pack(U[r][0], U[r][1]);
+          else cs_slices(U[r][0], U[r][1], a[0][r], a[1][r], a[2][r]);
         }
-        split_tf32(a[0] + a[CS_C * CS_TS], h0, l0);
-        split_tf32(a[4] + a[4 + CS_C * CS_TS], h1, l1);
-        mma_parts<EXACT, false>(acc, x, hi, lo, h0, h1, l0, l1);
+#pragma unroll
+        for (int r = 0; r < 2; ++r) {
+          const float* at = bf + LO::A + (part * 8 + g) * CS_TS + r * 8 + 2 * t;
+          const float2 a0 = *reinterpret_cast<const float2*>(at), a1 = *reinterpret_cast<const float2*>(at + CS_C * CS_TS);
+          w[r][0] = a0.x + a1.x;
+          w[r][1] = a0.y + a1.y;
+        }
+        const float most = cs_most_of_four(fmaxf(fmaxf(fabsf(w[0][0]), fabsf(w[0][1])), fmaxf(fabsf(w[1][0]), fabsf(w[1][1]))));
+#pragma unroll
+        for (int r = 0; r < 2; ++r) cs_grid_slices(w[r][0], w[r][1], 0.f, 0.f, most, b[0][r], b[1][r], b[2][r]);
+        cs_products<EXACT, false, true>(acc, x, a, b);
       }
       const float* sh = shares + part * 4 * LO::SHARE;
 #pragma unroll

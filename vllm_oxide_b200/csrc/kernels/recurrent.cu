@@ -379,7 +379,7 @@ struct LightningChunks {
   __device__ __forceinline__ T q_raw(size_t t, int h, int d) const { return s.rows[t * s.width + (size_t)h * s.dk + d]; }
   __device__ __forceinline__ T k_raw(size_t t, int h, int d) const { return s.rows[t * s.width + (size_t)(s.heads + h) * s.dk + d]; }
   __device__ __forceinline__ T v_raw(size_t t, int h, int c) const { return s.rows[t * s.width + (size_t)2 * s.heads * s.dk + (size_t)h * s.dv + c]; }
-  __device__ __forceinline__ float act(float x) const { return x * sigmoid_t<T>(x); }
+  __device__ __forceinline__ float act(float x) const { return x / (1.f + expf(-x)); }
   __device__ __forceinline__ float2 gate_raw(size_t, int) const { return make_float2(0.f, 0.f); }
   __device__ __forceinline__ float2 gates(float2, const Fixed& x) const { return make_float2(x.f, 1.f); }
   __device__ __forceinline__ float out_scale() const { return 1.f; }
@@ -1297,15 +1297,15 @@ VOB_API int vob_hgrn2_can_fuse(int dk, int dv) { return scan_can_fuse(dk, dv) ? 
 // The same for steps of one token a request (`single` below: no request brings more).
 VOB_API int vob_matrix_scan_can_step(int dk, int dv) { return scan_can_step(dk, dv) ? 1 : 0; }
 
-// Ranges that a request's tokens of a step should be cut into (unfused walks): the fewest units of time by a count of float
-// instructions a state element (three a token in one walk, five over the two walks of a cut portion, and what the join and the
-// launches cost in tokens), given how many blocks fit the device at once.
 // The walk's time over portions of `n` tokens cut into c ranges, in units of some 0.15 us.
 static double walk_cost(double n, int c, long blocks) {
   const long waves = (blocks * c + sm_count() - 1) / sm_count();
   return c <= 1 ? 3.0 * n * waves : (5.0 * n / c + 120.0) * waves + 60.0;
 }
 
+// Ranges that a request's tokens of a step should be cut into (unfused walks): the fewest units of time by a count of float
+// instructions a state element (three a token in one walk, five over the two walks of a cut portion, and what the join and the
+// launches cost in tokens), given how many blocks fit the device at once.
 VOB_API int vob_matrix_scan_chunks(int T, int B, int heads, int dk, int dv) {
   if (B <= 0 || T <= 0 || heads <= 0 || dk <= 0 || dv <= 0) return 1;
   const long blocks = (long)heads * tile_col_blocks(dk, dv) * B;
@@ -1320,20 +1320,22 @@ VOB_API int vob_matrix_scan_chunks(int T, int B, int heads, int dk, int dv) {
 }
 
 // Whether portions with one decay a head and token go by chunks on the tensor cores (chunk_scan.cuh; bfloat16 steps).  There a
-// request's chain is its chunks, 1.36 us each for 128 x 128 heads (2.07 where q, k and v are no bfloat16 numbers) behind some 6 us, and the
-// blocks share the SMs; the walk is as long as its longest portion (cut into the ranges that it would be cut into).  Measured on
-// B200, chunks and walk in us, lightning attention then mLSTM: 16 heads, 333 + 1,055 + 1,777 tokens: 233 and 476, 164 and 437; 1,501
-// beside 24 single tokens: 195 and 717, 143 and 736; one of 2,048: 265 and 182 (walks), 184 and 183; 32 heads, 4,001 tokens: 517 and
-// 764, 353 and 651; eight of 16 tokens: 18 and 16 (walks), 25 and 25 (walks).
+// request's chain is its chunks, 1.9 us each for 128 x 128 heads (3.0 where q, k and v are no bfloat16 numbers and take three slices)
+// behind some 6 us, and the blocks share the SMs; the walk is as long as its longest portion (cut into the ranges that it would be cut
+// into).  Heads of 64 x 64 take some two thirds of either.  Measured on B200, chunks and walk in us, lightning attention then mLSTM:
+// 16 heads, 333 + 1,055 + 1,777 tokens: 337 and 467, 226 and 466; 1,501 beside 24 single tokens: 285 and 733, 198 and 764; 200
+// beside 24: 64 and 127, 77 and 147; one of 2,048: 381 and 193, 243 and 205 (walks); one of 256: 61 and 54 (walk), 55 and 64; eight of
+// 16: 34 and 28, 40 and 41 (walks); 32 heads, one of 4,001: 745 and 778 (too near: walk), 451 and 675; one of 1,000: 196 and 203,
+// 135 and 210.
 VOB_API int vob_matrix_scan_by_chunks(int T, int B, int longest, int heads, int dk, int dv, int exact) {
   if (B <= 0 || T <= 0 || longest <= 1 || !chunk_scan_takes(dk, dv, heads, B)) return 0;
   const long blocks = (long)heads * tile_col_blocks(dk, dv) * B;
   const int c = vob_matrix_scan_chunks(T, B, heads, dk, dv);
   double walk = walk_cost((double)T / B, c, blocks);
   if (walk < walk_cost(longest, c, 1)) walk = walk_cost(longest, c, 1);
-  const double per = exact ? 1.36 : 2.07, chain = 6.0 + per * ((longest + CS_C - 1) / CS_C);
-  const double all = (double)heads * ((dv + CS_COLS - 1) / CS_COLS) * (6.0 * B + per * ((double)T / CS_C + 0.5 * B)) / sm_count();
-  return (chain > all ? chain : all) < 0.15 * walk ? 1 : 0;
+  const double per = exact ? 1.9 : 3.0, chain = 6.0 + per * ((longest + CS_C - 1) / CS_C);
+  const double all = (double)heads * ((dv + CS_COLS - 1) / CS_COLS) * (3.0 * B + per * ((double)T / CS_C + 0.5 * B)) / sm_count();
+  return (chain > all ? chain : all) < 0.14 * walk ? 1 : 0;
 }
 
 VOB_API int vob_hgrn2_scan(const void* qfv, const void* bf, const float* lower, const float* nw, float* state, const int* cu_q,
