@@ -141,6 +141,62 @@ def test_no_further_from_64_bits_than_the_walk(kind, dk, dv, T):
             assert mine <= 1.1 * walk + 3e-9, (h, mine, walk)
 
 
+# what is planted, and where: (part of the row, token), or the state; the places are the second request's
+ODD = {"infinite v": ("v", 21, float("inf")), "NaN in q": ("q", 40, float("nan")), "infinite k": ("k", 17, float("-inf")),
+       "NaN in v, first token": ("v", 0, float("nan")), "large v": ("v", 5, 2.0 ** 100), "large k, last token": ("k", 49, 2.0 ** 90),
+       "infinite state": ("state", 0, float("inf")), "large state": ("state", 0, 2.0 ** 70)}
+
+
+@pytest.mark.parametrize("what", list(ODD))
+@pytest.mark.parametrize("kind", ["lightning", "mlstm"])
+@pytest.mark.parametrize("dk,dv", [(128, 128), (40, 33)])
+def test_values_that_are_not_usual(dk, dv, kind, what):
+    """Infinities, NaN and numbers near the end of the range go where the walk takes them and nowhere else: not to another request, head or
+    column, nor to an earlier token."""
+    from vllm_oxide_b200 import kernels
+    place, token, value = ODD[what]
+    heads, lens = 2, [20, 50, 33]
+    T, B, W = sum(lens), len(lens), heads * (2 * dk + dv)
+    g = torch.Generator().manual_seed(dk + token)
+    rows = torch.randn(T, W + 2 * heads + heads * dv, generator=g).bfloat16()
+    state0 = torch.randn(B, (heads * (dk * (dv + 1) + 1) + 3) // 4 * 4, generator=g) * 0.3
+    state0[:, heads * dk * (dv + 1):] = 0.1
+    cu = torch.tensor([0] + torch.tensor(lens).cumsum(0).tolist(), dtype=torch.int32, device=DEV)
+    slots, err = torch.arange(B, dtype=torch.int32, device=DEV), torch.zeros(1, dtype=torch.int32, device=DEV)
+
+    def run(by_chunks):
+        state, raw, nq = state0.to(DEV), torch.zeros(T, heads * dv, device=DEV), torch.zeros(T, heads, device=DEV)
+        if kind == "lightning":
+            kernels.lightning_scan(rows.to(DEV), torch.tensor([0.9, 0.5], device=DEV), state, cu, slots, raw, B, heads, dk, dv, err,
+                                   by_chunks=by_chunks)
+        else:
+            kernels.mlstm_scan(rows.to(DEV), W, W + heads, W + 2 * heads, torch.zeros(heads, device=DEV), torch.full((heads,), 3.0, device=DEV),
+                               torch.ones(heads * dv, device=DEV), state, cu, slots, B, heads, dk, dv, dk ** -0.5, 15.0, 1e-6, err,
+                               gates=torch.empty(T, heads * 4, device=DEV), raw=raw, nq=nq, by_chunks=by_chunks)
+        return raw.cpu(), state.cpu(), nq.cpu()
+
+    clean = run(True)
+    if place == "state":
+        state0[1, dk * dv + 3 * dv + 7] = value                      # head 1, row 3, column 7
+    else:
+        rows[lens[0] + token, {"q": 0, "k": heads * dk, "v": 2 * heads * dk}[place] + 5] = value          # head 0, place 5
+    mine, walk = run(True), run(False)
+    assert int(err.item()) == 0
+    odd = 0
+    others = [[t for t in range(T) if not lens[0] <= t < lens[0] + lens[1]], [0, 2], [t for t in range(T) if not lens[0] <= t < lens[0] + lens[1]]]
+    for x, want, plain, rest in zip(mine, walk, clean, others):
+        assert torch.equal(x[rest], plain[rest])
+        for is_odd in (torch.isnan, torch.isposinf, torch.isneginf):
+            assert torch.equal(is_odd(x), is_odd(want))
+        usual = torch.isfinite(want)
+        odd += int((~usual).sum()) + int((want[usual].abs() > 1e9).sum())
+        # sums of large numbers cancel: an error counts against the largest of its row and column
+        most = torch.where(usual, want, 0.0).abs()
+        size = torch.maximum(most.amax(dim=1, keepdim=True), most.amax(dim=0, keepdim=True))[usual]
+        assert ((x[usual] - want[usual]).abs() <= 1e-5 * size).all()
+    assert odd > 0
+
+
 def test_which_steps_go_by_chunks():
     """The rule: bfloat16 heads of up to 128 rows whose longest portion is the shorter way on the tensor cores."""
     from vllm_oxide_b200 import kernels

@@ -20,6 +20,8 @@
 //     far below that one then leave nothing to cut off;
 //   * products of decays carry their rounding errors along (hi + lo), and b_15 multiplies S as such a pair: over a long text
 //     nothing drifts.
+// Values that are infinite, NaN or not below 2^36 would mix in such sums.  A chunk that holds one is walked token by token in the same
+// registers, with the walk's own operations, and so is a share of S with one: a token never reaches another column or an earlier token.
 #pragma once
 #include "common.cuh"
 
@@ -28,6 +30,7 @@ namespace vob {
 constexpr int CS_C = 16, CS_COLS = 32;                 // tokens of a chunk, columns of a block
 constexpr int CS_COMPUTE = 256, CS_LOADERS = 256, CS_DECAYS = 32, CS_THREADS = CS_COMPUTE + CS_LOADERS + CS_DECAYS;
 constexpr int CS_VS = CS_COLS + 4, CS_TS = CS_C + 4;   // rows in shared memory: a fragment's reads fall into different banks
+constexpr float CS_MOST = 68719476736.f;               // 2^36: values that are not below go by multiply-adds (q k v of 2^108 still adds up)
 // named barriers: a buffer is full (everyone), a buffer is empty (computing warps and loaders; computing warps and decays), a chunk's
 // rows and decays are there (loaders, decays), the shares of 16 columns are there (their computing warps)
 enum { CS_FULL = 1, CS_EMPTY = 3, CS_ROWS = 5, CS_SHARES = 6, CS_EMPTY_DECAYS = 8 };
@@ -40,12 +43,14 @@ template <int KP, bool EXACT> struct ChunkLayout {
   static constexpr int D = A + 2 * CS_C * CS_TS;       // D_ij put_j, times the read-out's scale
   static constexpr int PRE = D + CS_C;                 // b_i, times the read-out's scale: column 16 of the rows of D
   static constexpr int END = D + CS_C * CS_TS;         // D_15,j put_j, behind them what is missing from each
-  static constexpr int ALL = END + 2 * CS_C;           // b_15, and what is missing from it
+  static constexpr int KEEP = END + 2 * CS_C, PUT = KEEP + CS_C;
+  static constexpr int ODD = PUT + CS_C;               // a loader warp's word: it has seen a value that is not below CS_MOST
+  static constexpr int ALL = ODD + CS_LOADERS / 32;    // b_15, and what is missing from it
   static constexpr int FLOATS = ALL + 4;
   // behind the two buffers: the shares of S^T q, by the chunk's parity, 16 columns, 8 tokens and quarter of the rows
   static constexpr int SHARES = 2 * FLOATS, SHARE = 4 * 32;
   static constexpr int TOTAL = SHARES + 2 * 2 * 2 * 4 * SHARE;
-  static_assert(KS % 4 == 0 && FLOATS % 4 == 0 && END % 4 == 0 && D % 4 == 0, "rows and vectors start on 16 bytes");
+  static_assert(KS % 4 == 0 && FLOATS % 4 == 0 && ODD % 4 == 0 && END % 4 == 0 && D % 4 == 0, "rows and vectors start on 16 bytes");
 };
 
 __device__ __forceinline__ void cs_mma(float (&d)[4], const uint32_t (&a)[4], uint32_t b0, uint32_t b1) {
@@ -60,6 +65,12 @@ __device__ __forceinline__ void cs_ldmatrix(uint32_t (&r)[4], const float* row) 
 __device__ __forceinline__ void cs_ldmatrix_trans(uint32_t (&r)[4], const float* row) {
   asm volatile("ldmatrix.sync.aligned.m8n8.x4.trans.shared.b16 {%0,%1,%2,%3}, [%4];\n"
                : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]) : "r"((unsigned)__cvta_generic_to_shared(row)));
+}
+// The larger magnitude, NaN if one is NaN.
+__device__ __forceinline__ float cs_larger(float x, float y) {
+  float m;
+  asm("max.NaN.f32 %0, %1, %2;\n" : "=f"(m) : "f"(fabsf(x)), "f"(fabsf(y)));
+  return m;
 }
 // Two bfloat16 numbers in a word, the first in the low half.
 __device__ __forceinline__ uint32_t cs_pack(float x, float y) {
@@ -76,6 +87,16 @@ __device__ __forceinline__ void cs_slices(float x, float y, uint32_t& hi, uint32
   mid = cs_pack(x, y);
   const float2 m = cs_unpack(mid);
   lo = cs_pack(x - m.x, y - m.y);
+}
+// The same for values of any size, cut off instead of rounded: an infinity or NaN is hi alone.
+__device__ __forceinline__ uint32_t cs_top(float x) { return __float_as_uint(x != x ? __uint_as_float(0x7fff0000u) : x) & 0xffff0000u; }
+__device__ __forceinline__ void cs_slices_any(float x, float y, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
+  const uint32_t hx = cs_top(x), hy = cs_top(y);
+  const float rx = isfinite(x) ? x - __uint_as_float(hx) : 0.f, ry = isfinite(y) ? y - __uint_as_float(hy) : 0.f;
+  const uint32_t mx = cs_top(rx), my = cs_top(ry);
+  hi = hx >> 16 | hy;
+  mid = mx >> 16 | my;
+  lo = cs_top(rx - __uint_as_float(mx)) >> 16 | cs_top(ry - __uint_as_float(my));
 }
 // (x + rx, y + ry) as slices of which hi lies on the grid of 2^-7 of the power of two in `most` (the largest |x| of those that are summed).
 __device__ __forceinline__ void cs_grid_slices(float x, float y, float rx, float ry, float most, uint32_t& hi, uint32_t& mid, uint32_t& lo) {
@@ -219,6 +240,8 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
         const float end = run * gt.y;
         bf[LO::END + lane] = end;
         bf[LO::END + CS_C + lane] = fmaf(rest, gt.y, fmaf(run, gt.y, -end));
+        bf[LO::KEEP + lane] = gt.x;
+        bf[LO::PUT + lane] = gt.y;
       }
       if (lane == CS_C) {
         const float all = run + rest;
@@ -301,28 +324,35 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
       float* bf = sm + (c & 1) * LO::FLOATS;
       const int n = min(CS_C, t1 - t0 - c * CS_C);
       if (c >= 2) named_sync(CS_EMPTY + (c & 1), CS_COMPUTE + CS_LOADERS);
+      bool odd = false;
 #pragma unroll
       for (int tt = 0; tt < TPW; ++tt) {
         const int i = lw + STEP * tt;
         uint32_t* qd = reinterpret_cast<uint32_t*>(bf) + LO::Q + i * KS + lane;
         uint32_t* kd = reinterpret_cast<uint32_t*>(bf) + LO::K + i * KS + lane;
+        float x[2 * NV], most = 0.f;                       // q's and k's rows, two by two
 #pragma unroll
-        for (int j = 0; j < NV; j += 2) {
-          const int d = 2 * lane + 32 * j;
-          float x[4] = {to_f(qv[tt][j]), to_f(qv[tt][j + 1]), to_f(kv[tt][j]), to_f(kv[tt][j + 1])};
-#pragma unroll
-          for (int e = 0; e < 4; ++e) x[e] = i < n && d + (e & 1) < dk ? src.act(x[e]) : 0.f;
-#pragma unroll
-          for (int e = 0; e < 4; e += 2) {
-            uint32_t s[3];
-            if (EXACT) s[0] = cs_pack(x[e], x[e + 1]);
-            else cs_slices(x[e], x[e + 1], s[0], s[1], s[2]);
-#pragma unroll
-            for (int p = 0; p < SLICES; ++p) (e ? kd : qd)[p * LO::SLICE + 16 * j] = s[p];
-          }
+        for (int e = 0; e < 2 * NV; ++e) {
+          const int j = (e >> 2) * 2 + (e & 1);
+          x[e] = i < n && 2 * lane + 32 * (j & ~1) + (j & 1) < dk ? src.act(to_f(e & 2 ? kv[tt][j] : qv[tt][j])) : 0.f;
+          most = cs_larger(most, x[e]);
         }
-        bf[LO::V + i * CS_VS + lane] = i < n && v_live ? src.act(to_f(vv[tt])) : 0.f;
+        const bool usual = most < CS_MOST;
+#pragma unroll
+        for (int e = 0; e < 2 * NV; e += 2) {
+          uint32_t s[3];
+          if (EXACT) s[0] = cs_pack(x[e], x[e + 1]);
+          else if (usual) cs_slices(x[e], x[e + 1], s[0], s[1], s[2]);
+          else cs_slices_any(x[e], x[e + 1], s[0], s[1], s[2]);
+#pragma unroll
+          for (int p = 0; p < SLICES; ++p) (e & 2 ? kd : qd)[p * LO::SLICE + 32 * (e >> 2)] = s[p];
+        }
+        const float v = i < n && v_live ? src.act(to_f(vv[tt])) : 0.f;
+        odd |= !(cs_larger(most, v) < CS_MOST);
+        bf[LO::V + i * CS_VS + lane] = v;
       }
+      odd = __any_sync(0xffffffffu, odd);
+      if (lane == 0) bf[LO::ODD + lw] = __int_as_float(odd ? 1 : 0);
       if (c + 1 < chunks) fetch(c + 1);
       named_sync(CS_ROWS, CS_LOADERS + CS_DECAYS);
       // scores: a warp of the first four takes 8 of the chunk's k and half of the rows
@@ -374,11 +404,55 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
       const int row = d0 + k * 8 + 2 * t + (e & 1), j = col + (e >> 1) * 8;
       S[k][e] = row < dk && c0 + j < dv ? mine[(size_t)row * dv + j] : 0.f;
     }
+  auto odd_share = [&]() {                              // (the same for the warp)
+    float most[4] = {};
+#pragma unroll
+    for (int k = 0; k < NT; ++k)
+#pragma unroll
+      for (int e = 0; e < 4; ++e) most[e] = cs_larger(most[e], S[k][e]);
+    return __any_sync(0xffffffffu, !(cs_larger(cs_larger(most[0], most[1]), cs_larger(most[2], most[3])) < CS_MOST)) != 0;
+  };
+  bool share_is_odd = odd_share();
   for (int c = 0; c < chunks; ++c) {
     const float* bf = sm + (c & 1) * LO::FLOATS;
     const int base = t0 + c * CS_C, n = min(CS_C, t1 - base);
     float* shares = sm + LO::SHARES + ((c & 1) * 2 + ct) * (2 * 4 * LO::SHARE) + lane;
+    // the chunk's tokens one after the other by multiply-adds, as the walk: S updated by them, S^T q of this warp's rows read out, or both
+    auto walk = [&](bool update, bool read) {
+      auto element = [&](int at, int i, int row) {
+        float x = 0.f;
+#pragma unroll
+        for (int p = SLICES - 1; p >= 0; --p) {
+          const float2 two = cs_unpack(__float_as_uint(bf[at + p * LO::SLICE + i * KS + (row >> 1)]));
+          x += row & 1 ? two.y : two.x;
+        }
+        return x;
+      };
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        const float keep = bf[LO::KEEP + i], put = bf[LO::PUT + i], v[2] = {bf[LO::V + i * CS_VS + col], bf[LO::V + i * CS_VS + col + 8]};
+        float o[2] = {0.f, 0.f};
+#pragma unroll
+        for (int k = 0; k < NT; ++k)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) {
+            const int row = d0 + k * 8 + 2 * t + (e & 1);
+            if (row >= dk) continue;
+            if (update) S[k][e] = fmaf(keep, S[k][e], element(LO::K, i, row) * put * v[e >> 1]);
+            if (read) o[e >> 1] = fmaf(S[k][e], element(LO::Q, i, row), o[e >> 1]);
+          }
+        if (!read) continue;
+#pragma unroll
+        for (int half = 0; half < 2; ++half) {
+          o[half] += __shfl_xor_sync(0xffffffffu, o[half], 1);
+          o[half] += __shfl_xor_sync(0xffffffffu, o[half], 2);
+          if (t == (i & 7) >> 1) shares[((i >> 3) * 4 + part) * LO::SHARE + ((i & 1) + 2 * half) * 32] = o[half];
+        }
+      }
+    };
     named_sync(CS_FULL + (c & 1), CS_THREADS);
+    const uint4 odd0 = *reinterpret_cast<const uint4*>(bf + LO::ODD), odd1 = *reinterpret_cast<const uint4*>(bf + LO::ODD + 4);
+    const bool odd = (odd0.x | odd0.y | odd0.z | odd0.w | odd1.x | odd1.y | odd1.z | odd1.w) != 0;      // (the same for the block)
     // v^T as an A operand: tokens 2t, 2t + 1 of columns col and col + 8, then tokens 2t + 8, 2t + 9
     const float* vs = bf + LO::V + col;
     float U[4][2];
@@ -386,7 +460,9 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
     for (int r = 0; r < 4; ++r)
 #pragma unroll
       for (int e = 0; e < 2; ++e) U[r][e] = vs[(2 * t + e + (r >> 1) * 8) * CS_VS + (r & 1) * 8];
-    {
+    if (odd || share_is_odd) {
+      walk(odd, true);
+    } else {
       // S^T q over this warp's rows: [16 columns] x [16 tokens]
       float O[2][NT / 2][4] = {}, Ox[2][4] = {};
       const float* qr = bf + LO::Q + ((lane & 7) + (lane >> 4) * 8) * KS + d0 / 2 + ((lane >> 3) & 1) * 4;
@@ -418,7 +494,9 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
         }
     }
     // S = b_15 S + sum_j D_15,j put_j k_j v_j^T
-    {
+    if (!odd && share_is_odd) {
+      walk(true, false);
+    } else if (!odd) {
       uint32_t u[3][4];
       {
         const float* end = bf + LO::END + 2 * t;
@@ -460,6 +538,7 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
         }
       }
     }
+    share_is_odd = odd_share();
     // o = b S^T q + sum_j A_ij v_j: warps 0 and 1 of the four finish tokens 8 part + 2t, + 1, the others only hand their shares in
     if (part >= 2) {
       __threadfence_block();
@@ -467,7 +546,7 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
     } else {
       named_sync(CS_SHARES + ct, 128);
       float acc[4] = {}, x[4] = {};
-      {
+      if (!odd) {
         uint32_t a[3][4], b[3][2];
         float w[2][2];
 #pragma unroll
@@ -492,7 +571,7 @@ chunk_scan_kernel(const SRC src, float* state, long state_stride, const int* __r
       for (int e = 0; e < 4; ++e) {
         const int tok = part * 8 + 2 * t + (e & 1), j = col + (e >> 1) * 8;
         const float o = (sh[e * 32] + sh[LO::SHARE + e * 32]) + (sh[2 * LO::SHARE + e * 32] + sh[3 * LO::SHARE + e * 32]);
-        const float y = fmaf(bf[LO::PRE + tok * CS_TS], o, acc[e] + x[e]);
+        const float y = odd ? o * scale : fmaf(bf[LO::PRE + tok * CS_TS], o, acc[e] + x[e]);
         if (tok < n && c0 + j < dv) raw[((size_t)(base + tok) * heads + h) * dv + c0 + j] = y;
       }
     }

@@ -1320,20 +1320,20 @@ VOB_API int vob_matrix_scan_chunks(int T, int B, int heads, int dk, int dv) {
 }
 
 // Whether portions with one decay a head and token go by chunks on the tensor cores (chunk_scan.cuh; bfloat16 steps).  There a
-// request's chain is its chunks, 1.9 us each for 128 x 128 heads (3.0 where q, k and v are no bfloat16 numbers and take three slices)
+// request's chain is its chunks, 2.1 us each for 128 x 128 heads (3.3 where q, k and v are no bfloat16 numbers and take three slices)
 // behind some 6 us, and the blocks share the SMs; the walk is as long as its longest portion (cut into the ranges that it would be cut
 // into).  Heads of 64 x 64 take some two thirds of either.  Measured on B200, chunks and walk in us, lightning attention then mLSTM:
-// 16 heads, 333 + 1,055 + 1,777 tokens: 337 and 467, 226 and 466; 1,501 beside 24 single tokens: 285 and 733, 198 and 764; 200
-// beside 24: 64 and 127, 77 and 147; one of 2,048: 381 and 193, 243 and 205 (walks); one of 256: 61 and 54 (walk), 55 and 64; eight of
-// 16: 34 and 28, 40 and 41 (walks); 32 heads, one of 4,001: 745 and 778 (too near: walk), 451 and 675; one of 1,000: 196 and 203,
-// 135 and 210.
+// 16 heads, 333 + 1,055 + 1,777 tokens: 375 and 465, 255 and 464; 1,501 beside 24 single tokens: 315 and 732, 224 and 765; 200
+// beside 24: 69 and 129, 85 and 155; one of 2,048: 421 and 192, 276 and 204 (walks); one of 256: 67 and 54 (walk), 59 and 64; eight of
+// 16: 36 and 28, 41 and 41 (walks); 32 heads, one of 4,001: 813 and 785 (walk), 520 and 676; one of 1,000: 216 and 203 (walk),
+// 158 and 217.
 VOB_API int vob_matrix_scan_by_chunks(int T, int B, int longest, int heads, int dk, int dv, int exact) {
   if (B <= 0 || T <= 0 || longest <= 1 || !chunk_scan_takes(dk, dv, heads, B)) return 0;
   const long blocks = (long)heads * tile_col_blocks(dk, dv) * B;
   const int c = vob_matrix_scan_chunks(T, B, heads, dk, dv);
   double walk = walk_cost((double)T / B, c, blocks);
   if (walk < walk_cost(longest, c, 1)) walk = walk_cost(longest, c, 1);
-  const double per = exact ? 1.9 : 3.0, chain = 6.0 + per * ((longest + CS_C - 1) / CS_C);
+  const double per = exact ? 2.1 : 3.3, chain = 6.0 + per * ((longest + CS_C - 1) / CS_C);
   const double all = (double)heads * ((dv + CS_COLS - 1) / CS_COLS) * (3.0 * B + per * ((double)T / CS_C + 0.5 * B)) / sm_count();
   return (chain > all ? chain : all) < 0.14 * walk ? 1 : 0;
 }
