@@ -50,3 +50,39 @@ def test_keys_and_values_of_one_plane(hd, block_size, window, nh):
     got, want = run_attention(attention, torch.bfloat16, nh, 1, hd, block_size, window, [2, 300, 129, 64], [2, 517, 129, 200], craft=same_rows)
     # (two roundings to bfloat16 of values of order one, as for every case of this kernel)
     assert torch.allclose(got, want, rtol=2e-2, atol=2e-2)
+
+
+@pytest.mark.parametrize("kernel", [dict(), dict(use_tc5=False), dict(use_tc5=False, use_tma=False)], ids=["tcgen05", "TMA", "cp.async"])
+@pytest.mark.parametrize("hd,bias", [(64, False), (128, True), (192, False), (256, True)])
+def test_capped_scores_in_tiles_without_a_mask(hd, bias, kernel):
+    """A cap on the scores (and a bias behind it) counts in every tile, also in those that lie wholly before the queries: against
+    64 bits, over contexts of many tiles, with scores that the cap changes by half."""
+    import math
+    from vllm_oxide_b200 import kernels
+    dev, nh, kvh, bs, cap = "cuda:0", 4, 2, 64, 4.0
+    q_lens, ctx_lens = [70, 2], [700, 300]
+    g = torch.Generator(device=dev).manual_seed(hd)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev)
+    pages = [-(-c // bs) for c in ctx_lens]
+    kc, vc = rnd(sum(pages), kvh, bs, hd).bfloat16(), rnd(sum(pages), kvh, bs, hd).bfloat16()
+    bt = torch.full((2, max(pages)), -1, dtype=torch.int32)
+    bt[0, :pages[0]], bt[1, :pages[1]] = torch.arange(pages[0]).int(), torch.arange(pages[0], sum(pages)).int()
+    T = sum(q_lens)
+    q, table = (rnd(T, nh * hd) * 3).bfloat16(), rnd(nh, 400) if bias else None
+    cu, ctx = (torch.tensor(x, dtype=torch.int32, device=dev) for x in ([0, q_lens[0], T], ctx_lens))
+    out, err, scale = torch.empty(T, nh * hd, device=dev), torch.zeros(1, dtype=torch.int32, device=dev), 1 / math.sqrt(hd)
+    kernels.attention_prefill(q, nh * hd, out, kc, vc, bt.to(dev), cu, ctx, 2, max(q_lens), nh, kvh, hd, 0, scale, err, softcap=cap,
+                              dist_bias=table, **kernel)
+    assert int(err.item()) == 0
+    at = 0
+    for b, (n, c) in enumerate(zip(q_lens, ctx_lens)):
+        rows = bt[b, :pages[b]].long().to(dev)
+        k, v = (x[rows].double().transpose(0, 1).reshape(kvh, -1, hd)[:, :c].repeat_interleave(nh // kvh, 0) for x in (kc, vc))
+        s = cap * torch.tanh(q[at:at + n].double().view(n, nh, hd).transpose(0, 1) @ k.transpose(1, 2) * scale / cap)
+        dist = torch.arange(c - n, c, device=dev)[:, None] - torch.arange(c, device=dev)[None]
+        if bias:
+            s = s + table.double()[:, dist.clamp(0, table.shape[1] - 1)]
+        want = (torch.softmax(s.masked_fill(dist < 0, -math.inf), 2) @ v).transpose(0, 1).reshape(n, -1)
+        # probabilities in bfloat16, half an ulp of which is 2^-9: the norm of the error stays below that
+        assert ((out[at:at + n].double() - want).norm() / want.norm()).item() < 2 ** -9
+        at += n

@@ -368,8 +368,13 @@ attention_prefill_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
           for (int e = 0; e < 4; ++e) {
             const int h = e >> 1;
             const int key = k0 + i * 8 + tq * 2 + (e & 1);
-            sv[i][e] = sv[i][e] * sc + dist_term(brow[h], rpos[h] - key, ep.dist_rows - 1);
+            sv[i][e] = score2(sv[i][e], sc, ep) + dist_term(brow[h], rpos[h] - key, ep.dist_rows - 1);
           }
+      } else if (ep.cap_out > 0.f) {
+#pragma unroll
+        for (int i = 0; i < 8; ++i)
+#pragma unroll
+          for (int e = 0; e < 4; ++e) sv[i][e] = score2(sv[i][e], sc, ep);
       } else {
 #pragma unroll
         for (int i = 0; i < 8; ++i) { sv[i][0] *= sc; sv[i][1] *= sc; sv[i][2] *= sc; sv[i][3] *= sc; }
