@@ -86,3 +86,33 @@ def test_capped_scores_in_tiles_without_a_mask(hd, bias, kernel):
         # probabilities in bfloat16, half an ulp of which is 2^-9: the norm of the error stays below that
         assert ((out[at:at + n].double() - want).norm() / want.norm()).item() < 2 ** -9
         at += n
+
+
+@pytest.mark.parametrize("hd,nh,kvh,window,one_plane", [(256, 16, 1, 0, True), (256, 8, 4, 300, False), (192, 12, 3, 0, False), (192, 16, 1, 100, True)])
+def test_large_heads_are_no_further_from_64_bits(hd, nh, kvh, window, one_plane):
+    """The probabilities of a row are rounded to bfloat16 against the row's own maximum, as in the mma.sync kernel, so that the largest is
+    exact: the tcgen05 kernel's error against 64 bits is that kernel's (float output, so that nothing hides it)."""
+    import math
+    from vllm_oxide_b200 import kernels
+    dev, bs, n, c = "cuda:0", 64, 300, 1100
+    g = torch.Generator(device=dev).manual_seed(hd + nh)
+    rnd = lambda *s: torch.randn(*s, generator=g, device=dev)
+    pages = -(-c // bs)
+    kc = rnd(pages, kvh, bs, hd).bfloat16()
+    vc = kc if one_plane else rnd(pages, kvh, bs, hd).bfloat16()
+    q, scale = (rnd(n, nh * hd) * 1.5).bfloat16(), 1 / math.sqrt(hd)
+    bt, err = torch.arange(pages, dtype=torch.int32, device=dev)[None], torch.zeros(1, dtype=torch.int32, device=dev)
+    cu, ctx = torch.tensor([0, n], dtype=torch.int32, device=dev), torch.tensor([c], dtype=torch.int32, device=dev)
+    k, v = (x.double().transpose(0, 1).reshape(kvh, -1, hd)[:, :c].repeat_interleave(nh // kvh, 0) for x in (kc, vc))
+    dist = torch.arange(c - n, c, device=dev)[:, None] - torch.arange(c, device=dev)[None]
+    seen = (dist >= 0) & ((dist < window) if window else (dist >= 0))
+    s = (q.double().view(n, nh, hd).transpose(0, 1) @ k.transpose(1, 2) * scale).masked_fill(~seen, -math.inf)
+    want = (torch.softmax(s, 2) @ v).transpose(0, 1).reshape(n, -1)
+    errors = []
+    for kernel in (dict(), dict(use_tc5=False)):
+        out = torch.empty(n, nh * hd, device=dev)
+        kernels.attention_prefill(q, nh * hd, out, kc, vc, bt, cu, ctx, 1, n, nh, kvh, hd, window, scale, err, **kernel)
+        assert int(err.item()) == 0
+        errors.append(((out.double() - want).norm() / want.norm()).item())
+    # (a hundredth: what two sums of the same rounded terms in another order may differ by is far below that)
+    assert errors[0] <= 1.01 * errors[1], errors

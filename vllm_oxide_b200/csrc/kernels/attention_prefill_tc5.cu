@@ -47,12 +47,13 @@ constexpr int F5_TILE = 64;                                // keys per step
 constexpr int F5_SLICES = HD / 64;                         // 64-column slices of a head
 constexpr int F5_Q_BYTES = F5_SLICES * F5_ROWS * 128;      // a query tile: [slice][128 rows][128 bytes]
 constexpr int F5_KV_BYTES = F5_SLICES * F5_TILE * 128;     // one of K or V: [slice][64 keys][128 bytes]
-constexpr float F5_MAX_SLACK = 8.f;                        // how far a row's maximum may run ahead of its reference
+// How far a row's maximum may run ahead of its reference.  At 0 the largest P of a row is 1, which bfloat16 holds exactly, and an output is
+// as near as from the mma.sync kernel (errors of 8.7e-4 against 64 bits where a slack of 8 left 1.1e-3: 2,048 tokens of 16 heads of
+// 256 over one plane, 53 us so, 48 with the slack, 235 by mma.sync).
+constexpr float F5_MAX_SLACK = HD <= 128 ? 8.f : 0.f;
 
 // NQ: query tiles of a block (two only for heads of up to 128: shared and tensor memory hold no more).  ONE_PLANE: keys and
-// values are the same rows (latent attention), which a stage then holds once, read as K and, MN-major, as V.  Heads of 256 over one
-// plane (16 heads, 2,048 tokens, window 1,024) were taken by the mma.sync kernel before, at 242 us a layer: 184 us less here (a step of
-// eight layers, four of them such: 3.91 ms before, 3.17 now).
+// values are the same rows (latent attention), which a stage then holds once, read as K and, MN-major, as V.
 template <int NQ, bool ONE_PLANE> struct F5 {
   static constexpr int STAGE_BYTES = (ONE_PLANE ? 1 : 2) * F5_KV_BYTES;
   static constexpr int THREADS = (5 * NQ + 1) * 32;        // 4 softmax warps and one issuing warp per tile, a producer
@@ -447,30 +448,30 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
         sum = (part[0] + part[1]) + (part[2] + part[3]);
       };
       load_scores();
-      // The reference maximum moves only when the row's maximum has run ahead of it, which is rare after a row's
-      // first steps.  So from the second step on the exponentials are taken against the old reference at once, beside
+      // The reference maximum moves only when the row's maximum has run ahead of it, which with some slack is rare after a
+      // row's first steps.  So from the second step on the exponentials are taken against the old reference at once, beside
       // the search for the maximum (the two do not depend on each other, and the chain of maxima hides behind the
       // exponentials); only if some row of the warp has to move its reference are the scores read again and the
-      // step's exponentials taken anew.
+      // step's exponentials taken anew.  Without slack most steps move some row's: the maximum comes first.
+      constexpr bool AHEAD = F5_MAX_SLACK > 0.f;
       float mx = 0.f;
       bool moved = i == 0;
-      if (i > 0) {
+      if (AHEAD && i > 0) {
         exponentials(m_ref == -INFINITY ? 0.f : -m_ref);
         mx = row_max();
         moved = __any_sync(0xffffffffu, mx > m_ref + F5_MAX_SLACK);
         if (moved) load_scores();
       } else {
         mx = row_max();
+        moved = i == 0 || __any_sync(0xffffffffu, mx > m_ref + F5_MAX_SLACK);
       }
       float factor = 1.f;
-      if (moved) {
-        if (mx > m_ref + F5_MAX_SLACK) {
-          factor = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - mx);
-          m_ref = mx;
-          l *= factor;
-        }
-        exponentials(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that has seen no key yet: a finite stand-in
+      if (moved && mx > m_ref + F5_MAX_SLACK) {
+        factor = m_ref == -INFINITY ? 0.f : fast_exp2(m_ref - mx);
+        m_ref = mx;
+        l *= factor;
       }
+      if (moved || !AHEAD) exponentials(m_ref == -INFINITY ? 0.f : -m_ref);     // a row that has seen no key yet: a finite stand-in
       l += sum;
       // O is touched only to rescale it, and then the product of the step before must have updated it
       const bool rescale = i > 0 && moved;
