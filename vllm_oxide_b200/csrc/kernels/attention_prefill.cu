@@ -162,8 +162,8 @@ attention_prefill_kernel(const __nv_bfloat16* q, long q_stride, __nv_bfloat16* o
 
 #if VOB_HD % 64 == 0
 // ---- the same attention with TMA copies, 128 rows per block and 64 keys per softmax step ----------------
-// For head sizes that are a multiple of 64 (head sizes 64 and 128 normally take the tcgen05 kernel of
-// attention_prefill_tc5.cu instead).  Eight consumer warps own 16 rows each (128 rows: twice the reuse of every key
+// For head sizes that are a multiple of 64, where a call does not have what the tcgen05 kernel of attention_prefill_tc5.cu needs (its
+// aligned queries and output; heads of 192 and 256 also a positive scale and up to 128 heads a group).  Eight consumer warps own 16 rows each (128 rows: twice the reuse of every key
 // and value brought in); a ninth warp is the producer: its lanes look the pages of eight tiles up at once, a chunk
 // ahead, and one thread issues one TMA copy of K and one of V per tile (per run of 16 keys when pages do not hold
 // a multiple of 64), into a ring of stages guarded by mbarriers with bounded waits.  A consumer multiplies

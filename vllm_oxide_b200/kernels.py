@@ -1004,11 +1004,12 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
                       softcap: float = 0.0, chunk: int = 0, value_div: int = 1, keep_first: int = 0, dist_bias=None,
                       portions: int = 0, portion_tokens: int = 0) -> None:
     """Requests that bring more than one token; the others are skipped.  `portions` and `portion_tokens`: how many such requests there
-    are and their tokens, where the caller knows (the tcgen05 kernel then launches no block for the other requests).  Head sizes 64, 128, 192 and 256 run on the tcgen05
-    tensor cores (`use_tc5`; `tiles_by_tma` False makes that kernel bring its query tiles in by cp.async and store its
-    output row by row also where TMA could), other multiples of 64 on mma.sync with TMA copies (`use_tma`), the rest with
-    cp.async.  `sink`, `gate`, `gate_stride`, `softcap`, `chunk`: as for paged_attention_generic; `value_div`: as for
-    attention_decode.  `keep_first`, `dist_bias`: as for paged_attention_generic; all three kernels take them."""
+    are and their tokens, where the caller knows (the tcgen05 kernel then launches no block for the other requests).  Head sizes 64,
+    128, 192 and 256 run on the tcgen05 tensor cores (`use_tc5`; `tiles_by_tma` False makes that kernel bring its query tiles in by
+    cp.async and store its output row by row also where TMA could).  Their calls with a query stride that is no multiple of 8, and for
+    heads of 192 and 256 also those with addresses or a scale that the kernel does not take, run on mma.sync with TMA copies
+    (`use_tma`); other head sizes with cp.async.  `sink`, `gate`, `gate_stride`, `softcap`, `chunk`: as for paged_attention_generic;
+    `value_div`: as for attention_decode.  `keep_first`, `dist_bias`: as for paged_attention_generic; all three kernels take them."""
     _cuda(q, out, kcache, vcache, block_tables, cu_q, context_lens, gate, dist_bias)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape[0] == nh)
     assert q.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and (gate is None or gate.dtype == torch.bfloat16)
@@ -1020,7 +1021,12 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
         bs = kcache.shape[2]
         keys, slices = L.vob_attention_decode_box_keys(bs), L.vob_attention_decode_box_slices(bs)
         map_k, map_v = tensor_map(kcache.view(-1, hd), keys, slices), tensor_map(vcache.view(-1, hd), keys, slices)
-        if use_tc5 and L.vob_attention_prefill_has_tc5() and q_stride % 8 == 0:
+        # (what the tcgen05 kernel's 16-byte loads, 32-byte stores and tiles of whole tokens need; for heads of up to 128 its entry
+        # reports a call that does not have it)
+        fits = hd <= 128 or (out.data_ptr() % 32 == 0 and q.data_ptr() % 16 == 0 and scale > 0 and nh // kvh <= 128)
+        if use_tc5 and L.vob_attention_prefill_has_tc5() and q_stride % 8 == 0 and fits:
+            if not portions:
+                portions, portion_tokens = num_requests, out.shape[0]      # the most there can be
             # the query tiles come and whole output tiles leave by TMA too (a tile holds whole tokens: 128 // group of them)
             box_heads = L.vob_attention_prefill_q_box_heads(nh, kvh) if tiles_by_tma else 0
             map_q = tensor_map_heads(q, q_stride, nh, hd, box_heads, 128 // box_heads) if box_heads > 0 else None
