@@ -78,3 +78,13 @@ def test_logits_of_many_rows(M, N, K):
     got, want = held[:M].cpu(), x.double() @ w.double().T
     assert torch.equal(got, got.bfloat16().float())
     assert ((got.double() - want).abs() <= 2 ** -8 * want.abs() + 2e-5).all()
+
+
+def test_which_logits_go_by_this_kernel():
+    """The rule: wide matrices and rounds of items that leave many SMs idle are the library's, small or full ones this kernel's."""
+    from vllm_oxide_b200 import kernels
+    pays = lambda rows, vocab, width: kernels.logits_tc5_pays(torch.empty(rows, width, dtype=torch.bfloat16, device=DEV),
+                                                              torch.empty(vocab, width, dtype=torch.bfloat16, device=DEV))
+    assert pays(1357, 32768, 2048) and pays(512, 32768, 2048) and pays(256, 32768, 4096) and pays(1024, 4096, 1024)
+    assert not pays(256, 4096, 2048) and not pays(384, 32768, 4096) and not pays(1024, 32768, 8192)
+    assert not pays(512, 32768, 2044)             # a width that is no multiple of 8

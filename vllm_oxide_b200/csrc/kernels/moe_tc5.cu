@@ -286,6 +286,20 @@ static int mt_resident_clusters(KERNEL kernel) {
 // Rows of the box of the sorted rows' tensor map.
 VOB_API int vob_moe_tc5_row_box() { return MT_BOX; }
 
+// Whether logits of `rows` rows go by this kernel rather than by the library's product and the pass that turns its bfloat16 into float.
+// That pass costs the same for every width while this kernel's product is the slower one (1.1 to 1.2 PFLOP/s against 1.3 to 1.5), more so where the
+// last round of items leaves pairs of SMs idle: the wider the matrix, the fuller the rounds must be.  Measured on B200, the library's
+// time over this kernel's, at widths of 1,024 / 2,048 / 4,096 / 5,120 / 8,192: 1,024 rows of a vocabulary of 32,768 (97 % full): 2.1, 2.1, 1.4,
+// 1.3, 1.0; 384 rows (65 %): 1.4, 1.2, 0.97, 0.94, 0.8; 256 rows of 151,936 (89 %): 2.1, 1.8, 1.4, 1.4, 1.3; 384 (71 %): 1.6, 1.3, 1.03, 0.98,
+// 0.9; 1,024 rows of 4,096 (86 %): 1.4, 1.3, 1.2, 1.2, 1.05; 1,357 (59 %): 1.2, 1.04, 0.9, 0.9, 0.8; 256 (22 %): 1.0, 0.8, 0.6, 0.6, 0.5.
+VOB_API int vob_logits_by_tc5(int rows, int N, int K) {
+  if (rows <= 0 || N <= 0 || K <= 0 || K > 5120) return 0;
+  const long pairs = sm_count() / 2, tiles = (rows + MT_NT - 1) / MT_NT, cols = (N + 2 * MT_ROWS - 1) / (2 * MT_ROWS);
+  const long rounds = ((tiles / 2 + tiles % 2) * cols + pairs - 1) / pairs;
+  const double full = 0.5 * (double)(tiles * cols) / (double)(rounds * pairs);      // (an odd last row tile is half an item's work)
+  return full >= (K <= 2048 ? 0.55 : (K <= 4096 ? 0.7 : 0.84)) ? 1 : 0;
+}
+
 // map_w: tensor map of W [experts * N, K] with box 128 rows; map_x: tensor map of the sorted rows [max_rows, K] with box
 // vob_moe_tc5_row_box() rows (vob_tensor_map_bf16_2d).  out [max_rows, ldo]: bfloat16 with the squared relu (epilogue 0), float (1),
 // bfloat16 SiLU(gate) * up over rows of W in (gate, up) pairs (2: N / 2 columns; with glu_limit > 0 the clamped form

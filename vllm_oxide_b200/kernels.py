@@ -583,6 +583,11 @@ def moe_gemm_tc5(a, w, c, row_token, tile_expert, relu_squared: bool, err, silu_
            "moe_gemm_tc5")
 
 
+def logits_tc5_pays(x, w) -> bool:
+    """Whether logits_tc5 takes x and w and is the shorter way to float logits (else: the library's product and a pass over it)."""
+    return moe_gemm_tc5_supported(x, w) and bool(lib().vob_logits_by_tc5(x.shape[0], w.shape[0], w.shape[1]))
+
+
 def logits_tc5(x, w, out, err) -> None:
     """out[M,N] = x[M,K] @ w[N,K]^T as float, rounded to bfloat16 first, for any number of rows: the experts' product with one expert
     (moe_gemm_tc5_supported says which x and w)."""

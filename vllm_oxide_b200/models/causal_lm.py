@@ -169,9 +169,9 @@ class CausalLM:
             kernels.gemm_skinny(normed, self.lm_head, out, kernels.EPI_F32, ctx.err)   # rounds to bfloat16, stores float
         elif tc5_product(normed, self.lm_head, out, kernels.EPI_F32, ctx):
             pass
-        elif kernels.moe_gemm_tc5_supported(normed, self.lm_head):
-            # more rows than those two take: the product of this package that stores float itself (the library's bfloat16
-            # result takes another pass: 1,357 rows x 32,768 of width 2048, 126 + 118 us, 167 here)
+        elif R > 128 and kernels.logits_tc5_pays(normed, self.lm_head):
+            # more rows than those two take, where the product of this package that stores float itself is the shorter way (the
+            # library's bfloat16 result takes another pass)
             kernels.logits_tc5(normed, self.lm_head, out, ctx.err)
         else:
             out.copy_(linear(normed, self.lm_head, ctx.ws.get_rows("logits", R, V, self.dtype), ctx))
