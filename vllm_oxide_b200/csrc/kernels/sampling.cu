@@ -18,6 +18,7 @@
 namespace vob {
 
 constexpr int SAMPLE_THREADS = 1024;
+constexpr int SAMPLE_TOP_K = SAMPLE_THREADS / 16 * 15;      // the most that top-k gathers by the threads' maxima
 constexpr int SAMPLE_CANDIDATES = 4096;    // tokens that top-p may still keep after one look at the row, held in shared memory
 
 __device__ __forceinline__ uint32_t ordered_key(float x) {
@@ -157,16 +158,17 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
 
   // ---- top-k: key of the k-th largest scaled logit (0 keeps everything)
   // A token among the k largest is at least as large as the k-th largest of the threads' own maxima (k of them are tokens).  So
-  // the first look at the row only takes maxima, the second gathers the tokens from that bound on, few more than k, into shared
-  // memory, and everything after (the digits of the exact threshold, the maximum, top-p, the draw) runs over them alone.  (A
-  // histogram of the row's keys, which did this before, is bound by atomics to a handful of bins: 48 rows of 151,936 took 139 us
-  // with top-k 50 and top-p 0.9, 39 with the maxima.)
-  // More than SAMPLE_THREADS tokens asked for, or too many at the bound: the first digit (sign and most of the exponent) is found by
-  // a histogram over the row, and the tokens whose first digit is at least that of the k-th largest are gathered if they are few.
+  // the first look at the row only takes maxima, the second gathers the tokens from that bound on into shared memory, and
+  // everything after (the digits of the exact threshold, the maximum, top-p, the draw) runs over them alone: some
+  // -1024 ln(1 - k / 1024) tokens of a long row, 51 for k = 50, 2,839 for 960.  (48 rows of 151,936 with top-k 50 and top-p 0.9: 39 us;
+  // 139 by the histogram alone, which is bound by atomics to a handful of bins.)
+  // More than SAMPLE_TOP_K asked for, or more than half of the threads' maxima equal to the bound (a masked vocabulary with fewer
+  // than k tokens left: every masked token is at the bound): the first digit (sign and most of the exponent) is found by a histogram
+  // over the row, and the tokens whose first digit is at least that of the k-th largest are gathered if they are few.
   uint32_t thr = 0;
   bool gathered = false;
   if (k >= 1 && k < V) {
-    if (k <= SAMPLE_THREADS) {
+    if (k <= SAMPLE_TOP_K) {
       uint32_t most = 0;
       each_logit(l, V, [&](float x, int) { most = max(most, ordered_key(x * inv_t)); });
       uint32_t bound = 0;
@@ -174,17 +176,20 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
         const uint32_t higher = bound | (1u << bit);
         if (__syncthreads_count(most >= higher) >= k) bound = higher;
       }
-      if (tid == 0) s_ncand = 0;
-      __syncthreads();
-      each_logit(l, V, [&](float x, int i) {
-        const uint32_t key = ordered_key(x * inv_t);
-        if (key >= bound) {
-          const unsigned pos = atomicAdd(&s_ncand, 1u);
-          if (pos < (unsigned)SAMPLE_CANDIDATES) { cand_key[pos] = key; cand_idx[pos] = (uint32_t)i; }
-        }
-      });
-      __syncthreads();
-      gathered = s_ncand <= (unsigned)SAMPLE_CANDIDATES;
+      // (a bound of 0: fewer threads than that have a token, and the row is short)
+      if (__syncthreads_count(most == bound) <= SAMPLE_THREADS / 2 || bound == 0) {
+        if (tid == 0) s_ncand = 0;
+        __syncthreads();
+        each_logit(l, V, [&](float x, int i) {
+          const uint32_t key = ordered_key(x * inv_t);
+          if (key >= bound) {
+            const unsigned pos = atomicAdd(&s_ncand, 1u);
+            if (pos < (unsigned)SAMPLE_CANDIDATES) { cand_key[pos] = key; cand_idx[pos] = (uint32_t)i; }
+          }
+        });
+        __syncthreads();
+        gathered = s_ncand <= (unsigned)SAMPLE_CANDIDATES;
+      }
     }
     __syncthreads();
     if (tid == 0) { s_prefix = 0; s_remaining_k = (unsigned)k; s_gather = 0; }
