@@ -218,3 +218,43 @@ def test_a_slot_out_of_range_is_reported():
     kernels.lightning_scan(rows, one, torch.zeros(2, 256, device=DEV), torch.tensor([0, 20], dtype=torch.int32, device=DEV),
                            torch.tensor([2], dtype=torch.int32, device=DEV), torch.zeros(20, 16, device=DEV), 1, 1, 16, 16, err, by_chunks=True)
     assert int(err.item()) == 4      # VOB_ERR_SLOT
+
+
+@pytest.mark.parametrize("kind", ["lightning", "mlstm"])
+def test_a_layer_beside_decoding_requests_goes_by_chunks(kind, monkeypatch):
+    """A portion of 500 tokens beside 24 requests that decode: the layer takes the chunks by the rule, every request goes on from its own
+    state, and what follows (decoding, by the walk) finds the states that the chunks left."""
+    from helpers import Alone, assert_close, held, rand
+    from plain import laruzen_plain, nesezen_plain
+    from test_gpu_nesezen_parts import draw, hold, load
+    from vllm_oxide_b200 import kernels
+    from vllm_oxide_b200.parts import PartSpec, build_part
+    dt, D, eps, sizes = torch.bfloat16, 40, 1e-5, dict(num_heads=3, dim=128, vdim=128)
+    if kind == "lightning":
+        part = build_part("mixer", PartSpec("lightning_attention", dict(hidden_size=D, decay=[0.999, 0.9, 0.5], eps=eps, prefix="m.", **sizes)), dtype=dt,
+                          device=DEV)
+    else:
+        part = build_part("mixer", PartSpec("mlstm", dict(hidden_size=D, gate_cap=6.0, eps=eps, prefix="m.", **sizes)), dtype=dt, device=DEV)
+    w = draw(part, 17)
+    load(part, w, dt)
+    wh, ways = hold(part, w, dt), []
+    name = kind + "_scan"
+    scan = getattr(kernels, name)
+    monkeypatch.setattr(kernels, name, lambda *a, **k: (ways.append(bool(k.get("by_chunks"))), scan(*a, **k))[1])
+    alone = Alone([part], dt, block_size=16, pages=80, slots=25)
+    xs = {rid: held(rand((506 if rid == 24 else 9, D), 60 + rid), dt) for rid in range(25)}
+    got = {rid: [] for rid in xs}
+    for step in ([(rid, 0, 6) for rid in range(24)], [(rid, 6, 7) for rid in range(24)] + [(24, 0, 500)], [(rid, 7, 8) for rid in range(24)] + [(24, 500, 501)],
+                 [(24, 501, 506)] + [(rid, 8, 9) for rid in range(24)]):
+        out, at = alone.step([(rid, xs[rid][a:b]) for rid, a, b in step])[0], 0
+        for rid, a, b in step:
+            got[rid].append(out[at:at + b - a])
+            at += b - a
+    assert ways[1] and not ways[2], ways
+    m = dict(heads=3, dim=128, vdim=128)
+    for rid, x in xs.items():
+        if kind == "lightning":
+            want = laruzen_plain.lightning(x, wh, "m.", dict(m, decay=[0.999, 0.9, 0.5]), eps, torch.float64)
+        else:
+            want = nesezen_plain.mlstm(x, wh, "m.", dict(m, gate_cap=6.0), eps, torch.float64, noise=lambda t: held(t, dt))
+        assert_close(torch.cat(got[rid]), want, dt, f"{kind}, request {rid}", 0.04)
