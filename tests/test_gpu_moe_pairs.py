@@ -88,3 +88,32 @@ def test_which_logits_go_by_this_kernel():
     assert pays(1357, 32768, 2048) and pays(512, 32768, 2048) and pays(256, 32768, 4096) and pays(1024, 4096, 1024)
     assert not pays(256, 4096, 2048) and not pays(384, 32768, 4096) and not pays(1024, 32768, 8192)
     assert not pays(512, 32768, 2044)             # a width that is no multiple of 8
+
+
+@pytest.mark.parametrize("kind,N,K,tiles", [("float", 8200, 72, [6, 5, 5]), ("relu2", 4096, 136, [16, 1, 17]), ("pairs", 2048, 2048, [25, 24, 23]),
+                                            ("float", 300, 64, [200, 201]), ("pairs", 520, 64, [300])])
+def test_items_of_two_tiles_and_of_one(kind, N, K, tiles):
+    """Steps with so many items that two tiles of an expert share one (the last: too little to multiply, so none do): the 64-bit products,
+    and rows that name no token left alone."""
+    from vllm_oxide_b200 import kernels
+    E, rows = len(tiles), 128 * (sum(tiles) + 2)
+    g = torch.Generator(device=DEV).manual_seed(N)
+    a = torch.randn(rows, K, generator=g, device=DEV).bfloat16()
+    w = (torch.randn(E, N, K, generator=g, device=DEV) / K ** 0.5).bfloat16()
+    owner = torch.cat([torch.full((128 * n,), e) for e, n in enumerate(tiles)] + [torch.full((256,), -1)]).int().to(DEV)
+    token = torch.where((owner >= 0) & (torch.rand(rows, generator=g, device=DEV) < 0.9), torch.arange(rows, device=DEV).int(), -1)
+    gated = kind == "pairs"
+    out = torch.full((rows, N // 2 if gated else N), -7.0, dtype=torch.float32 if kind == "float" else torch.bfloat16, device=DEV)
+    err = torch.zeros(1, dtype=torch.int32, device=DEV)
+    kernels.moe_gemm_tc5(a, w, out, token, owner[::64].contiguous(), kind == "relu2", err, silu_pairs=gated)
+    assert int(err.item()) == 0 and (out[token < 0] == -7.0).all()
+    for e in range(E):
+        at = (owner == e) & (token >= 0)
+        want = a[at].double() @ w[e].double().T
+        if kind == "relu2":
+            want = want.clamp(min=0) ** 2
+        elif gated:
+            want = torch.nn.functional.silu(want[:, 0::2]) * want[:, 1::2]
+        # float sums of up to 2,048 products of order 1 / sqrt(K): 2e-5; one rounding to bfloat16 behind them: 2^-8 of the value
+        tol = 2e-5 if kind == "float" else 2 ** -8 * want.abs() + 2e-5
+        assert ((out[at].double() - want).abs() <= tol).all()

@@ -4,8 +4,9 @@
 //
 // The step's (token, choice) pairs lie sorted by expert (moe.cu: moe_align), every expert's rows padded to a tile of 128,
 // so a row tile belongs to one expert: C[rows of the tile] = f(A[rows] W_e^T) with W stacked [experts * N, K].  The weights are the
-// operand of 256 rows: a work item is 256 rows of W_e against the rows of two neighbouring row tiles of one expert, or of one where
-// its neighbour is another expert's.  A cluster of two blocks, one per SM, shares an item (cta_group::2): each brings 128 rows of W
+// operand of 256 rows: a work item is 256 rows of W_e against the rows of two row tiles of one expert, or of one where the step has
+// none to join (tiles 2 i and 2 i + 1 are joined, so one at an odd place whose right neighbour is the same expert's stays alone) or too
+// few items for it to pay.  A cluster of two blocks, one per SM, shares an item (cta_group::2): each brings 128 rows of W
 // and half of the item's rows, and holds the 128 x 256 accumulators of its rows of W; the tensor cores read the other half of the
 // rows from the neighbour's shared memory.  What bounds the product is bringing operands in: an SM brings 32 KB per
 // 128 x 256 x 64 products, where blocks of their own with 128 x 128 accumulators brought 32 KB per 128 x 128 x 64.
@@ -53,7 +54,7 @@ template <int EPI>
 __global__ void __launch_bounds__(MT_THREADS, 1)
 moe_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ CUtensorMap tmX, void* out, long ldo,
                const int* row_token, const float* row_weight, const int* tile_expert, int first_tile, int row_tiles, int rows, int N,
-               int K, float glu_limit, int* err) {
+               int K, float glu_limit, float pair_cost, int* err) {
   constexpr int S = MT_S, STAGE_BYTES = MT_STAGE_BYTES;
   constexpr int ACC_COLS = 2 * MT_NT, TMEM_COLS = 2 * ACC_COLS;
   extern __shared__ __align__(1024) char smem_raw[];
@@ -85,11 +86,26 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
   pdl_wait();                       // which items exist, and the rows themselves, come from the kernels ahead
   auto expert_of = [&](int tile) { return tile >= row_tiles ? -1 : (tile_expert ? tile_expert[(first_tile + tile) * (MT_NT / 64)] : 0); };
   if (warp == 2) {
+    // An item of two tiles takes as long as `pair_cost` items of one, so it pays where it saves rounds of items enough: the rounds
+    // at the items' mean, the last one at a pair's.
+    int live = 0, joined = 0;
+    for (int mt = 2 * lane; mt < row_tiles; mt += 64) {
+      const int e0 = expert_of(mt), e1 = expert_of(mt + 1);
+      live += (e0 >= 0) + (e1 >= 0);
+      joined += e0 >= 0 && e1 == e0;
+    }
+    live = __reduce_add_sync(0xffffffffu, live);
+    joined = __reduce_add_sync(0xffffffffu, joined);
+    const unsigned clusters = gridDim.x / 2;
+    const unsigned rounds = ((unsigned)live * n_tiles + clusters - 1) / clusters, rounds_joined = ((unsigned)(live - joined) * n_tiles + clusters - 1) / clusters;
+    const float mean = 1.f + (pair_cost - 1.f) * (float)joined / (float)max(live - joined, 1);
+    const bool join = joined > 0 && (float)(rounds_joined - 1) * mean + pair_cost <= (float)rounds;
     int count = 0;
     for (int p0 = 0; 2 * p0 < row_tiles; p0 += 32) {
       const int mt = 2 * (p0 + lane);
       const int e0 = expert_of(mt), e1 = expert_of(mt + 1);
-      const int mine = (e0 >= 0) + (e1 >= 0 && e1 != e0);
+      const bool both = join && e1 == e0;
+      const int mine = (e0 >= 0) + (e1 >= 0 && !both);
       int upto = mine;
 #pragma unroll
       for (int d = 1; d < 32; d <<= 1) {
@@ -97,8 +113,8 @@ moe_tc5_kernel(const __grid_constant__ CUtensorMap tmW, const __grid_constant__ 
         if (lane >= d) upto += v;
       }
       int at = count + upto - mine;
-      if (e0 >= 0) units[at++] = (uint16_t)(mt * 2 + (e1 == e0));
-      if (e1 >= 0 && e1 != e0) units[at] = (uint16_t)((mt + 1) * 2);
+      if (e0 >= 0) units[at++] = (uint16_t)(mt * 2 + both);
+      if (e1 >= 0 && !both) units[at] = (uint16_t)((mt + 1) * 2);
       count += __shfl_sync(0xffffffffu, upto, 31);
     }
     if (lane == 0) *num_units = count;
@@ -314,6 +330,14 @@ VOB_API int vob_moe_gemm_tc5(const void* map_w, const void* map_x, void* out, lo
       (row_token && max_rows % MT_NT))
     return VOB_BAD_ARGUMENT;
   const int all_tiles = (max_rows + MT_NT - 1) / MT_NT;
+  // What an item of two row tiles costs in items of one: less than the sum, for the rows of W are brought in once; the activation's
+  // epilogue, which hides behind the next item's products, is twice as long and shows at small K.  Measured on B200 over 8, 16 and 64
+  // experts and 64 to 4,001 tokens, in us with two tiles an item, with one, and by the rule: SiLU of 3,072 x 2,048, 16 experts, 1,000 tokens of 4
+  // choices: 98, 94, 94; 4,001: 228, 279, 228; of 512 x 1,024, 8 experts, 2,048 of 2: 35, 27, 27; of 6,144 x 4,096, 16 experts, 1,000 of 4:
+  // 280, 296, 280; no activation, 4,096 x 3,072, 4,001 of 4: 334, 494, 334; 2,048 x 768, 8 experts, 1,000 of 2: 29, 23, 23.
+  float pair_cost = 1.2f;
+  if (epilogue == MT_EPI_SILU_PAIRS_BF16) pair_cost = 0.8f + 2048.f / (float)K;
+  pair_cost = pair_cost < 1.2f ? 1.2f : (pair_cost > 2.f ? 2.f : pair_cost);
 #define VOB_MT(EPI)                                                                                                        \
   do {                                                                                                                     \
     static int resident = 0;                                                                                               \
@@ -331,7 +355,7 @@ VOB_API int vob_moe_gemm_tc5(const void* map_w, const void* map_x, void* out, lo
       const int code = launch_kernel_cluster(moe_tc5_kernel<EPI>, dim3(2 * pairs), MT_THREADS,                             \
                                              MT_SMEM + (2 * tiles + 15) / 16 * 16, stream, 2u, *(const CUtensorMap*)map_w, \
                                              *(const CUtensorMap*)map_x, out, ldo, row_token, row_weight, tile_expert,     \
-                                             first, tiles, max_rows, N, K, glu_limit, err);                                \
+                                             first, tiles, max_rows, N, K, glu_limit, pair_cost, err);                                \
       if (code != 0) return code;                                                                                          \
     }                                                                                                                      \
     return 0;                                                                                                              \
