@@ -523,8 +523,8 @@ VOB_API int vob_attention_prefill_tma(const void* map_k, const void* map_v, cons
 // rules for the scores: `softcap` > 0 (a score becomes softcap * tanh(score / softcap)), `chunk` > 0 (a query sees the
 // keys of its own block of `chunk` positions; `window` is then not looked at), `value_div` > 1 (the value plane has
 // kvh / value_div heads and key head k reads value head k / value_div), `out_float` (out is float), `keep_first` > 0 (the
-// keys at positions below it are seen whatever the window) and `dist_bias` (float [dist_rows, nh]: a bias by the distance
-// between query and key): both mma.sync kernels take the last two, the tcgen05 kernel does not.
+// keys at positions below it are seen whatever the window) and `dist_bias` (float [nh, dist_rows]: a bias by the distance
+// between query and key).
 VOB_API int vob_attention_prefill_ex(const void* map_k, const void* map_v, const void* q, long q_stride, void* out,
                                      const void* kcache, const void* vcache, const int* block_tables, int table_stride,
                                      const int* cu_q, const int* context_lens, int num_requests, int max_q, int nh,

@@ -29,10 +29,11 @@
 // softmax thread that has to rescale O at step i waits on it for step i - 1, when it can be in two states only (that
 // product pending or done: the next one needs this thread's own P).  At the end it could be in three (the last two
 // products pending, the last one, none), so the end of a tile's last product has a barrier of its own, used once.
-// O stays in tensor memory over all steps.  The running maximum that the exponentials refer to is moved only when a
-// row's new maximum exceeds it by more than 8 (in base-2 units: P stays below 256, exact enough in bfloat16 since
-// its error is relative); only then the row's O is read, scaled and written back, which is rare after the first
-// steps.  Sums, maxima and the scaling are in float.  Every wait on an mbarrier is bounded; a block that gives up
+// O stays in tensor memory over all steps.  For heads of up to 128 the running maximum that the exponentials refer to is
+// moved only when a row's new maximum exceeds it by more than 8 (in base-2 units: P stays below 256, its error in
+// bfloat16 is relative); only then the row's O is read, scaled and written back, which is rare after the first
+// steps.  For larger heads it is the maximum itself (see F5_MAX_SLACK), and the search for it comes before the
+// exponentials.  Sums, maxima and the scaling are in float.  Every wait on an mbarrier is bounded; a block that gives up
 // sets an error bit, stops issuing work, waits for what is in flight, and frees its tensor memory.
 #define VOB_TIMEOUT_WHERE 0x1000
 #include "attention_mma.cuh"
@@ -70,9 +71,9 @@ template <int NQ, bool ONE_PLANE> struct F5 {
 
 // The block's place among the step's portions.  The blocks of the requests that bring more than one token (`per` tokens a block)
 // are numbered request after request; a warp sums the requests' counts 32 at a time until it has passed number `blk`.  So a
-// step of few portions among many decoding requests launches blocks for the portions alone: with a grid of (longest portion) x
-// (requests), a step of 5 portions beside 224 decoding requests launched 14,656 blocks of which 176 had work, and the empty
-// ones, each an SM to itself for its shared memory, cost 94 us a layer (28 layers, heads 16 over 8 of 128: 11.58 ms a step, now 8.96).
+// step of few portions among many decoding requests launches blocks for the portions alone.  (An empty block too waits for the
+// shared memory of an SM: a grid of the longest portion times the requests has 14,656 blocks for 5 portions beside 224 decoding
+// requests, 176 of them with work, and takes 94 us longer; 16 heads over 8 of 128.)
 struct PortionBlock { int b, t0, n, tok_base; };
 
 __device__ __forceinline__ bool find_portion(const int* __restrict__ cu_q, int num_requests, int blk, int per, int lane, PortionBlock& at) {
@@ -416,8 +417,8 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
         }
         if (need_mask) {
           // Columns from `from` to `to` are seen, and those below `kept`: comparisons with numbers and nothing that a branch guards.
-          // (With the bias's test inside, and a tile that ends inside a request masked throughout, 1,000 tokens of 16 heads over 8 took
-          // 74 us, 23 so; 2,048 of 32 heads over 8 took 61, 46 so; the same bits.)
+          // (1,000 tokens of 16 heads over 8 of 128: 23 us; 74 with a test for the bias in this loop and with tiles that end inside a
+          // request masked throughout.  2,048 of 32 heads over 8: 46 and 61.)
           const int to = valid ? rpos - k0 : -1, from = row_lo - k0, kept = ep.keep_first - k0;
 #pragma unroll
           for (int c = 0; c < 64; ++c) s[c] = (c <= to) & ((c >= from) | (c < kept)) ? s[c] : -INFINITY;

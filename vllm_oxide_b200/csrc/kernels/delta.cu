@@ -349,7 +349,8 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
   // this thread's rows of its column: seg, seg + LANES, ... (row r of the thread is row seg + LANES * r of the head), two to a
   // 64-bit register: a multiply-add instruction serves both.  A token is a chain: the dot product with k, its exchange between the
   // column's lanes, the update.  What the next token needs from shared memory is on its way meanwhile, and the read-out's exchange
-  // runs beside the next token's: 742 us a portion of 2,048 tokens (16 heads of 128 x 128) before, 505 so, the same bits.
+  // runs beside the next token's.  (A portion of 2,048 tokens, 16 heads of 128 x 128: 505 us; 742 with a row an instruction and one
+  // exchange behind the other.  The same sums in the same order.)
   f32x2 S[ROWS / 2];
   // (the slot keeps a head's matrix column by column, [vdim][dim]: the LANES threads of a column then read neighbours)
   float* mine = state + (size_t)slot * state_stride + ((size_t)h * vdim + col) * dim;

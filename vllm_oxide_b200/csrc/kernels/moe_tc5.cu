@@ -10,8 +10,8 @@
 // and half of the item's rows, and holds the 128 x 256 accumulators of its rows of W; the tensor cores read the other half of the
 // rows from the neighbour's shared memory.  What bounds the product is bringing operands in: an SM brings 32 KB per
 // 128 x 256 x 64 products, where blocks of their own with 128 x 128 accumulators brought 32 KB per 128 x 128 x 64.
-// B200, 16,004 pairs of 16 experts, 4096 -> 2 x 3072 -> 4096: 1,009 + 543 us by such blocks, 689 + 347 here, 1.17 PFLOP/s; same
-// bits, the order of a sum along K has not changed.
+// B200, 16,004 pairs of 16 experts, 4096 -> 2 x 3072 -> 4096: 689 + 347 us here, 1.17 PFLOP/s; 1,009 + 543 by such blocks.  A sum
+// runs along K in order, whatever its item is shared with.
 // The blocks are persistent; a warp of each lists the step's items first (which exist is only known on the device), row tile major,
 // so that clusters side by side share an expert's matrix in L2.
 //   warp 0      producer: per 64 columns of K one TMA copy of the W tile [128 x 64] and one or two of the rows [64 x 64]

@@ -1,8 +1,10 @@
 // Recurrent token mixers: the state of a request is carried in float from token to token, in a state slot.
 //
-// Both kernels walk the tokens of one request in order, whatever the step holds of it (a whole prompt, a portion, one
-// decoded token), starting from the slot's state and leaving the new state there.  The chain of float operations of a
-// channel therefore depends on the request's tokens only: not on how they were cut into steps nor on the batch.
+// The kernels take the tokens of one request in order, whatever the step holds of it (a whole prompt, a portion, one
+// decoded token), starting from the slot's state and leaving the new state there.  A walk in one range is one chain of float
+// operations a channel, which depends on the request's tokens only: not on how they were cut into steps nor on the batch.  A
+// portion that is cut into ranges (the rules below look at the step's tokens and requests), and in bfloat16 a portion of lightning
+// attention or mLSTM by chunks, adds the same terms in another order, so its last bits depend on those.
 // Projections come in the model's type T (bfloat16 when serving); gates, decays, the state and the norm are float.
 #include "chunk_scan.cuh"
 

@@ -974,7 +974,8 @@ def attention_decode(q, q_stride, out, kcache, vcache, block_tables, cu_q, conte
     run as persistent blocks that draw their pairs from it (the kernel leaves it at zero), without it as one block per
     pair.  Same bits either way.  `sink`, `gate`, `gate_stride`, `softcap`, `chunk`: as for paged_attention_generic.
     `value_div` > 1: `vcache` has kvh // value_div heads, and key head k reads value head k // value_div.  `out` is
-    bfloat16 or float32.  `keep_first`, `dist_bias`: as for paged_attention_generic (with either, a block a pair).  A float tensor [nh] as `sink` as there."""
+    bfloat16 or float32.  `keep_first`, `dist_bias`: as for paged_attention_generic (with either, a block a pair).  A float tensor
+    [nh] as `sink` as there."""
     sink, sinks = _sinks(sink, nh)
     _cuda(q, out, kcache, vcache, block_tables, cu_q, context_lens, scratch, pairs, gate, dist_bias)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape[0] == nh)

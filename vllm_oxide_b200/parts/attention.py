@@ -260,8 +260,8 @@ def paged_attend(q, q_stride, out, keys, values, group: int, ctx, T: int, nh: in
 FAST_SINK_AND_GATE = True
 # Whether they take capped scores, blocks of positions and values with fewer heads than keys (else the plain kernel does).
 FAST_CAP_AND_CHUNK = True
-# Whether they take kept first keys beside a window and a bias by distance (else the plain kernel does): the mma.sync
-# kernels do, for every head size they are built for.
+# Whether they take kept first keys beside a window and a bias by distance (else the plain kernel does): all of them do, for
+# every head size they are built for.
 FAST_KEEP_AND_BIAS = True
 
 DECODE_BLOCKS_PER_SM = 2   # blocks of the decode attention kernel that fit an SM (its shared memory decides)
