@@ -782,8 +782,12 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
   dim3 grid(num_splits, kvh, num_requests);
   int rc;
 #if VOB_HD % 64 == 0
-  if (map_k && map_v && block_size % 16 == 0) {
-    const int extras = ep.keep_first || ep.dist_bias;
+  const int extras = ep.keep_first || ep.dist_bias;
+  // Heads of 192 leave one block of this kernel on an SM (its registers), two of the cp.async kernel, which answers these calls where there
+  // are more blocks than SMs (24 requests of 600 keys, 4 heads, 3 splits: 21 us, 29 here; 40, 1 head, 4 splits: 23 and 30; 8 requests, 4
+  // splits, fit: 14 and 9).
+  const bool second_places = HD == 192 && extras && (long)num_splits * kvh * num_requests > sm_count() && (num_splits == 1 || scratch);
+  if (map_k && map_v && block_size % 16 == 0 && !second_places) {
     auto kernel = extras ? attention_decode_tma_kernel<true> : attention_decode_tma_kernel<false>;
     static bool tma_configured[2] = {false, false};
     constexpr int MERGE = (2 * DEC_WARPS * 16 + DEC_WARPS * 16 * HD) * 4 + (16 * HD + 16) * 4;
