@@ -224,8 +224,10 @@ constexpr int DS_THREADS = DS_COMPUTE + DS_LOADERS;
 // walk the tokens, CH at a time from one of two buffers in shared memory, while four more warps fill the other buffer:
 // unit vectors (laid out so that a thread finds its rows side by side), decay, beta and the block's slice of the values.
 // The two groups meet on named barriers: "full" when a buffer is ready, "empty" when its tokens have been walked.
-template <typename T, int LANES, int ROWS, bool CHD>
-__global__ void __launch_bounds__(DS_THREADS)
+// AHEAD: a token's rows are asked for while the token before is worked on; without it a thread takes a quarter fewer registers and
+// three blocks share an SM, which is what many requests of one or few tokens wait for (their states come from memory).
+template <typename T, int LANES, int ROWS, bool CHD, bool AHEAD>
+__global__ void __launch_bounds__(DS_THREADS, !AHEAD && ROWS == 16 ? 3 : 1)
 delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int a_off, const float* __restrict__ A_log,
                   const float* __restrict__ dt_bias, float* state, long state_stride, const int* __restrict__ cu_q,
                   const int* __restrict__ state_slots, float* raw, int heads, int kvh, int dim, int vdim, long num_slots,
@@ -294,8 +296,8 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
           gs[i] = expf(neg_rate * sp);
         }
       }
-      // the sums of squares of all tokens side by side (one after the other they are a chain of forty exchanges); then one lane a sum
-      // takes its root and quotient
+      // The sums of squares of all tokens side by side (one after the other they are a chain of forty exchanges); then one lane a sum
+      // takes its root and quotient.  With a token or two a request only those that there are, below.
       float sums[2 * TPW];
 #pragma unroll
       for (int tt = 0; tt < TPW; ++tt) {
@@ -306,18 +308,23 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
           sums[2 * tt + 1] = fmaf(kv[tt][j], kv[tt][j], sums[2 * tt + 1]);
         }
       }
+      float unit = 0.f;
+      if (AHEAD) {
 #pragma unroll
-      for (int o = 16; o > 0; o >>= 1)
+        for (int o = 16; o > 0; o >>= 1)
 #pragma unroll
-        for (int r = 0; r < 2 * TPW; ++r) sums[r] += __shfl_xor_sync(0xffffffffu, sums[r], o);
-      float sum = sums[0];
+          for (int r = 0; r < 2 * TPW; ++r) sums[r] += __shfl_xor_sync(0xffffffffu, sums[r], o);
+        float sum = sums[0];
 #pragma unroll
-      for (int r = 1; r < 2 * TPW; ++r) sum = lane % (2 * TPW) == r ? sums[r] : sum;
-      const float unit = (lane & 1 ? 1.f : qscale) / sqrtf(sum + 1e-6f);
+        for (int r = 1; r < 2 * TPW; ++r) sum = lane % (2 * TPW) == r ? sums[r] : sum;
+        unit = (lane & 1 ? 1.f : qscale) / sqrtf(sum + 1e-6f);
+      }
 #pragma unroll
       for (int tt = 0; tt < TPW; ++tt) {
         const int i = lw + tt * (DS_LOADERS / 32);
-        const float iq = __shfl_sync(0xffffffffu, unit, 2 * tt), ik = __shfl_sync(0xffffffffu, unit, 2 * tt + 1);
+        if (!AHEAD && i >= n) continue;
+        const float iq = AHEAD ? __shfl_sync(0xffffffffu, unit, 2 * tt) : qscale / sqrtf(warp_sum(sums[2 * tt]) + 1e-6f);
+        const float ik = AHEAD ? __shfl_sync(0xffffffffu, unit, 2 * tt + 1) : 1.f / sqrtf(warp_sum(sums[2 * tt + 1]) + 1e-6f);
         if (i >= n) continue;
 #pragma unroll
         for (int j = 0; j < NV; ++j) {
@@ -382,13 +389,21 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
         x[2 * r + 1] = y.y;
       }
     };
-    load_rows(ks, 0, k);
-    if (!CHD) g = gs[0];
-    beta = bs[0];
-    v = vs[colb];
-#pragma unroll 2
+    if (AHEAD) {
+      load_rows(ks, 0, k);
+      if (!CHD) g = gs[0];
+      beta = bs[0];
+      v = vs[colb];
+    }
+#pragma unroll(AHEAD ? 2 : 1)
     for (int i = 0; i < n; ++i) {
       f32x2 q[ROWS / 2], gr[CHD ? ROWS / 2 : 1];
+      if (!AHEAD) {
+        load_rows(ks, i, k);
+        if (!CHD) g = gs[i];
+        beta = bs[i];
+        v = vs[i * COLS + colb];
+      }
       if constexpr (CHD) load_rows(gv, i, gr);
       else gr[0] = pack2(g, g);
       f32x2 a[2] = {0ull, 0ull};
@@ -417,10 +432,12 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
       const int next = min(i + 1, n - 1);
 #pragma unroll
       for (int r = 0; r < ROWS / 2; ++r) S[r] = fma2(k[r], u2, S[r]);
-      load_rows(ks, next, k);
-      if (!CHD) g = gs[next];
-      beta = bs[next];
-      v = vs[next * COLS + colb];
+      if (AHEAD) {
+        load_rows(ks, next, k);
+        if (!CHD) g = gs[next];
+        beta = bs[next];
+        v = vs[next * COLS + colb];
+      }
 #pragma unroll
       for (int r = 0; r < ROWS / 2; ++r) y[r & 1] = fma2(S[r], q[r], y[r & 1]);
       const float2 y01 = unpack2(y[0]), y23 = unpack2(y[1]);
@@ -601,45 +618,51 @@ VOB_API int vob_short_conv_step(const void* x, long x_stride, const float* w, co
 template <typename T>
 static int launch_delta_scan(const float* qkv, const void* ab, long ab_stride, int b_off, int a_off, const float* A_log,
                              const float* dt_bias, float* state, long state_stride, const int* cu_q, const int* state_slots,
-                             float* raw, int B, int heads, int kvh, int dim, int vdim, long num_slots, int channel_decay,
+                             float* raw, long T_all, int B, int heads, int kvh, int dim, int vdim, long num_slots, int channel_decay,
                              int* err, cudaStream_t stream) {
   // rows a thread keeps, and threads a column: the fewest threads whose rows cover the head
   const int rows = dim <= 128 ? 16 : 32;
   const int lanes = dim <= rows ? 1 : (dim <= 2 * rows ? 2 : (dim <= 4 * rows ? 4 : 8));
-#define VOB_DS(L, R)                                                                                                       \
-  if (lanes == L && rows == R) {                                                                                           \
+  // Without AHEAD where more blocks than two an SM have up to eight tokens a request on average (decoding): 64 requests of one token, 16
+  // heads of 128 x 128: 59 us, 75 with; of four: 83 and 95; 16 of sixteen: 47 and 44.
+  const long blocks = (long)((vdim + DS_COMPUTE / lanes - 1) / (DS_COMPUTE / lanes)) * heads * B;
+  const bool ahead = blocks <= 2 * sm_count() || T_all > 8 * (long)B;
+#define VOB_DS_LAUNCH(L, R, D, A)                                                                                          \
+  do {                                                                                                                     \
     constexpr int cols = DS_COMPUTE / L, ch = R > 16 ? 8 : 16;                                                             \
     dim3 grid((vdim + cols - 1) / cols, heads, B);                                                                         \
-    if (channel_decay) {                                                                                                   \
-      const size_t smem = (size_t)2 * ch * (3 * L * (R + 4) + cols + 2) * sizeof(float);                                   \
-      if (smem > 48 * 1024)                                                                                                \
-        cudaFuncSetAttribute(delta_scan_kernel<T, L, R, true>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);    \
-      return launch_kernel(delta_scan_kernel<T, L, R, true>, grid, DS_THREADS, smem, stream, qkv, (const T*)ab, ab_stride, \
-                           b_off, a_off, A_log, dt_bias, state, state_stride, cu_q, state_slots, raw, heads, kvh, dim,     \
-                           vdim, num_slots, err);                                                                          \
-    }                                                                                                                      \
-    const size_t smem = (size_t)2 * ch * (2 * L * (R + 4) + cols + 2) * sizeof(float);                                     \
-    return launch_kernel(delta_scan_kernel<T, L, R, false>, grid, DS_THREADS, smem, stream, qkv, (const T*)ab, ab_stride,  \
+    constexpr size_t smem = (size_t)2 * ch * ((D ? 3 : 2) * L * (R + 4) + cols + 2) * sizeof(float);                       \
+    if (smem > 48 * 1024)                                                                                                  \
+      cudaFuncSetAttribute(delta_scan_kernel<T, L, R, D, A>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);      \
+    return launch_kernel(delta_scan_kernel<T, L, R, D, A>, grid, DS_THREADS, smem, stream, qkv, (const T*)ab, ab_stride,   \
                          b_off, a_off, A_log, dt_bias, state, state_stride, cu_q, state_slots, raw, heads, kvh, dim, vdim, \
                          num_slots, err);                                                                                  \
+  } while (0)
+#define VOB_DS(L, R)                                                                                                       \
+  if (lanes == L && rows == R) {                                                                                           \
+    if (channel_decay && ahead) VOB_DS_LAUNCH(L, R, true, true);                                                           \
+    if (channel_decay) VOB_DS_LAUNCH(L, R, true, false);                                                                   \
+    if (ahead) VOB_DS_LAUNCH(L, R, false, true);                                                                           \
+    VOB_DS_LAUNCH(L, R, false, false);                                                                                     \
   }
   VOB_DS(1, 16) VOB_DS(2, 16) VOB_DS(4, 16) VOB_DS(8, 16) VOB_DS(8, 32)
 #undef VOB_DS
+#undef VOB_DS_LAUNCH
   return VOB_UNSUPPORTED;
 }
 
 VOB_API int vob_delta_scan(const float* qkv, const void* ab, long ab_stride, int b_off, int a_off, const float* A_log,
                            const float* dt_bias, float* state, long state_stride, const int* cu_q, const int* state_slots,
-                           float* raw, int B, int heads, int kvh, int dim, int vdim, long num_slots, int channel_decay,
+                           float* raw, int num_tokens, int B, int heads, int kvh, int dim, int vdim, long num_slots, int channel_decay,
                            int dtype, int* err, cudaStream_t stream) {
   if (B <= 0) return 0;
   if (heads <= 0 || kvh <= 0 || heads % kvh || dim <= 0 || dim > 256 || vdim <= 0 || B > 65535) return VOB_UNSUPPORTED;
   if (dtype == VOB_F32)
     return launch_delta_scan<float>(qkv, ab, ab_stride, b_off, a_off, A_log, dt_bias, state, state_stride, cu_q, state_slots, raw,
-                                    B, heads, kvh, dim, vdim, num_slots, channel_decay, err, stream);
+                                    num_tokens, B, heads, kvh, dim, vdim, num_slots, channel_decay, err, stream);
   if (dtype == VOB_BF16)
     return launch_delta_scan<__nv_bfloat16>(qkv, ab, ab_stride, b_off, a_off, A_log, dt_bias, state, state_stride, cu_q,
-                                            state_slots, raw, B, heads, kvh, dim, vdim, num_slots, channel_decay, err, stream);
+                                            state_slots, raw, num_tokens, B, heads, kvh, dim, vdim, num_slots, channel_decay, err, stream);
   return VOB_BAD_ARGUMENT;
 }
 

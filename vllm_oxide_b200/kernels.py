@@ -493,7 +493,7 @@ def delta_scan(qkv, ab, b_off: int, a_off: int, A_log, dt_bias, state, cu_q, sta
     assert state.dtype == torch.float32 and state.stride(1) == 1 and state.shape[1] >= heads * dim * vdim and ab.stride(1) == 1
     assert dt_bias.numel() == (heads * dim if channel_decay else heads)
     _check(lib().vob_delta_scan(_p(qkv), _p(ab), ctypes.c_long(ab.stride(0)), b_off, a_off, _p(A_log), _p(dt_bias), _p(state),
-                                ctypes.c_long(state.stride(0)), _p(cu_q), _p(state_slots), _p(raw), num_requests, heads, kvh,
+                                ctypes.c_long(state.stride(0)), _p(cu_q), _p(state_slots), _p(raw), raw.shape[0], num_requests, heads, kvh,
                                 dim, vdim, ctypes.c_long(state.shape[0]), int(bool(channel_decay)), _code(ab.dtype), _p(err),
                                 _stream()), "delta_scan")
 
