@@ -218,6 +218,20 @@ constexpr int DS_COMPUTE = 128;   // threads that hold the state
 constexpr int DS_LOADERS = 128;   // threads that prepare the next tokens meanwhile
 constexpr int DS_THREADS = DS_COMPUTE + DS_LOADERS;
 
+// The request of grid layer z, the longest portion first (up to 32 requests; else in the order of the batch): blocks start in the
+// order of the grid, and a long portion that starts late ends late.  Every lane of the warp must call.
+__device__ __forceinline__ int longest_first(const int* __restrict__ cu_q) {
+  const int B = gridDim.z, lane = threadIdx.x & 31;
+  if (B == 1 || B > 32) return blockIdx.z;
+  const int mine = lane < B ? cu_q[lane + 1] - cu_q[lane] : -1;
+  int rank = 0;
+  for (int j = 0; j < B; ++j) {
+    const int other = __shfl_sync(0xffffffffu, mine, j);
+    rank += other > mine || (other == mine && j < lane);
+  }
+  return __ffs(__ballot_sync(0xffffffffu, lane < B && rank == (int)blockIdx.z)) - 1;
+}
+
 // qkv: float [tokens, 2 * kvh * dim + heads * vdim] (q heads, k heads, v heads: the convolutions' output);
 // ab: rows of ab_stride elements of T, beta's pre-activation of head h at b_off + h, the decay's at a_off + h.
 // A column of the state is held by LANES neighbouring threads, ROWS rows each (LANES * ROWS >= dim); 128 such threads
@@ -227,7 +241,7 @@ constexpr int DS_THREADS = DS_COMPUTE + DS_LOADERS;
 // AHEAD: a token's rows are asked for while the token before is worked on; without it a thread takes a quarter fewer registers and
 // three blocks share an SM, which is what many requests of one or few tokens wait for (their states come from memory).
 template <typename T, int LANES, int ROWS, bool CHD, bool AHEAD>
-__global__ void __launch_bounds__(DS_THREADS, !AHEAD && ROWS == 16 ? 3 : 1)
+__global__ void __launch_bounds__(DS_THREADS, ROWS != 16 ? 1 : (!AHEAD ? 3 : (CHD ? 1 : 2)))
 delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int a_off, const float* __restrict__ A_log,
                   const float* __restrict__ dt_bias, float* state, long state_stride, const int* __restrict__ cu_q,
                   const int* __restrict__ state_slots, float* raw, int heads, int kvh, int dim, int vdim, long num_slots,
@@ -239,8 +253,9 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
   constexpr int BUF = CH * ((CHD ? 3 : 2) * KW + COLS + 2);     // CHD: a decay for every row of the head beside k and q
   extern __shared__ __align__(16) float ds_smem[];
   pdl_launch_dependents();
-  const int b = blockIdx.z, h = blockIdx.y, c0 = blockIdx.x * COLS;
+  const int h = blockIdx.y, c0 = blockIdx.x * COLS;
   const int tid = threadIdx.x, lane = tid & 31;
+  const int b = AHEAD ? longest_first(cu_q) : blockIdx.z;
   const int t0 = cu_q[b], t1 = cu_q[b + 1];
   const int slot = state_slots[b];
   const float neg_rate = -expf(A_log[h]), bias = CHD ? 0.f : dt_bias[h];
@@ -354,10 +369,7 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
   const int col = c0 + colb;
   const bool live = col < vdim;
   // this thread's rows of its column: seg, seg + LANES, ... (row r of the thread is row seg + LANES * r of the head), two to a
-  // 64-bit register: a multiply-add instruction serves both.  A token is a chain: the dot product with k, its exchange between the
-  // column's lanes, the update.  What the next token needs from shared memory is on its way meanwhile, and the read-out's exchange
-  // runs beside the next token's.  (A portion of 2,048 tokens, 16 heads of 128 x 128: 505 us; 742 with a row an instruction and one
-  // exchange behind the other.  The same sums in the same order.)
+  // 64-bit register: a multiply-add instruction serves both.
   f32x2 S[ROWS / 2];
   // (the slot keeps a head's matrix column by column, [vdim][dim]: the LANES threads of a column then read neighbours)
   float* mine = state + (size_t)slot * state_stride + ((size_t)h * vdim + col) * dim;
@@ -367,87 +379,149 @@ delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int 
     S[r / 2] = pack2((live && row < dim) ? mine[row] : 0.f, (live && row + LANES < dim) ? mine[row + LANES] : 0.f);
   }
   float* dst = raw + ((size_t)t0 * heads + h) * vdim + col;
-  const size_t dst_step = (size_t)heads * vdim;
-  float o_ = 0.f;                                // this thread's share of the read-out of the token before
-  for (int c = 0; c < chunks; ++c) {
-    const float* ks = ds_smem + (c & 1) * BUF;
-    const float* qs = ks + CH * KW;
-    const float* vs = qs + CH * KW;
-    const float* gs = vs + CH * COLS;
-    const float* bs = gs + CH;
-    const float* gv = bs + CH;
-    const int n = min(CH, t1 - t0 - c * CH);
-    named_sync(1 + (c & 1), DS_THREADS);
-    f32x2 k[ROWS / 2];
-    float g = 1.f, beta, v;
-    auto load_rows = [&](const float* rows, int i, f32x2 (&x)[ROWS / 2]) {
-      const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(rows + i * KW + seg * RS);
+  const long dst_step = (long)heads * vdim;
+  const bool writes = seg == 0 && live;
+  auto load_rows = [&](const float* rows, int i, f32x2 (&x)[ROWS / 2]) {
+    const ulonglong2* x2 = reinterpret_cast<const ulonglong2*>(rows + i * KW + seg * RS);
 #pragma unroll
-      for (int r = 0; r < ROWS / 4; ++r) {
-        const ulonglong2 y = x2[r];
-        x[2 * r] = y.x;
-        x[2 * r + 1] = y.y;
-      }
-    };
-    if (AHEAD) {
-      load_rows(ks, 0, k);
-      if (!CHD) g = gs[0];
-      beta = bs[0];
-      v = vs[colb];
+    for (int r = 0; r < ROWS / 4; ++r) {
+      const ulonglong2 y = x2[r];
+      x[2 * r] = y.x;
+      x[2 * r + 1] = y.y;
     }
-#pragma unroll(AHEAD ? 2 : 1)
-    for (int i = 0; i < n; ++i) {
-      f32x2 q[ROWS / 2], gr[CHD ? ROWS / 2 : 1];
-      if (!AHEAD) {
+  };
+  auto fold = [](const f32x2 (&a)[2]) {          // four partial sums of a thread
+    const float2 a01 = unpack2(a[0]), a23 = unpack2(a[1]);
+    return (a01.x + a01.y) + (a23.x + a23.y);
+  };
+  if constexpr (AHEAD) {
+    // A token is a chain: the decay, the dot product with k, its exchange between the column's lanes, the update.  Everything else runs
+    // beside that exchange: the read-out of the token before (from the registers that the decay has not replaced), the loads
+    // of the next token's rows, and the read-outs' own exchanges, a level a token (o_[e]: a share with e levels done).  Nothing in a
+    // token branches: a branch keeps the compiler from putting these between the exchange's steps (448 us instead of 340).  One
+    // portion of 2,048 tokens, 16 heads of 128 x 128: 340 us, 379 with the read-out in the chain; portions of 333, 1,055 and 1,777: 446 us,
+    // 516 so and in the order of the batch.  The same sums in the same order.
+    constexpr int LEVELS = LANES >= 8 ? 3 : (LANES >= 4 ? 2 : (LANES >= 2 ? 1 : 0));
+    f32x2 k[ROWS / 2], q[ROWS / 2];
+#pragma unroll
+    for (int r = 0; r < ROWS / 2; ++r) q[r] = 0ull;
+    float o_[LEVELS + 1];
+#pragma unroll
+    for (int e = 0; e <= LEVELS; ++e) o_[e] = 0.f;
+    int at = -(LEVELS + 2);                      // the token whose read-out the next pass completes
+    // the tokens' read-outs move on by a level; `share`: this thread's share of the newest
+    auto pass_read_outs = [&](float share) {
+      float in[LEVELS + 1];
+#pragma unroll
+      for (int e = 0; e < LEVELS; ++e) in[e] = __shfl_xor_sync(0xffffffffu, o_[e], 1 << e);
+      const float done = o_[LEVELS];
+#pragma unroll
+      for (int e = LEVELS; e > 0; --e) o_[e] = o_[e - 1] + in[e - 1];
+      o_[0] = share;
+      asm volatile("{\n.reg .pred p;\nsetp.ge.s32 p, %0, 0;\n@p st.global.f32 [%1], %2;\n}\n" ::"r"(writes ? at : -1),
+                   "l"(dst + (long)at * dst_step), "f"(done));
+      ++at;
+    };
+    for (int c = 0; c < chunks; ++c) {
+      const float* ks = ds_smem + (c & 1) * BUF;
+      const float* qs = ks + CH * KW;
+      const float* vs = qs + CH * KW;
+      const float* gs = vs + CH * COLS;
+      const float* bs = gs + CH;
+      const float* gv = bs + CH;
+      const int n = min(CH, t1 - t0 - c * CH);
+      named_sync(1 + (c & 1), DS_THREADS);
+      f32x2 gr[CHD ? ROWS / 2 : 1];
+      float g = 1.f;
+      load_rows(ks, 0, k);
+      if constexpr (CHD) load_rows(gv, 0, gr);
+      else g = gs[0];
+      float beta = bs[0], v = vs[colb];
+#pragma unroll 2
+      for (int i = 0; i < n; ++i) {
+        if constexpr (!CHD) gr[0] = pack2(g, g);
+        f32x2 D[ROWS / 2], a[2] = {0ull, 0ull}, y[2] = {0ull, 0ull};
+#pragma unroll
+        for (int r = 0; r < ROWS / 2; ++r) {
+          D[r] = mul2(S[r], gr[CHD ? r : 0]);
+          a[r & 1] = fma2(D[r], k[r], a[r & 1]);
+        }
+        float dot = fold(a);
+        const float first = LANES > 1 ? __shfl_xor_sync(0xffffffffu, dot, 1) : 0.f;
+#pragma unroll
+        for (int r = 0; r < ROWS / 2; ++r) y[r & 1] = fma2(S[r], q[r], y[r & 1]);
+        load_rows(qs, i, q);
+        // (the last token of a buffer reads its own row again: what follows it comes with the next buffer)
+        const int next = min(i + 1, n - 1);
+        f32x2 k_next[ROWS / 2];
+        load_rows(ks, next, k_next);
+        if constexpr (CHD) load_rows(gv, next, gr);
+        else g = gs[next];
+        const float beta_next = bs[next], v_next = vs[next * COLS + colb];
+        if (LANES > 1) dot += first;
+        pass_read_outs(fold(y));
+#pragma unroll
+        for (int o = 2; o < LANES; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float u = beta * (v - dot);
+        const f32x2 u2 = pack2(u, u);
+#pragma unroll
+        for (int r = 0; r < ROWS / 2; ++r) {
+          S[r] = fma2(k[r], u2, D[r]);
+          k[r] = k_next[r];
+        }
+        beta = beta_next;
+        v = v_next;
+      }
+      if (c + 2 < chunks) named_arrive(3 + (c & 1), DS_THREADS);
+    }
+    f32x2 y[2] = {0ull, 0ull};
+#pragma unroll
+    for (int r = 0; r < ROWS / 2; ++r) y[r & 1] = fma2(S[r], q[r], y[r & 1]);
+    pass_read_outs(fold(y));
+#pragma unroll
+    for (int e = 0; e <= LEVELS; ++e) pass_read_outs(0.f);
+  } else {
+    for (int c = 0; c < chunks; ++c) {
+      const float* ks = ds_smem + (c & 1) * BUF;
+      const float* qs = ks + CH * KW;
+      const float* vs = qs + CH * KW;
+      const float* gs = vs + CH * COLS;
+      const float* bs = gs + CH;
+      const float* gv = bs + CH;
+      const int n = min(CH, t1 - t0 - c * CH);
+      named_sync(1 + (c & 1), DS_THREADS);
+#pragma unroll 1
+      for (int i = 0; i < n; ++i) {
+        f32x2 k[ROWS / 2], q[ROWS / 2], gr[CHD ? ROWS / 2 : 1];
         load_rows(ks, i, k);
-        if (!CHD) g = gs[i];
-        beta = bs[i];
-        v = vs[i * COLS + colb];
-      }
-      if constexpr (CHD) load_rows(gv, i, gr);
-      else gr[0] = pack2(g, g);
-      f32x2 a[2] = {0ull, 0ull};
+        if constexpr (CHD) load_rows(gv, i, gr);
+        else gr[0] = pack2(gs[i], gs[i]);
+        f32x2 a[2] = {0ull, 0ull}, y[2] = {0ull, 0ull};
 #pragma unroll
-      for (int r = 0; r < ROWS / 2; ++r) {
-        S[r] = mul2(S[r], gr[CHD ? r : 0]);
-        a[r & 1] = fma2(S[r], k[r], a[r & 1]);
-      }
-      load_rows(qs, i, q);
-      const float2 a01 = unpack2(a[0]), a23 = unpack2(a[1]);
-      float dot = (a01.x + a01.y) + (a23.x + a23.y);
+        for (int r = 0; r < ROWS / 2; ++r) {
+          S[r] = mul2(S[r], gr[CHD ? r : 0]);
+          a[r & 1] = fma2(S[r], k[r], a[r & 1]);
+        }
+        load_rows(qs, i, q);
+        float dot = fold(a);
 #pragma unroll
-      for (int o = 1; o < LANES; o <<= 1) {
-        const float other = __shfl_xor_sync(0xffffffffu, dot, o), before = __shfl_xor_sync(0xffffffffu, o_, o);
-        dot += other;
-        o_ += before;
-      }
-      if (c + i > 0) {
-        if (seg == 0 && live) *dst = o_;
+        for (int o = 1; o < LANES; o <<= 1) dot += __shfl_xor_sync(0xffffffffu, dot, o);
+        const float u = bs[i] * (vs[i * COLS + colb] - dot);
+        const f32x2 u2 = pack2(u, u);
+#pragma unroll
+        for (int r = 0; r < ROWS / 2; ++r) {
+          S[r] = fma2(k[r], u2, S[r]);
+          y[r & 1] = fma2(S[r], q[r], y[r & 1]);
+        }
+        float o_ = fold(y);
+#pragma unroll
+        for (int o = 1; o < LANES; o <<= 1) o_ += __shfl_xor_sync(0xffffffffu, o_, o);
+        if (writes) *dst = o_;
         dst += dst_step;
       }
-      const float u = beta * (v - dot);
-      const f32x2 u2 = pack2(u, u);
-      f32x2 y[2] = {0ull, 0ull};
-      // (the last token of a buffer reads its own row again: what follows it comes with the next buffer)
-      const int next = min(i + 1, n - 1);
-#pragma unroll
-      for (int r = 0; r < ROWS / 2; ++r) S[r] = fma2(k[r], u2, S[r]);
-      if (AHEAD) {
-        load_rows(ks, next, k);
-        if (!CHD) g = gs[next];
-        beta = bs[next];
-        v = vs[next * COLS + colb];
-      }
-#pragma unroll
-      for (int r = 0; r < ROWS / 2; ++r) y[r & 1] = fma2(S[r], q[r], y[r & 1]);
-      const float2 y01 = unpack2(y[0]), y23 = unpack2(y[1]);
-      o_ = (y01.x + y01.y) + (y23.x + y23.y);
+      if (c + 2 < chunks) named_arrive(3 + (c & 1), DS_THREADS);
     }
-    if (c + 2 < chunks) named_arrive(3 + (c & 1), DS_THREADS);
   }
-#pragma unroll
-  for (int o = 1; o < LANES; o <<= 1) o_ += __shfl_xor_sync(0xffffffffu, o_, o);
-  if (seg == 0 && live) *dst = o_;
 #pragma unroll
   for (int r = 0; r < ROWS; r += 2) {
     const float2 x = unpack2(S[r / 2]);
