@@ -28,47 +28,52 @@ namespace vob {
 constexpr int ATT_WARPS = 4;
 constexpr int ATT_MAXD = 16;  // value dims per lane: hd <= 512
 
+// N neighbouring elements of a row as they are loaded, and element j of them as a float.
+template <typename T> struct RowPiece;
+template <> struct RowPiece<float> {
+  typedef float4 Raw;
+  static constexpr int N = 4;
+  static __device__ __forceinline__ float at(const Raw& r, int j) { return j == 0 ? r.x : (j == 1 ? r.y : (j == 2 ? r.z : r.w)); }
+};
+template <> struct RowPiece<__nv_bfloat16> {
+  typedef uint4 Raw;
+  static constexpr int N = 8;
+  static __device__ __forceinline__ float at(const Raw& r, int j) {
+    const uint32_t w = j < 2 ? r.x : (j < 4 ? r.y : (j < 6 ? r.z : r.w));
+    return __uint_as_float(j & 1 ? w & 0xffff0000u : w << 16);
+  }
+};
+
+// One chain of multiply-adds over the row, eight 16-byte loads in flight.
 template <typename T>
-__device__ __forceinline__ float dot_row(const float* q, const T* k, int hd);
-
-template <>
-__device__ __forceinline__ float dot_row<float>(const float* q, const float* k, int hd) {
+__device__ __forceinline__ float dot_row(const float* q, const T* k, int hd) {
+  using P = RowPiece<T>;
   float s = 0.f;
-  if (hd % 4) {                        // rows that do not start on 16-byte boundaries: element by element
-    for (int i = 0; i < hd; ++i) s += q[i] * k[i];
+  if (hd % P::N) {                     // rows that do not start on 16-byte boundaries: element by element
+    for (int i = 0; i < hd; ++i) s += q[i] * to_f<T>(k[i]);
     return s;
   }
-  const float4* k4 = reinterpret_cast<const float4*>(k);
-  for (int i = 0; i < hd / 4; ++i) {
-    const float4 v = k4[i];
-    s += q[4 * i] * v.x; s += q[4 * i + 1] * v.y; s += q[4 * i + 2] * v.z; s += q[4 * i + 3] * v.w;
-  }
-  return s;
-}
-
-template <>
-__device__ __forceinline__ float dot_row<__nv_bfloat16>(const float* q, const __nv_bfloat16* k,
-                                                         int hd) {
-  float s = 0.f;
-  if (hd % 8) {                        // rows that do not start on 16-byte boundaries: element by element
-    for (int i = 0; i < hd; ++i) s += q[i] * __bfloat162float(k[i]);
-    return s;
-  }
-  const uint4* k8 = reinterpret_cast<const uint4*>(k);
-  for (int i = 0; i < hd / 8; ++i) {
-    const uint4 raw = k8[i];
-    const __nv_bfloat162* h2 = reinterpret_cast<const __nv_bfloat162*>(&raw);
+  const typename P::Raw* pieces = reinterpret_cast<const typename P::Raw*>(k);
+  const int n = hd / P::N;
+  for (int i0 = 0; i0 < n; i0 += 8) {
+    typename P::Raw v[8];
 #pragma unroll
-    for (int j = 0; j < 4; ++j) {
-      const float2 f = __bfloat1622float2(h2[j]);
-      s += q[8 * i + 2 * j] * f.x;
-      s += q[8 * i + 2 * j + 1] * f.y;
-    }
+    for (int e = 0; e < 8; ++e)
+      if (i0 + e < n) v[e] = pieces[i0 + e];
+#pragma unroll
+    for (int e = 0; e < 8; ++e)
+      if (i0 + e < n) {
+#pragma unroll
+        for (int j = 0; j < P::N; ++j) s += q[(i0 + e) * P::N + j] * P::at(v[e], j);
+      }
   }
   return s;
 }
 
-template <typename T>
+// DIMS: value dims a lane holds (a lane has dims lane, lane + 32, ...).  Short prompts are a chain of latencies here, the cache's rows
+// one behind the other; so a tile's value rows are asked for some at a time, by addresses that their lanes have made once.
+// (303 tokens of six prompts, 6 heads of 32, float: 15 us; 44 a row after the other.)
+template <typename T, int DIMS>
 __global__ void __launch_bounds__(ATT_WARPS * 32)
 paged_attention_generic_kernel(const T* q, long q_stride, T* out,
                                const T* kcache, const T* vcache,
@@ -78,6 +83,7 @@ paged_attention_generic_kernel(const T* q, long q_stride, T* out,
                                int window, float scale, long num_pages, int sink, const float* __restrict__ sinks, const T* gate, long gate_stride,
                                int vkvh, int v_row, float softcap, int chunk, int out_float, int keep_first,
                                const float* __restrict__ dist_bias, int dist_rows, int* err) {
+  constexpr int AHEAD = DIMS > 4 ? 32 / DIMS : 8;      // value rows in flight
   extern __shared__ float smem[];
   float* qs = smem;                        // [hd]
   float* accs = smem + hd;                 // [ATT_WARPS][vd]
@@ -100,9 +106,9 @@ paged_attention_generic_kernel(const T* q, long q_stride, T* out,
   const int* table = block_tables + (size_t)req * table_stride;
 
   float m = -INFINITY, l = 0.f;
-  float acc[ATT_MAXD];
+  float acc[DIMS];
 #pragma unroll
-  for (int j = 0; j < ATT_MAXD; ++j) acc[j] = 0.f;
+  for (int j = 0; j < DIMS; ++j) acc[j] = 0.f;
 
   // kept first keys: the tiles that hold them are walked too, the ones between them and the window are passed over
   const int keep = min(max(keep_first, 0), lo);
@@ -111,12 +117,14 @@ paged_attention_generic_kernel(const T* q, long q_stride, T* out,
     if (tile * 32 >= keep && tile * 32 + 31 < lo) continue;
     const int key = tile * 32 + lane;
     const bool valid = (key >= lo || key < keep) && key <= pos;
-    long row = -1;  // element offset of this key's row for kv head kh
-    int page = -1;
+    long row = -1, vrow = -1;  // element offsets of this key's row and value row
     if (valid) {
-      page = table[key / block_size];
-      if (page < 0 || page >= num_pages) { atomicOr(err, VOB_ERR_PAGE); page = -1; }
-      else row = (((long)page * kvh + kh) * block_size + key % block_size) * (long)hd;
+      const int page = table[key / block_size], place = key % block_size;
+      if (page < 0 || page >= num_pages) atomicOr(err, VOB_ERR_PAGE);
+      else {
+        row = (((long)page * kvh + kh) * block_size + place) * (long)hd;
+        vrow = (((long)page * vkvh + vh) * block_size + place) * (long)v_row;
+      }
     }
     float s = -INFINITY;
     if (row >= 0) {
@@ -129,23 +137,32 @@ paged_attention_generic_kernel(const T* q, long q_stride, T* out,
     const float corr = (m == -INFINITY) ? 0.f : expf(m - m_new);
     l = l * corr + warp_sum(p);
 #pragma unroll
-    for (int j = 0; j < ATT_MAXD; ++j) acc[j] *= corr;
-    for (int kk = 0; kk < 32; ++kk) {
-      const int pg = __shfl_sync(0xffffffffu, page, kk);
-      if (pg < 0) continue;
-      const float pk = __shfl_sync(0xffffffffu, p, kk);
-      const T* vrow = vcache + (((long)pg * vkvh + vh) * block_size + (tile * 32 + kk) % block_size) * (long)v_row;
+    for (int j = 0; j < DIMS; ++j) acc[j] *= corr;
+    for (int k0 = 0; k0 < 32; k0 += AHEAD) {
+      float v[AHEAD][DIMS];
+      long at[AHEAD];
 #pragma unroll
-      for (int j = 0; j < ATT_MAXD; ++j) {
-        const int d = lane + 32 * j;
-        if (d < vd) acc[j] += pk * to_f<T>(vrow[d]);
+      for (int kk = 0; kk < AHEAD; ++kk) {
+        at[kk] = __shfl_sync(0xffffffffu, vrow, k0 + kk);
+#pragma unroll
+        for (int j = 0; j < DIMS; ++j) {
+          const int d = lane + 32 * j;
+          v[kk][j] = at[kk] >= 0 && d < vd ? to_f<T>(vcache[at[kk] + d]) : 0.f;
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < AHEAD; ++kk) {
+        const float pk = __shfl_sync(0xffffffffu, p, k0 + kk);
+        if (at[kk] < 0) continue;
+#pragma unroll
+        for (int j = 0; j < DIMS; ++j) acc[j] += pk * v[kk][j];
       }
     }
     m = m_new;
   }
   if (lane == 0) { ms[warp] = m; ls[warp] = l; }
 #pragma unroll
-  for (int j = 0; j < ATT_MAXD; ++j) {
+  for (int j = 0; j < DIMS; ++j) {
     const int d = lane + 32 * j;
     if (d < vd) accs[warp * vd + d] = acc[j];
   }
@@ -203,16 +220,22 @@ VOB_API int vob_paged_attention_generic(const void* q, long q_stride, void* out,
     return VOB_UNSUPPORTED;
   dim3 grid(T, nh);
   const size_t smem = (size_t)(hd + ATT_WARPS * vd) * sizeof(float);
-  if (dtype == VOB_F32)
-    return launch_kernel(paged_attention_generic_kernel<float>, grid, ATT_WARPS * 32, smem, stream, (const float*)q, q_stride,
-                         (float*)out, (const float*)kcache, (const float*)vcache, block_tables, table_stride, token_req,
-                         positions, skip_single_cu_q, nh, kvh, hd, vd, block_size, window, scale, num_pages, sink, sinks,
-                         (const float*)gate, gate_stride, vkvh, v_row, softcap, chunk, out_float, keep_first, dist_bias, dist_rows, err);
-  if (dtype == VOB_BF16)
-    return launch_kernel(paged_attention_generic_kernel<__nv_bfloat16>, grid, ATT_WARPS * 32, smem, stream,
-                         (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, (const __nv_bfloat16*)kcache,
-                         (const __nv_bfloat16*)vcache, block_tables, table_stride, token_req, positions, skip_single_cu_q,
-                         nh, kvh, hd, vd, block_size, window, scale, num_pages, sink, sinks, (const __nv_bfloat16*)gate,
-                         gate_stride, vkvh, v_row, softcap, chunk, out_float, keep_first, dist_bias, dist_rows, err);
+#define VOB_GA(TT, DIMS)                                                                                                              \
+  return launch_kernel(paged_attention_generic_kernel<TT, DIMS>, grid, ATT_WARPS * 32, smem, stream, (const TT*)q, q_stride, (TT*)out, \
+                       (const TT*)kcache, (const TT*)vcache, block_tables, table_stride, token_req, positions, skip_single_cu_q, nh, kvh, \
+                       hd, vd, block_size, window, scale, num_pages, sink, sinks, (const TT*)gate, gate_stride, vkvh, v_row, softcap,  \
+                       chunk, out_float, keep_first, dist_bias, dist_rows, err)
+#define VOB_GA_TYPE(TT)            \
+  do {                             \
+    if (vd <= 32) VOB_GA(TT, 1);   \
+    if (vd <= 64) VOB_GA(TT, 2);   \
+    if (vd <= 128) VOB_GA(TT, 4);  \
+    if (vd <= 256) VOB_GA(TT, 8);  \
+    VOB_GA(TT, ATT_MAXD);          \
+  } while (0)
+  if (dtype == VOB_F32) VOB_GA_TYPE(float);
+  if (dtype == VOB_BF16) VOB_GA_TYPE(__nv_bfloat16);
+#undef VOB_GA_TYPE
+#undef VOB_GA
   return VOB_BAD_ARGUMENT;
 }

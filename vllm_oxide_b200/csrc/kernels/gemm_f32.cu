@@ -26,16 +26,27 @@ gemm_f32_kernel(const float* A, long lda, const float* __restrict__ W, long ldw,
 #pragma unroll
     for (int j = 0; j < 4; ++j) acc[i][j] = 0.f;
 
-  // each thread loads 4 elements of A and 4 of W per slice: row = tid / 4, k = (tid % 4) * 4 .. +3
+  // each thread loads 4 elements of A and 4 of W per slice: row = tid / 4, k = (tid % 4) * 4 .. +3; the next slice's are on their
+  // way while a slice is multiplied
   const int lr = tid / 4, lk = (tid % 4) * 4;
-  for (int k0 = 0; k0 < K; k0 += GK) {
+  const int am = m0 + lr, wn = n0 + lr;
+  float a_next[4], w_next[4];
+  auto fetch = [&](int k0) {
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
       const int k = k0 + lk + j;
-      const int am = m0 + lr, wn = n0 + lr;
-      As[lk + j][lr] = (am < M && k < K) ? A[(size_t)am * lda + k] : 0.f;
-      Ws[lk + j][lr] = (wn < N && k < K) ? W[(size_t)wn * ldw + k] : 0.f;
+      a_next[j] = (am < M && k < K) ? A[(size_t)am * lda + k] : 0.f;
+      w_next[j] = (wn < N && k < K) ? W[(size_t)wn * ldw + k] : 0.f;
     }
+  };
+  fetch(0);
+  for (int k0 = 0; k0 < K; k0 += GK) {
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      As[lk + j][lr] = a_next[j];
+      Ws[lk + j][lr] = w_next[j];
+    }
+    if (k0 + GK < K) fetch(k0 + GK);
     __syncthreads();
 #pragma unroll
     for (int k = 0; k < GK; ++k) {
