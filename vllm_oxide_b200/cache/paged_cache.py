@@ -19,7 +19,7 @@ from typing import List, Optional
 
 import torch
 
-from .. import host
+from .. import host, kernels
 from ..parts.base import CachePlane, CacheSpec, StateSpec
 
 
@@ -101,9 +101,13 @@ class PagedCache:
         return any(s is not None for s in self.states)
 
     def zero_states(self, slots: List[int]) -> None:
-        if not slots:
+        """Zeros in these slots of every state: on the device by one launch that the host does not wait for."""
+        kept = [s for s in self.states if s is not None and s.numel()]
+        if not slots or not kept:
+            return
+        if kept[0].is_cuda:
+            kernels.clear_states(kept, slots)
             return
         idx = torch.as_tensor(slots, dtype=torch.long, device=self.device)
-        for s in self.states:
-            if s is not None:
-                s.index_fill_(0, idx, 0)
+        for s in kept:
+            s.index_fill_(0, idx, 0)

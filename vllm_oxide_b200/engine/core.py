@@ -122,14 +122,21 @@ class EngineCore:
         if self._copied is not None:
             self._copied.synchronize()   # the previous step's copy has left the pinned buffer
         counts = fill(layout)
-        fresh = [int(s) for s, f in zip(self._host_np[layout.state_slots:layout.state_slots + counts.num_requests],
-                                        self._host_np[layout.state_fresh:layout.state_fresh + counts.num_requests]) if f]
-        self.cache.zero_states(fresh)
+        self._zero_fresh_states(layout, counts)
         self._dev_buf[:layout.total].copy_(self._host_buf[:layout.total], non_blocking=True)
         if self._copied is not None:
             self._copied.record()
         self.h2d_bytes_last = layout.total * 4
         return StepContext(layout, self._dev_buf, self._host_np, counts, self.ws, self.err)
+
+    def _zero_fresh_states(self, layout, counts) -> None:
+        """The state slots of requests that begin with this step (before the copy of the step's arrays, behind which its kernels run)."""
+        if not self.cache.has_states:
+            return
+        n = counts.num_requests
+        fresh = self._host_np[layout.state_fresh:layout.state_fresh + n] != 0
+        if fresh.any():
+            self.cache.zero_states(self._host_np[layout.state_slots:layout.state_slots + n][fresh].tolist())
 
     # ---- decode steps from CUDA graphs
     def _graph_bucket(self, entries) -> Optional[int]:
@@ -148,10 +155,7 @@ class EngineCore:
             self._copied.synchronize()
         counts = fill(g.layout)
         L = g.layout
-        if self.cache.has_states:
-            fresh = [int(s) for s, f in zip(self._host_np[L.state_slots:L.state_slots + counts.num_requests],
-                                            self._host_np[L.state_fresh:L.state_fresh + counts.num_requests]) if f]
-            self.cache.zero_states(fresh)
+        self._zero_fresh_states(L, counts)
         if g.host_view is None:
             g.host_view, g.dev_view = self._host_buf[:L.total], g.dev[:L.total]
         g.dev_view.copy_(g.host_view, non_blocking=True)

@@ -1248,6 +1248,21 @@ def apply_penalties(logits, row_of, token, count, presence, frequency, repetitio
            "apply_penalties")
 
 
+def clear_states(states, slots) -> None:
+    """Zeros in the given slots (a list of ints) of every tensor [slots, ...] in `states`; nothing is copied to the device."""
+    _cuda(*states)
+    for t in states:
+        if not t.is_contiguous():
+            raise KernelError("states must be contiguous: a slot is one piece of memory")
+    n, m = len(states), len(slots)
+    if n == 0 or m == 0 or any(t.numel() == 0 for t in states):
+        raise KernelError("nothing to clear: states and slots must not be empty")
+    longs = ctypes.c_long * n
+    _check(lib().vob_clear_states((ctypes.c_ulonglong * n)(*[t.data_ptr() for t in states]),
+                                  longs(*[t.numel() // t.shape[0] * t.element_size() for t in states]),
+                                  longs(*[t.shape[0] for t in states]), n, (ctypes.c_int * m)(*slots), m, _stream()), "clear_states")
+
+
 def copy_pages(cache_plane, pairs, n_pairs: int) -> None:
     _cuda(cache_plane, pairs)
     page_elems = cache_plane[0].numel()
