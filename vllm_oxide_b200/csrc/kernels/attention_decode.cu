@@ -182,8 +182,27 @@ constexpr int DT_THREADS = (DEC_WARPS + 1) * 32;
 
 // EXTRAS: kept first keys or a bias by distance.  (An instance of its own: the map of the keys costs a plain step's layer a
 // microsecond, 1 % of a decode step of Qwen3-8B's sizes at batch 8.)
-template <bool EXTRAS>
-__global__ void __launch_bounds__(DT_THREADS)
+// SHARED: keys and values are one plane (heads of 192 and 256: a latent), whose tiles are brought in and held once.
+// STAGES, QUERIES in shared memory and BLOCKS an SM go together: see DecodeShape.
+template <bool EXTRAS, bool SHARED, bool DENSE> struct DecodeShape {
+  // A block of heads of 192 or 256 needs its registers for the outputs: queries that lie in shared memory leave room for a second one
+  // on the SM, where tiles are held once or heads are 192 (two stages of 48 KB each fit).  DENSE: heads of 128 with extras in two
+  // stages and with queries in shared memory, three blocks an SM, where there are more blocks than two an SM: they would begin a
+  // second round.  (At most 168 registers where two are to fit: the five warps of a block lie unevenly over the SM's quarters.)
+  // Measured on B200 with a cold L2, before and after: a latent of 256, 16 heads, 40 requests of 1,500 to 2,300 keys 53 -> 39 us, 24 of 700 to
+  // 2,100 41 -> 30, of 192 49 -> 32, heads of 192 with 8 x 2, 8 requests 33 -> 23; kept keys and a bias, 8 kv heads of 128, 40 requests of
+  // 1,088 keys 66 -> 48.
+  static constexpr bool QUERIES = HD >= 192 || DENSE;
+  static constexpr int TILE = DT_TILE_BYTES, STAGE = SHARED ? TILE : 2 * TILE;
+  static constexpr int STAGES = DENSE ? 2 : (SHARED ? 3 : DT_STAGES);
+  static constexpr int BLOCKS = DENSE ? 3 : (HD < 192 ? 0 : (SHARED || HD == 192 ? 2 : 1));      // (0: the compiler's choice)
+  static constexpr int MERGE = (2 * DEC_WARPS * 16 + DEC_WARPS * 16 * HD) * 4, FINAL = (16 * HD + 16) * 4;
+  static constexpr int DATA = STAGES * STAGE > MERGE + FINAL ? STAGES * STAGE : MERGE + FINAL;
+  static constexpr int SMEM = 1024 + DATA + (QUERIES ? 16 * Q_ROW_BYTES : 0) + 2 * STAGES * 8 + 32;
+};
+
+template <bool EXTRAS, bool SHARED, bool DENSE>
+__global__ void __launch_bounds__(DT_THREADS, DecodeShape<EXTRAS, SHARED, DENSE>::BLOCKS)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                             const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                             const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
@@ -192,19 +211,20 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             int box_keys, int cluster, int* err, HeadEpilogue ep) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
-  constexpr int MERGE_BYTES = (2 * DEC_WARPS * 16 + DEC_WARPS * 16 * HD) * 4;
-  constexpr int FINAL_BYTES = (16 * HD + 16) * 4;
-  constexpr int DATA_BYTES = DT_STAGES * DT_STAGE_BYTES > MERGE_BYTES + FINAL_BYTES ? DT_STAGES * DT_STAGE_BYTES : MERGE_BYTES + FINAL_BYTES;
-  uint64_t* full = reinterpret_cast<uint64_t*>(smem + DATA_BYTES);
-  uint64_t* empty = full + DT_STAGES;
-  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + DT_STAGES);
+  using SHAPE = DecodeShape<EXTRAS, SHARED, DENSE>;
+  constexpr int STAGES = SHAPE::STAGES, STAGE_BYTES = SHAPE::STAGE, MERGE_BYTES = SHAPE::MERGE;
+  constexpr bool QUERIES = SHAPE::QUERIES;
+  char* qrows = smem + SHAPE::DATA;                           // [16] rows of the group's queries, where they are kept here
+  uint64_t* full = reinterpret_cast<uint64_t*>(qrows + (QUERIES ? 16 * Q_ROW_BYTES : 0));
+  uint64_t* empty = full + STAGES;
+  volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + STAGES);
   pdl_launch_dependents();
   const int split = blockIdx.x, num_splits = gridDim.x, kh = blockIdx.y, b = blockIdx.z;
   const int t = cu_q[b];
   const int t_next = cu_q[b + 1], context = context_lens[b];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (threadIdx.x == 0) {
-    for (int s = 0; s < DT_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], DEC_WARPS); }
+    for (int s = 0; s < STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], DEC_WARPS); }
     *abort_flag = 0;
     tma_prefetch_map(&tmK);
     tma_prefetch_map(&tmV);
@@ -242,18 +262,18 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       bool ok = true, waited = false;
       int it = 0;
       for (; it < n_tiles; ++it) {
-        const int s = it % DT_STAGES;
+        const int s = it % STAGES;
         wp.advance(table, block_size, start, it, lane, lo, EXTRAS ? pos + 1 : end, km, keep);
         int pg[4];
 #pragma unroll
         for (int run = 0; run < 4; ++run) pg[run] = wp.page(it, run);
         if (lane == 0) {
-          if (it >= DT_STAGES) ok = mbar_wait(&empty[s], (unsigned)(((it / DT_STAGES) - 1) & 1), abort_flag, err);
+          if (it >= STAGES) ok = mbar_wait(&empty[s], (unsigned)(((it / STAGES) - 1) & 1), abort_flag, err);
           if (ok) {
             const int tile_start = km.real(start + it * DEC_TILE);
             if (!waited && tile_start + DEC_TILE > pos) { pdl_wait(); waited = true; }
-            mbar_expect_tx(&full[s], (unsigned)DT_STAGE_BYTES);
-            char* kt = smem + s * DT_STAGE_BYTES;
+            mbar_expect_tx(&full[s], (unsigned)STAGE_BYTES);
+            char* kt = smem + s * STAGE_BYTES;
             if (box_keys == DEC_TILE) {
               // the tile lies in one page: one copy of K, one of V (any run that is wanted names the page)
               const int page = pg[0] != PAGE_NONE ? pg[0] : (pg[1] != PAGE_NONE ? pg[1] : (pg[2] != PAGE_NONE ? pg[2] : pg[3]));
@@ -262,7 +282,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
               const int row = page_ok ? (page * kvh + kh) * block_size + tile_start % block_size : 0;
                 const int vrow = page_ok ? (page * value_heads(kvh, ep) + value_head(kh, ep)) * block_size + tile_start % block_size : 0;
               tma_load_3d(kt, &tmK, 0, row, 0, &full[s]);
-              tma_load_3d(kt + DT_TILE_BYTES, &tmV, 0, vrow, 0, &full[s]);
+              if (!SHARED) tma_load_3d(kt + DT_TILE_BYTES, &tmV, 0, vrow, 0, &full[s]);
             } else {
 #pragma unroll
               for (int run = 0; run < 4; ++run) {
@@ -276,7 +296,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 #pragma unroll
                 for (int c = 0; c < DT_SLICES; ++c) {
                   tma_load_3d(kt + c * DEC_TILE * 128 + run * RUN_KEYS * 128, &tmK, 0, row, c, &full[s]);
-                  tma_load_3d(kt + DT_TILE_BYTES + c * DEC_TILE * 128 + run * RUN_KEYS * 128, &tmV, 0, vrow, c, &full[s]);
+                  if (!SHARED) tma_load_3d(kt + DT_TILE_BYTES + c * DEC_TILE * 128 + run * RUN_KEYS * 128, &tmV, 0, vrow, c, &full[s]);
                 }
               }
             }
@@ -286,10 +306,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
         if (!ok) break;
       }
       if (lane == 0) {
-        const int first = it > DT_STAGES ? it - DT_STAGES : 0;     // copies in flight must land before the block exits
+        const int first = it > STAGES ? it - STAGES : 0;     // copies in flight must land before the block exits
         for (int j = first; j < it; ++j) {
           bool done = false;
-          for (unsigned i = 0; i < MBAR_SPIN_LIMIT && !done; ++i) done = mbar_try_wait(&full[j % DT_STAGES], (unsigned)((j / DT_STAGES) & 1));
+          for (unsigned i = 0; i < MBAR_SPIN_LIMIT && !done; ++i) done = mbar_try_wait(&full[j % STAGES], (unsigned)((j / STAGES) & 1));
           if (!done) atomicOr(err, VOB_ERR_TIMEOUT_BITS);
         }
       }
@@ -298,8 +318,20 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
     pdl_wait();
     const int g = lane >> 2, tq = lane & 3;
-    uint32_t qf[KSTEPS][4];
-    {
+    uint32_t qf[QUERIES ? 1 : KSTEPS][4];
+    if constexpr (QUERIES) {
+      for (int i = threadIdx.x; i < 16 * (HD / 8); i += DEC_WARPS * 32) {
+        const int r = i / (HD / 8), d = i % (HD / 8) * 8;
+        uint4 x = make_uint4(0u, 0u, 0u, 0u);
+        if (r < G) {
+          const __nv_bfloat16* src = q + (size_t)t * q_stride + (size_t)(kh * G + r) * HD + d;
+          const uint32_t* s2 = reinterpret_cast<const uint32_t*>(src);      // (rows start on four bytes: q_stride is even)
+          x = make_uint4(s2[0], s2[1], s2[2], s2[3]);
+        }
+        *reinterpret_cast<uint4*>(qrows + r * Q_ROW_BYTES + d * 2) = x;
+      }
+      named_sync(1, DEC_WARPS * 32);
+    } else {
       const __nv_bfloat16* qrow0 = q + (size_t)t * q_stride + (size_t)(kh * G + g) * HD;
       const __nv_bfloat16* qrow1 = qrow0 + (size_t)8 * HD;
 #pragma unroll
@@ -316,16 +348,17 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     const float* brow8 = EXTRAS ? dist_row(ep, kh * G + g + 8, nh) : nullptr;
     const int last_dist = ep.dist_rows - 1;
     for (int it = 0; it < n_tiles; ++it) {
-      const int s = it % DT_STAGES;
-      bool ok = mbar_wait(&full[s], (unsigned)((it / DT_STAGES) & 1), abort_flag, err);
+      const int s = it % STAGES;
+      bool ok = mbar_wait(&full[s], (unsigned)((it / STAGES) & 1), abort_flag, err);
       ok = __all_sync(0xffffffffu, ok);
       if (!ok) break;
-      const char* kt = smem + s * DT_STAGE_BYTES;
+      const char* kt = smem + s * STAGE_BYTES;
       const int v0 = start + it * DEC_TILE + warp * 16;      // virtual; a run of 16 keys lies on one side of the map's seam
       const int k0 = km.real(v0);
       if (v0 < end && (k0 + 16 > lo || k0 < keep)) {
         float sv[2][4];
-        qk_16keys_swizzled<DEC_TILE>(qf, kt, warp * 16, lane, sv);
+        if constexpr (QUERIES) qk_16keys_swizzled<DEC_TILE>(qrows, kt, warp * 16, lane, sv);
+        else qk_16keys_swizzled<DEC_TILE>(qf, kt, warp * 16, lane, sv);
 #pragma unroll
         for (int i = 0; i < 2; ++i) {
           const int key = k0 + i * 8 + tq * 2, vkey = v0 + i * 8 + tq * 2;
@@ -342,7 +375,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
             sv[i][3] += dist_term(brow8, max(d - 1, 0), last_dist);
           }
         }
-        softmax_pv_16keys_swizzled<DEC_TILE>(st, sv, kt + DT_TILE_BYTES, warp * 16, lane);
+        softmax_pv_16keys_swizzled<DEC_TILE>(st, sv, SHARED ? kt : kt + DT_TILE_BYTES, warp * 16, lane);
       }
       // ordinary loads of the stage before the copy engine's next write to it: a proxy fence, then the release
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
@@ -379,17 +412,42 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     }
   }
   __syncthreads();
+  // a row's maximum, its warps' weights and the sum: once a row where there are many outputs, else where an output is made
+  constexpr bool ROW_FIRST = HD >= 192;
+  if constexpr (ROW_FIRST) {
+    if (threadIdx.x < G) {
+      const int r = threadIdx.x;
+      float M = -INFINITY, L = 0.f;
+#pragma unroll
+      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, wm[w * 16 + r]);
+#pragma unroll
+      for (int w = 0; w < DEC_WARPS; ++w) {
+        const float f = wm[w * 16 + r] == -INFINITY ? 0.f : fast_exp2(wm[w * 16 + r] - M);
+        L += wl[w * 16 + r] * f;
+        wm[w * 16 + r] = f;
+      }
+      wl[r] = L;
+      wl[16 + r] = M;
+    }
+    __syncthreads();
+  }
   for (int idx = threadIdx.x; idx < G * HD; idx += DT_THREADS) {
     const int r = idx / HD, d = idx % HD;
-    float M = -INFINITY;
+    float M = -INFINITY, L = 0.f, O = 0.f;
+    if constexpr (ROW_FIRST) {
+      L = wl[r];
+      M = wl[16 + r];
 #pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, wm[w * 16 + r]);
-    float L = 0.f, O = 0.f;
+      for (int w = 0; w < DEC_WARPS; ++w) O += wo[((size_t)w * 16 + r) * HD + d] * wm[w * 16 + r];
+    } else {
 #pragma unroll
-    for (int w = 0; w < DEC_WARPS; ++w) {
-      const float f = wm[w * 16 + r] == -INFINITY ? 0.f : fast_exp2(wm[w * 16 + r] - M);
-      L += wl[w * 16 + r] * f;
-      O += wo[((size_t)w * 16 + r) * HD + d] * f;
+      for (int w = 0; w < DEC_WARPS; ++w) M = fmaxf(M, wm[w * 16 + r]);
+#pragma unroll
+      for (int w = 0; w < DEC_WARPS; ++w) {
+        const float f = wm[w * 16 + r] == -INFINITY ? 0.f : fast_exp2(wm[w * 16 + r] - M);
+        L += wl[w * 16 + r] * f;
+        O += wo[((size_t)w * 16 + r) * HD + d] * f;
+      }
     }
     const float val = L > 0.f ? O / L : 0.f;
     const float lse = (L > 0.f && !aborted) ? M + log2f(L) : -INFINITY;
@@ -788,15 +846,29 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
   // splits, fit: 14 and 9).
   const bool second_places = HD == 192 && extras && (long)num_splits * kvh * num_requests > sm_count() && (num_splits == 1 || scratch);
   if (map_k && map_v && block_size % 16 == 0 && !second_places) {
-    auto kernel = extras ? attention_decode_tma_kernel<true> : attention_decode_tma_kernel<false>;
-    static bool tma_configured[2] = {false, false};
-    constexpr int MERGE = (2 * DEC_WARPS * 16 + DEC_WARPS * 16 * HD) * 4 + (16 * HD + 16) * 4;
-    constexpr int DATA = DT_STAGES * DT_STAGE_BYTES > MERGE ? DT_STAGES * DT_STAGE_BYTES : MERGE;
-    const int tma_smem = 1024 + DATA + 2 * DT_STAGES * 8 + 32;
-    if (!tma_configured[extras]) {
+    // one plane for keys and values: a map of either, no head offset between them
+    const bool shared = HD >= 192 && kcache == vcache && ep.value_div == 1;
+    const bool dense = HD == 128 && extras && (long)num_splits * kvh * num_requests > 2 * sm_count();
+    const int form = extras + 2 * shared + 4 * dense;
+    static bool tma_configured[8] = {};
+    auto kernel = attention_decode_tma_kernel<false, false, false>;
+    int tma_smem = DecodeShape<false, false, false>::SMEM;
+#define VOB_FORM(X, S, D)                              \
+  if (form == (X) + 2 * (S) + 4 * (D)) {               \
+    kernel = attention_decode_tma_kernel<X, S, D>;     \
+    tma_smem = DecodeShape<X, S, D>::SMEM;             \
+  }
+    VOB_FORM(true, false, false)
+#if VOB_HD >= 192
+    VOB_FORM(false, true, false) VOB_FORM(true, true, false)
+#elif VOB_HD == 128
+    VOB_FORM(true, false, true)
+#endif
+#undef VOB_FORM
+    if (!tma_configured[form]) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
       if (e != cudaSuccess) return (int)e;
-      tma_configured[extras] = true;
+      tma_configured[form] = true;
     }
     const int box_keys = block_size % DEC_TILE == 0 ? DEC_TILE : RUN_KEYS;
     // one split and more (request, kv head) pairs than blocks fit the GPU: persistent blocks, the producer ahead across pairs (they

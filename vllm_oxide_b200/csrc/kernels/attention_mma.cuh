@@ -312,6 +312,26 @@ __device__ __forceinline__ void qk_16keys_swizzled(const uint32_t (&q)[KSTEPS][4
   }
 }
 
+// The same with the 16 query rows in shared memory, Q_ROW_BYTES apart (heads whose queries and outputs together would leave too few
+// registers for a second block on an SM).
+constexpr int Q_ROW_BYTES = ROW_BYTES;
+template <int ROWS>
+__device__ __forceinline__ void qk_16keys_swizzled(const char* qrows, const char* ktile, int row0, int lane, float (&s)[2][4]) {
+#pragma unroll
+  for (int i = 0; i < 2; ++i) s[i][0] = s[i][1] = s[i][2] = s[i][3] = 0.f;
+  const int mi = lane >> 3, r = lane & 7;
+  const int row = row0 + (mi >> 1) * 8 + r;
+  const char* qbase = qrows + ((mi & 1) * 8 + r) * Q_ROW_BYTES + (mi >> 1) * 16;
+#pragma unroll
+  for (int ks = 0; ks < KSTEPS; ++ks) {
+    uint32_t a[4], b[4];
+    ldmatrix_x4(a, qbase + ks * 32);
+    ldmatrix_x4(b, ktile + (ks >> 2) * ROWS * 128 + swizzled_offset(row, (ks & 3) * 2 + (mi & 1)));
+    mma_bf16(s[0], a, b[0], b[1]);
+    mma_bf16(s[1], a, b[2], b[3]);
+  }
+}
+
 template <int ROWS>
 __device__ __forceinline__ void softmax_pv_16keys_swizzled(WarpSoftmax& st, float (&s)[2][4], const char* vtile, int row0,
                                                            int lane) {
