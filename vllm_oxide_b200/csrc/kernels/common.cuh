@@ -149,6 +149,19 @@ template <> struct Wide16<__nv_bfloat16> {
   }
 };
 
+// Two neighbouring elements of the model's type as they are loaded, by one access.
+template <typename T> struct Pair2;
+template <> struct Pair2<float> {
+  typedef float2 Raw;
+  static __device__ __forceinline__ float2 get(const Raw& r) { return r; }
+  static __device__ __forceinline__ void put(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
+};
+template <> struct Pair2<__nv_bfloat16> {
+  typedef uint32_t Raw;
+  static __device__ __forceinline__ float2 get(const Raw& r) { return make_float2(__uint_as_float(r << 16), __uint_as_float(r & 0xffff0000u)); }
+  static __device__ __forceinline__ void put(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
+};
+
 // ---- programmatic dependent launch -------------------------------------------------------------
 // Kernels of the decode chain are launched so that the next kernel may start while the one before it
 // is still running: it sets up, reads what no earlier kernel writes (weights, tables, the step's index

@@ -64,40 +64,12 @@ __device__ __forceinline__ void conv_tokens(const T* x, long x_stride, const flo
   }
 }
 
-// FOUR: filters of four taps in large steps, without the selections that a filter of any length needs (an instance of its own: both ways in
-// one take registers from every filter, 3 to 12 % of their time).
-template <typename T, typename TO, bool FOUR>
-__global__ void __launch_bounds__(128)
-short_conv_silu_kernel(const T* x, long x_stride, const float* __restrict__ w, const float* __restrict__ bias_in,
-                       const float* __restrict__ bias_out, const float* state, long state_stride,
-                       long conv_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
-                       const int* __restrict__ state_slots, TO* out, int num_tokens, int walk, int C, int taps, long num_slots,
-                       int act, int* err) {
-  pdl_launch_dependents();
-  const int t_first = blockIdx.x * walk;
-  const int c = blockIdx.y * 128 + threadIdx.x;
-  float wt[DELTA_MAX_TAPS];
-#pragma unroll
-  for (int s = 0; s < DELTA_MAX_TAPS; ++s) wt[s] = (c < C && s < taps) ? w[(size_t)c * taps + s] : 0.f;
-  const float w_now = c < C ? w[(size_t)c * taps + taps - 1] : 0.f;      // the current token's tap
-  const float b_in = bias_in && c < C ? bias_in[c] : 0.f, b_out = bias_out && c < C ? bias_out[c] : 0.f;
-  pdl_wait();
-  if (c >= C) return;
-  // the usual case of a large step, all of the thread's tokens in one portion: every input is asked for before the first is used
-  if (walk == CONV_TOKENS && t_first + CONV_TOKENS <= num_tokens) {
-    const int req = token_req[t_first];
-    if (req >= 0 && req == token_req[t_first + CONV_TOKENS - 1]) {
-      const int j = t_first - cu_q[req];
-      const int slot = state_slots[req];
-      if (slot < 0 || slot >= num_slots) {
-        atomicOr(err, VOB_ERR_SLOT);
-        return;
-      }
-      const float* st = state + (size_t)slot * state_stride + conv_off;
-      conv_tokens<FOUR ? 4 : DELTA_MAX_TAPS, T, TO>(x, x_stride, st, wt, b_in, b_out, out, t_first, j, c, C, taps, act);
-      return;
-    }
-  }
+// A thread's `walk` tokens of channel c one by one, over any portions.
+template <typename T, typename TO>
+__device__ __forceinline__ void conv_walk(const T* x, long x_stride, const float* state, long state_stride, long conv_off, const int* __restrict__ token_req,
+                                          const int* __restrict__ cu_q, const int* __restrict__ state_slots, const float (&wt)[DELTA_MAX_TAPS],
+                                          float w_now, float b_in, float b_out, TO* out, int t_first, int num_tokens, int walk, int c, int C, int taps,
+                                          long num_slots, int act, int* err) {
   float win[DELTA_MAX_TAPS - 1];      // win[s]: the input taps - 1 - s tokens back
   bool have = false;
   for (int tt = 0; tt < walk; ++tt) {
@@ -135,6 +107,114 @@ short_conv_silu_kernel(const T* x, long x_stride, const float* __restrict__ w, c
       if (s < taps - 2) win[s] = win[s + 1 < DELTA_MAX_TAPS - 1 ? s + 1 : s];
       else if (s == taps - 2) win[s] = cur;
     }
+  }
+}
+
+// FOUR: filters of four taps in large steps, without the selections that a filter of any length needs (an instance of its own: both ways in
+// one take registers from every filter, 3 to 12 % of their time).
+template <typename T, typename TO, bool FOUR>
+__global__ void __launch_bounds__(128)
+short_conv_silu_kernel(const T* x, long x_stride, const float* __restrict__ w, const float* __restrict__ bias_in,
+                       const float* __restrict__ bias_out, const float* state, long state_stride,
+                       long conv_off, const int* __restrict__ token_req, const int* __restrict__ cu_q,
+                       const int* __restrict__ state_slots, TO* out, int num_tokens, int walk, int C, int taps, long num_slots,
+                       int act, int* err) {
+  pdl_launch_dependents();
+  const int t_first = blockIdx.x * walk;
+  const int c = blockIdx.y * 128 + threadIdx.x;
+  float wt[DELTA_MAX_TAPS];
+#pragma unroll
+  for (int s = 0; s < DELTA_MAX_TAPS; ++s) wt[s] = (c < C && s < taps) ? w[(size_t)c * taps + s] : 0.f;
+  const float w_now = c < C ? w[(size_t)c * taps + taps - 1] : 0.f;      // the current token's tap
+  const float b_in = bias_in && c < C ? bias_in[c] : 0.f, b_out = bias_out && c < C ? bias_out[c] : 0.f;
+  pdl_wait();
+  if (c >= C) return;
+  // the usual case of a large step, all of the thread's tokens in one portion: every input is asked for before the first is used
+  if (walk == CONV_TOKENS && t_first + CONV_TOKENS <= num_tokens) {
+    const int req = token_req[t_first];
+    if (req >= 0 && req == token_req[t_first + CONV_TOKENS - 1]) {
+      const int j = t_first - cu_q[req];
+      const int slot = state_slots[req];
+      if (slot < 0 || slot >= num_slots) {
+        atomicOr(err, VOB_ERR_SLOT);
+        return;
+      }
+      const float* st = state + (size_t)slot * state_stride + conv_off;
+      conv_tokens<FOUR ? 4 : DELTA_MAX_TAPS, T, TO>(x, x_stride, st, wt, b_in, b_out, out, t_first, j, c, C, taps, act);
+      return;
+    }
+  }
+  conv_walk<T, TO>(x, x_stride, state, state_stride, conv_off, token_req, cu_q, state_slots, wt, w_now, b_in, b_out, out, t_first, num_tokens, walk, c, C,
+                   taps, num_slots, act, err);
+}
+
+// Filters of four taps in large steps, two neighbouring channels a thread (an even number of channels, rows on two elements' boundaries):
+// the kernel is bound by memory, and 2-byte accesses leave it half of that.  (3,165 tokens of 4,096 channels into float: 30 us; 44 by a channel a
+// thread.)
+template <typename T, typename TO>
+__global__ void __launch_bounds__(128)
+short_conv_pairs_kernel(const T* x, long x_stride, const float* __restrict__ w, const float* __restrict__ bias_in,
+                        const float* __restrict__ bias_out, const float* state, long state_stride, long conv_off,
+                        const int* __restrict__ token_req, const int* __restrict__ cu_q, const int* __restrict__ state_slots, TO* out,
+                        int num_tokens, int C, long num_slots, int act, int* err) {
+  using P = Pair2<T>;
+  pdl_launch_dependents();
+  const int t_first = blockIdx.x * CONV_TOKENS;
+  const int c = 2 * (blockIdx.y * 128 + threadIdx.x);
+  if (c >= C) return;
+  float wt[2][4], b_in[2], b_out[2];
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+#pragma unroll
+    for (int s = 0; s < 4; ++s) wt[e][s] = w[(size_t)(c + e) * 4 + s];
+    b_in[e] = bias_in ? bias_in[c + e] : 0.f;
+    b_out[e] = bias_out ? bias_out[c + e] : 0.f;
+  }
+  const int req = token_req[t_first];
+  const bool one = t_first + CONV_TOKENS <= num_tokens && req >= 0 && req == token_req[min(t_first + CONV_TOKENS, num_tokens) - 1];
+  const int j = one ? t_first - cu_q[req] : 0, slot = one ? state_slots[req] : 0;
+  pdl_wait();
+  if (!one) {
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      const float all[DELTA_MAX_TAPS] = {wt[e][0], wt[e][1], wt[e][2], wt[e][3]};
+      conv_walk<T, TO>(x, x_stride, state, state_stride, conv_off, token_req, cu_q, state_slots, all, wt[e][3], b_in[e], b_out[e], out, t_first,
+                       num_tokens, CONV_TOKENS, c + e, C, 4, num_slots, act, err);
+    }
+    return;
+  }
+  if (slot < 0 || slot >= num_slots) {
+    atomicOr(err, VOB_ERR_SLOT);
+    return;
+  }
+  const float* st = state + (size_t)slot * state_stride + conv_off;
+  typename P::Raw raw[3 + CONV_TOKENS];      // inputs t_first - 3, ...
+#pragma unroll
+  for (int s = 0; s < 3 + CONV_TOKENS; ++s)
+    if (s >= 3 || j >= 3 - s) raw[s] = *reinterpret_cast<const typename P::Raw*>(x + (size_t)(t_first - 3 + s) * x_stride + c);
+  float in[2][3 + CONV_TOKENS];
+#pragma unroll
+  for (int s = 0; s < 3 + CONV_TOKENS; ++s) {
+    if (s >= 3 || j >= 3 - s) {
+      const float2 v = P::get(raw[s]);
+      in[0][s] = v.x + b_in[0];
+      in[1][s] = v.y + b_in[1];
+    } else {
+#pragma unroll
+      for (int e = 0; e < 2; ++e) in[e][s] = st[(size_t)(j + s) * C + c + e];      // (the slot's entry of the input 3 - s tokens back)
+    }
+  }
+#pragma unroll
+  for (int k = 0; k < CONV_TOKENS; ++k) {
+    float o[2];
+#pragma unroll
+    for (int e = 0; e < 2; ++e) {
+      float acc = b_out[e];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) acc = fmaf(wt[e][s], in[e][k + s], acc);          // oldest input first
+      o[e] = act ? silu_f(acc) : acc;
+    }
+    Pair2<TO>::put(out + (size_t)(t_first + k) * C + c, o[0], o[1]);
   }
 }
 
@@ -641,7 +721,12 @@ VOB_API int vob_short_conv_silu(const void* x, long x_stride, const float* w, co
   const int walk = T >= 32 * CONV_TOKENS ? CONV_TOKENS : 1;      // few tokens (decoding): one each, nothing to slide
   dim3 grid((T + walk - 1) / walk, (C + 127) / 128);
   if (grid.y > 65535) return VOB_UNSUPPORTED;
+  const size_t in_size = dtype == VOB_F32 ? 4 : 2, out_size = dtype == VOB_F32 || out_float ? 4 : 2;
+  const bool pairs = taps == 4 && walk > 1 && C % 2 == 0 && x_stride % 2 == 0 && (uintptr_t)x % (2 * in_size) == 0 && (uintptr_t)out % (2 * out_size) == 0;
 #define VOB_SC(TT, TO)                                                                                                           \
+  if (pairs)                                                                                                                     \
+    return launch_kernel(short_conv_pairs_kernel<TT, TO>, dim3(grid.x, (C + 255) / 256), 128, 0, stream, (const TT*)x, x_stride, w, bias_in, \
+                         bias_out, state, state_stride, conv_off, token_req, cu_q, state_slots, (TO*)out, T, C, num_slots, act, err); \
   if (taps == 4 && walk > 1)                                                                                                     \
     return launch_kernel(short_conv_silu_kernel<TT, TO, true>, grid, 128, 0, stream, (const TT*)x, x_stride, w, bias_in, bias_out, \
                          state, state_stride, conv_off, token_req, cu_q, state_slots, (TO*)out, T, walk, C, taps, num_slots, act, err); \

@@ -94,19 +94,6 @@ mingru_scan_kernel(const T* zxg, const T* __restrict__ bz, const T* __restrict__
   if (ch == NCH - 1 && live) state[(size_t)slot * W + c] = s;
 }
 
-// Two neighbouring elements of the model's type as they are loaded, by one access.
-template <typename T> struct Pair2;
-template <> struct Pair2<float> {
-  typedef float2 Raw;
-  static __device__ __forceinline__ float2 get(const Raw& r) { return r; }
-  static __device__ __forceinline__ void put(float* p, float a, float b) { *reinterpret_cast<float2*>(p) = make_float2(a, b); }
-};
-template <> struct Pair2<__nv_bfloat16> {
-  typedef uint32_t Raw;
-  static __device__ __forceinline__ float2 get(const Raw& r) { return make_float2(__uint_as_float(r << 16), __uint_as_float(r & 0xffff0000u)); }
-  static __device__ __forceinline__ void put(__nv_bfloat16* p, float a, float b) { *reinterpret_cast<__nv_bfloat162*>(p) = __floats2bfloat162_rn(a, b); }
-};
-
 // The same for portions, two neighbouring channels a thread (an even number of channels, rows on two elements' boundaries): the
 // ranges are the same and so are the bits.  The walks wait for memory, so a thread asks for PAIR_TOKENS tokens ahead of those that it
 // works on.  (One portion of 2,048 tokens, 4,096 channels: 70 us; 99 by a channel a thread, four tokens at a time.)
