@@ -56,61 +56,109 @@ __device__ __forceinline__ Best warp_best(Best x) {
 
 constexpr int ROUTE_NT = 256;
 
-constexpr int ROUTE_TOKENS = 4;   // tokens a block: the router's rows are read once for all of them
+constexpr int ROUTE_MOST = 8, ROUTE_OF_WARP = 4;      // tokens a block and a warp at most (a warp chooses for each of a block's)
 
-template <typename T>
-__global__ void __launch_bounds__(ROUTE_NT)
+// A block takes TOKENS tokens, whose rows lie in shared memory as they are; eight warps take up to four of them.  A warp takes two
+// experts at a time: every element of a row that it reads serves both, and the experts' rows, which come from L2 or from memory, are on
+// their way many pieces at once.  (2,048 x 16 experts, 40 tokens: 12 us timed alone, 16 with an
+// expert at a time; 500: 13, 17; 1,333: 17, 20; 2,048: 27, 25; 4,096 x 16, 4,001 tokens: 64, 80.)
+template <int TOKENS> struct RouteShape {
+  static constexpr int OWN = TOKENS < ROUTE_OF_WARP ? TOKENS : ROUTE_OF_WARP, GROUPS = TOKENS / OWN, THREADS = ROUTE_NT * GROUPS;
+  static constexpr int BLOCKS = TOKENS == 4 ? 3 : (TOKENS < 4 ? 2 : 1);      // an SM: with one fewer, 1,333 or 200 tokens take a second round
+};
+
+template <typename T, int TOKENS>
+__global__ void __launch_bounds__(RouteShape<TOKENS>::THREADS, RouteShape<TOKENS>::BLOCKS)
 moe_route_kernel(const T* h, const float* __restrict__ w_router, const float* __restrict__ router_bias,
                  const float* __restrict__ correction, const float* __restrict__ w_shared, float* shared_gate, int* ids, float* weights,
                  int W, int E, int top, int count, int keep, int sigmoid_scores, int group_top, int normalise, float weight_scale,
-                 int num_tokens, int per_block) {
+                 int num_tokens, int vec, int wide) {
+  constexpr int OWN = RouteShape<TOKENS>::OWN, NT = RouteShape<TOKENS>::THREADS, WARPS = ROUTE_NT / 32;
   extern __shared__ __align__(16) float route_smem[];
-  float* hrows = route_smem;                        // [per_block][W]
-  float* lists = hrows + (size_t)per_block * W;     // per token: [E] scores, [E] choice scores, [count] group scores, [1] shared gate
+  const int list = 2 * E + count + 1, logits = E + (w_shared ? 1 : 0);
+  float* lists = route_smem;                        // per token: [E] scores, [E] choice scores, [count] group scores, [1] shared gate
+  T* hrows = reinterpret_cast<T*>(lists + (TOKENS * list + 3) / 4 * 4);     // [TOKENS][W]
   pdl_launch_dependents();
   pdl_wait();
-  const int t0 = blockIdx.x * per_block, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  const int here = min(per_block, num_tokens - t0);
-  for (int d = threadIdx.x; d < here * W; d += ROUTE_NT) hrows[d] = to_f<T>(h[(size_t)t0 * W + d]);
+  const int t0 = blockIdx.x * TOKENS, warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int here = min(TOKENS, num_tokens - t0);
+  if (wide) {
+    struct alignas(4 * sizeof(T)) Four { T x[4]; };
+    const Four* src = reinterpret_cast<const Four*>(h + (size_t)t0 * W);
+#pragma unroll 4
+    for (int d = threadIdx.x; d < here * W / 4; d += NT) reinterpret_cast<Four*>(hrows)[d] = src[d];
+  } else {
+    for (int d = threadIdx.x; d < here * W; d += NT) hrows[d] = h[(size_t)t0 * W + d];
+  }
   __syncthreads();
-  // a warp takes experts warp, warp + 8, ...; a lane sums four elements at a time into four chains (one chain where the
-  // width is no multiple of 4): the order of a logit's additions depends on the width alone, not on the tokens beside it
-  const bool vec = W % 4 == 0 && (((uintptr_t)w_router | (uintptr_t)w_shared) % 16) == 0;
-  const int list = 2 * E + count + 1, logits = E + (w_shared ? 1 : 0);
-  for (int e = warp; e < logits; e += ROUTE_NT / 32) {
-    const float* wr = e < E ? w_router + (size_t)e * W : w_shared;
-    float z[ROUTE_TOKENS];
+  // a lane sums four elements at a time into four chains (one chain where rows start on no 16-byte boundary): the order of a logit's
+  // additions depends on the width alone, not on the tokens beside it
+  const int k0 = warp / WARPS * OWN;               // the warp's first token
+  const T* mine = hrows + (size_t)k0 * W;
+  for (int e0 = 2 * (warp % WARPS); e0 < logits; e0 += 2 * WARPS) {
+    const float* wr[2];
+#pragma unroll
+    for (int j = 0; j < 2; ++j) {
+      const int e = min(e0 + j, logits - 1);
+      wr[j] = e < E ? w_router + (size_t)e * W : w_shared;
+    }
+    float z[2][OWN];
     if (vec) {
-      float z4[ROUTE_TOKENS][4];
+      constexpr int AHEAD = OWN == 1 ? 8 : (TOKENS == 4 ? 2 : 4);      // pieces of the router's rows in flight
+      float z4[2][OWN][4];
 #pragma unroll
-      for (int k = 0; k < ROUTE_TOKENS; ++k) z4[k][0] = z4[k][1] = z4[k][2] = z4[k][3] = 0.f;
-      for (int d = lane * 4; d < W; d += 128) {
-        const float4 wv = *reinterpret_cast<const float4*>(wr + d);
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int k = 0; k < ROUTE_TOKENS; ++k) {
-          if (k < here) {
-            const float4 hv = *reinterpret_cast<const float4*>(hrows + (size_t)k * W + d);
-            z4[k][0] = fmaf(hv.x, wv.x, z4[k][0]); z4[k][1] = fmaf(hv.y, wv.y, z4[k][1]);
-            z4[k][2] = fmaf(hv.z, wv.z, z4[k][2]); z4[k][3] = fmaf(hv.w, wv.w, z4[k][3]);
+        for (int k = 0; k < OWN; ++k) z4[j][k][0] = z4[j][k][1] = z4[j][k][2] = z4[j][k][3] = 0.f;
+      for (int d0 = lane * 4; d0 < W; d0 += 128 * AHEAD) {
+        float4 wv[2][AHEAD];
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a)
+#pragma unroll
+          for (int j = 0; j < 2; ++j)
+            if (d0 + 128 * a < W) wv[j][a] = *reinterpret_cast<const float4*>(wr[j] + d0 + 128 * a);
+#pragma unroll
+        for (int a = 0; a < AHEAD; ++a) {
+          if (d0 + 128 * a >= W) break;
+#pragma unroll
+          for (int k = 0; k < OWN; ++k) {
+            float hv[4];
+            load4(mine + (size_t)k * W + d0 + 128 * a, hv);      // (rows of no token: what is there; their sums go nowhere)
+#pragma unroll
+            for (int j = 0; j < 2; ++j) {
+              z4[j][k][0] = fmaf(hv[0], wv[j][a].x, z4[j][k][0]); z4[j][k][1] = fmaf(hv[1], wv[j][a].y, z4[j][k][1]);
+              z4[j][k][2] = fmaf(hv[2], wv[j][a].z, z4[j][k][2]); z4[j][k][3] = fmaf(hv[3], wv[j][a].w, z4[j][k][3]);
+            }
           }
         }
       }
 #pragma unroll
-      for (int k = 0; k < ROUTE_TOKENS; ++k) z[k] = (z4[k][0] + z4[k][1]) + (z4[k][2] + z4[k][3]);
+      for (int j = 0; j < 2; ++j)
+#pragma unroll
+        for (int k = 0; k < OWN; ++k) z[j][k] = (z4[j][k][0] + z4[j][k][1]) + (z4[j][k][2] + z4[j][k][3]);
     } else {
 #pragma unroll
-      for (int k = 0; k < ROUTE_TOKENS; ++k) z[k] = 0.f;
-      for (int d = lane; d < W; d += 32) {
-        const float wv = wr[d];
+      for (int j = 0; j < 2; ++j)
 #pragma unroll
-        for (int k = 0; k < ROUTE_TOKENS; ++k)
-          if (k < here) z[k] = fmaf(hrows[(size_t)k * W + d], wv, z[k]);
+        for (int k = 0; k < OWN; ++k) z[j][k] = 0.f;
+      for (int d = lane; d < W; d += 32) {
+        const float w0 = wr[0][d], w1 = wr[1][d];
+#pragma unroll
+        for (int k = 0; k < OWN; ++k) {
+          const float hv = to_f<T>(mine[(size_t)k * W + d]);
+          z[0][k] = fmaf(hv, w0, z[0][k]);
+          z[1][k] = fmaf(hv, w1, z[1][k]);
+        }
       }
     }
 #pragma unroll
-    for (int k = 0; k < ROUTE_TOKENS; ++k) {
-      const float sum = warp_sum(z[k]);
-      if (lane == 0 && k < here) lists[(size_t)k * list + (e < E ? e : list - 1)] = router_bias && e < E ? sum + router_bias[e] : sum;
+    for (int k = 0; k < OWN; ++k) {
+#pragma unroll
+      for (int j = 0; j < 2; ++j) {
+        const float sum = warp_sum(z[j][k]);
+        const int e = e0 + j;
+        if (lane == 0 && k0 + k < here && e < logits) lists[(size_t)(k0 + k) * list + (e < E ? e : list - 1)] = router_bias && e < E ? sum + router_bias[e] : sum;
+      }
     }
   }
   __syncthreads();
@@ -195,6 +243,94 @@ moe_route_kernel(const T* h, const float* __restrict__ w_router, const float* __
 // One block.  n = tokens * top pairs; slot_of[n]: the row of a pair; row_token[max_rows]: a row's token (-1: padding);
 // tile_expert[max_rows / MOE_TM]: the expert of every MOE_TM rows (-1: past the end).  An expert's rows are padded to a
 // multiple of `pad`, itself a multiple of MOE_TM (a product with larger row tiles asks for more).
+// MANY experts (more than ALIGN_EXPERTS): the pairs are counted and placed by atomics.  Else every warp counts its pairs by itself, a
+// pair's place among the warp's pairs of its expert goes to slot_of, and a second look adds what comes before the warp: no two
+// warps ever meet at a counter.  (160 pairs of 16 experts: 5.4 us, 7.0 by atomics; 5,332,
+// timed alone: 12.2, 14.2; 16,004: 20.4, 22.4.)
+constexpr int ALIGN_EXPERTS = 256, ALIGN_KEPT = 16;
+
+__global__ void __launch_bounds__(1024)
+moe_align_warps_kernel(const int* ids, const float* weights, int* slot_of, int* row_token, float* row_weight, int* tile_expert, int n,
+                       int top, int E, int max_rows, int pad) {
+  extern __shared__ int align_smem[];
+  int* counts = align_smem;          // [E]
+  int* offsets = counts + E;         // [E], behind them the first row past all experts
+  int* of_warp = offsets + E + 1;    // [32][E]: a warp's pairs of an expert, then those of the warps before it
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  pdl_launch_dependents();
+  for (int i = threadIdx.x; i < 32 * E; i += 1024) of_warp[i] = 0;
+  pdl_wait();
+  __syncthreads();
+  int* mine = of_warp + warp * E;
+  // a lane's place of pair id among its warp's
+  auto place = [&](int id) {
+    const bool valid = id >= 0 && id < E;
+    const unsigned same = __match_any_sync(0xffffffffu, valid ? id : -1);
+    const int before = valid ? mine[id] : 0, rank = __popc(same & ((1u << lane) - 1));
+    __syncwarp();
+    if (valid && rank == 0) mine[id] = before + __popc(same);
+    __syncwarp();
+    return valid ? before + rank : -1;
+  };
+  // the first ALIGN_KEPT thousand pairs stay in registers, read all at once; the others' places wait in slot_of
+  int id[ALIGN_KEPT], at[ALIGN_KEPT];
+#pragma unroll
+  for (int g = 0; g < ALIGN_KEPT; ++g) id[g] = g * 1024 + (int)threadIdx.x < n ? ids[g * 1024 + threadIdx.x] : -1;
+#pragma unroll
+  for (int g = 0; g < ALIGN_KEPT; ++g)
+    if (g * 1024 < n) at[g] = place(id[g]);
+  for (int i0 = ALIGN_KEPT * 1024 + warp * 32; i0 < n; i0 += 1024) {
+    const int i = i0 + lane, p = place(i < n ? ids[i] : -1);
+    if (i < n) slot_of[i] = p;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < E; e += 1024) {
+    int sum = 0;
+#pragma unroll 8
+    for (int w = 0; w < 32; ++w) {
+      const int c = of_warp[w * E + e];
+      of_warp[w * E + e] = sum;
+      sum += c;
+    }
+    counts[e] = sum;
+  }
+  __syncthreads();
+  if (warp == 0) {
+    int off = 0;
+    for (int e0 = 0; e0 < E; e0 += 32) {
+      const int padded = e0 + lane < E ? (counts[e0 + lane] + pad - 1) / pad * pad : 0;
+      int upto = padded;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, upto, d);
+        if (lane >= d) upto += v;
+      }
+      if (e0 + lane < E) offsets[e0 + lane] = off + upto - padded;
+      off += __shfl_sync(0xffffffffu, upto, 31);
+    }
+    if (lane == 0) offsets[E] = off;
+  }
+  __syncthreads();
+  for (int e = warp; e < E; e += 32) {
+    const int first = offsets[e], end = offsets[e + 1];
+    for (int tile = first / MOE_TM + lane; tile < end / MOE_TM; tile += 32) tile_expert[tile] = e;
+    for (int r = first + counts[e] + lane; r < end; r += 32) row_token[r] = -1;
+  }
+  for (int tile = offsets[E] / MOE_TM + threadIdx.x; tile < max_rows / MOE_TM; tile += 1024) tile_expert[tile] = -1;
+  for (int r = offsets[E] + threadIdx.x; r < max_rows; r += 1024) row_token[r] = -1;
+  auto put = [&](int i, int e, int p) {
+    if (p < 0) { slot_of[i] = -1; return; }
+    const int row = offsets[e] + mine[e] + p;
+    slot_of[i] = row;
+    row_token[row] = i / top;
+    if (row_weight) row_weight[row] = weights[i];
+  };
+#pragma unroll
+  for (int g = 0; g < ALIGN_KEPT; ++g)
+    if (g * 1024 + (int)threadIdx.x < n) put(g * 1024 + threadIdx.x, id[g], at[g]);
+  for (int i = ALIGN_KEPT * 1024 + threadIdx.x; i < n; i += 1024) put(i, ids[i], slot_of[i]);
+}
+
 __global__ void __launch_bounds__(1024)
 moe_align_kernel(const int* ids, const float* weights, int* slot_of, int* row_token, float* row_weight, int* tile_expert, int n, int top,
                  int E, int max_rows, int pad) {
@@ -527,23 +663,34 @@ VOB_API int vob_moe_route(const void* h, const float* w_router, const float* rou
   if ((w_shared == nullptr) != (shared_gate == nullptr)) return VOB_BAD_ARGUMENT;
   if (E <= 0 || top <= 0 || top > E || count <= 0 || E % count || keep <= 0 || keep > count || (long)(E / count) * keep < top)
     return VOB_BAD_ARGUMENT;
-  // as many tokens a block as 96 KB hold (up to ROUTE_TOKENS) while the blocks still fill the device twice; one where the
-  // width is no multiple of 4 (rows stay aligned).  A token's arithmetic does not depend on how many share its block.
-  int per_block = (int)std::min<long>(ROUTE_TOKENS, std::max<long>(1, T / (2L * sm_count())));
-  while (per_block > 1 && ((size_t)per_block * (W + 2 * E + count + 1) * sizeof(float) > 96 * 1024 || W % 4)) --per_block;
-  const size_t smem = (size_t)per_block * (W + 2 * E + count + 1) * sizeof(float);
+  // as many tokens a block (1, 2, 4, 8) as leave every SM a block and as 96 KB hold; one where rows start on no boundary of four
+  // elements.  A token's arithmetic does not depend on how many share its block.
+  const size_t size = dtype == VOB_BF16 ? 2 : 4;
+  const int vec = W % 4 == 0 && (((uintptr_t)w_router | (uintptr_t)w_shared) % 16) == 0, wide = vec && (uintptr_t)h % (4 * size) == 0;
+  auto bytes = [&](int tokens) { return (size_t)(tokens * (2 * E + count + 1) + 3) / 4 * 16 + (size_t)tokens * W * size; };
+  int tokens = vec ? (W >= 4096 ? ROUTE_MOST : ROUTE_OF_WARP) : 1;      // (at a width of 2,048, 1,333 tokens: 27 us with eight)
+  while (tokens > 1 && (T < (long)tokens * sm_count() || bytes(tokens) > 96 * 1024)) tokens /= 2;
+  const size_t smem = bytes(tokens);
   if (smem > 200 * 1024) return VOB_UNSUPPORTED;
-#define VOB_ROUTE(TYPE)                                                                                                  \
+#define VOB_ROUTE_N(TYPE, N)                                                                                             \
   do {                                                                                                                   \
     if (smem > 48 * 1024)                                                                                                \
-      cudaFuncSetAttribute(moe_route_kernel<TYPE>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);              \
-    return launch_kernel(moe_route_kernel<TYPE>, dim3((T + per_block - 1) / per_block), ROUTE_NT, smem, stream,          \
-                         (const TYPE*)h, w_router, router_bias, correction, w_shared, shared_gate, ids, weights, W, E, top, count, keep, sigmoid_scores,     \
-                         group_top, normalise, weight_scale, T, per_block);                                              \
+      cudaFuncSetAttribute(moe_route_kernel<TYPE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
+    return launch_kernel(moe_route_kernel<TYPE, N>, dim3((T + N - 1) / N), RouteShape<N>::THREADS, smem, stream, (const TYPE*)h, w_router, router_bias, \
+                         correction, w_shared, shared_gate, ids, weights, W, E, top, count, keep, sigmoid_scores, group_top, normalise,   \
+                         weight_scale, T, vec, wide);                                                                      \
+  } while (0)
+#define VOB_ROUTE(TYPE)                    \
+  do {                                     \
+    if (tokens == 8) VOB_ROUTE_N(TYPE, 8); \
+    if (tokens == 4) VOB_ROUTE_N(TYPE, 4); \
+    if (tokens == 2) VOB_ROUTE_N(TYPE, 2); \
+    VOB_ROUTE_N(TYPE, 1);                  \
   } while (0)
   if (dtype == VOB_F32) VOB_ROUTE(float);
   if (dtype == VOB_BF16) VOB_ROUTE(__nv_bfloat16);
 #undef VOB_ROUTE
+#undef VOB_ROUTE_N
   return VOB_BAD_ARGUMENT;
 }
 
@@ -553,6 +700,9 @@ VOB_API int vob_moe_align(const int* ids, const float* weights, int* slot_of, in
   if (n <= 0) return 0;
   if (row_weight && !weights) return VOB_BAD_ARGUMENT;
   if (pad <= 0 || pad % MOE_TM || max_rows % pad || E <= 0 || E > 4096) return VOB_BAD_ARGUMENT;
+  if (E <= ALIGN_EXPERTS)
+    return launch_kernel(moe_align_warps_kernel, dim3(1), 1024, (size_t)(34 * E + 1) * sizeof(int), stream, ids, weights, slot_of, row_token,
+                         row_weight, tile_expert, n, top, E, max_rows, pad);
   return launch_kernel(moe_align_kernel, dim3(1), 1024, (size_t)2 * E * sizeof(int), stream, ids, weights, slot_of, row_token,
                        row_weight, tile_expert, n, top, E, max_rows, pad);
 }
