@@ -1,4 +1,4 @@
-// Sampling on the device: one block per row of float logits, token id out.
+// Sampling on the device: one to eight blocks per row of float logits, token id out.
 //
 // The pipeline is the reference's (vllm-oxide, crates/vllm-oxide/src/sampler.rs:207-261):
 // greedy short-circuit (temperature 0 or top_k 1) -> logits * (1/T) -> top-k (ties at the
@@ -13,7 +13,7 @@
 //     keeps a prefix of its sort, which is the same set unless equal logits straddle the
 //     boundary).  Probability mass is summed as 40-bit fixed point integers, so the set does
 //     not depend on the order of summation.
-#include "common.cuh"
+#include "cluster.cuh"
 
 namespace vob {
 
@@ -25,6 +25,9 @@ __device__ __forceinline__ uint32_t ordered_key(float x) {
   const uint32_t b = __float_as_uint(x + 0.f);      // -0 becomes +0: equal values get equal keys
   return (b & 0x80000000u) ? ~b : (b | 0x80000000u);
 }
+
+// The value that a key was made of (a zero without its sign).
+__device__ __forceinline__ float value_of(uint32_t key) { return __uint_as_float((key & 0x80000000u) ? key & 0x7fffffffu : ~key); }
 
 __device__ __forceinline__ unsigned long long pack_candidate(float value, int index) {
   return ((unsigned long long)ordered_key(value) << 32) | (unsigned long long)(0xFFFFFFFFu - (uint32_t)index);
@@ -73,14 +76,15 @@ __device__ __forceinline__ unsigned long long fixed_mass(float x, float maxv) {
   return (unsigned long long)(expf(x - maxv) * 1099511627776.0f);  // 2^40
 }
 
-// f(value, index) for a thread's share of a row: four values a load, four loads in flight, where the row starts on a 16-byte
-// boundary, the rest one by one.
+// f(value, index) for a thread's share of part `part` of `parts` of a row: four values a load, four loads in flight, where the row starts
+// on a 16-byte boundary, the rest one by one.
 template <typename F>
-__device__ __forceinline__ void each_logit(const float* l, int V, F f) {
+__device__ __forceinline__ void each_logit(const float* l, int V, int part, int parts, F f) {
   const float4* l4 = reinterpret_cast<const float4*>(l);
-  const int v4 = (uintptr_t)l % 16 == 0 ? V / 4 : 0;
-  int i = threadIdx.x;
-  for (; i + 3 * SAMPLE_THREADS < v4; i += 4 * SAMPLE_THREADS) {
+  const int v4 = (uintptr_t)l % 16 == 0 ? V / 4 : 0, rest = V - 4 * v4;
+  const int end4 = (int)((long)v4 * (part + 1) / parts), end = 4 * v4 + (int)((long)rest * (part + 1) / parts);
+  int i = (int)((long)v4 * part / parts) + threadIdx.x;
+  for (; i + 3 * SAMPLE_THREADS < end4; i += 4 * SAMPLE_THREADS) {
     float4 x[4];
 #pragma unroll
     for (int k = 0; k < 4; ++k) x[k] = l4[i + k * SAMPLE_THREADS];
@@ -90,11 +94,59 @@ __device__ __forceinline__ void each_logit(const float* l, int V, F f) {
       f(x[k].x, at); f(x[k].y, at + 1); f(x[k].z, at + 2); f(x[k].w, at + 3);
     }
   }
-  for (; i < v4; i += SAMPLE_THREADS) {
+  for (; i < end4; i += SAMPLE_THREADS) {
     const float4 x = l4[i];
     f(x.x, 4 * i); f(x.y, 4 * i + 1); f(x.z, 4 * i + 2); f(x.w, 4 * i + 3);
   }
-  for (i = 4 * v4 + threadIdx.x; i < V; i += SAMPLE_THREADS) f(l[i], i);
+  for (i = 4 * v4 + (int)((long)rest * part / parts) + threadIdx.x; i < end; i += SAMPLE_THREADS) f(l[i], i);
+}
+
+// The same with every thread at every step: f(value, index, whether there is one).
+template <typename F>
+__device__ __forceinline__ void each_logit_together(const float* l, int V, int part, int parts, F f) {
+  const float4* l4 = reinterpret_cast<const float4*>(l);
+  const int v4 = (uintptr_t)l % 16 == 0 ? V / 4 : 0, rest = V - 4 * v4;
+  const int end4 = (int)((long)v4 * (part + 1) / parts), end = 4 * v4 + (int)((long)rest * (part + 1) / parts);
+  for (int i0 = (int)((long)v4 * part / parts); i0 < end4; i0 += 2 * SAMPLE_THREADS) {
+    float4 x[2];
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = i0 + k * SAMPLE_THREADS + threadIdx.x;
+      x[k] = i < end4 ? l4[i] : make_float4(0.f, 0.f, 0.f, 0.f);
+    }
+#pragma unroll
+    for (int k = 0; k < 2; ++k) {
+      const int i = i0 + k * SAMPLE_THREADS + threadIdx.x;
+      const bool in = i < end4;
+      f(x[k].x, 4 * i, in); f(x[k].y, 4 * i + 1, in); f(x[k].z, 4 * i + 2, in); f(x[k].w, 4 * i + 3, in);
+    }
+  }
+  for (int i0 = 4 * v4 + (int)((long)rest * part / parts); i0 < end; i0 += SAMPLE_THREADS) {
+    const int i = i0 + threadIdx.x;
+    f(i < end ? l[i] : 0.f, i, i < end);
+  }
+}
+
+// The same variable of shared memory in block `rank` of the cluster.
+template <typename N>
+__device__ __forceinline__ const volatile N* in_block(const N* mine, int rank) {
+  unsigned long long a;
+  asm("mapa.u64 %0, %1, %2;\n" : "=l"(a) : "l"(mine), "r"(rank));
+  return reinterpret_cast<const volatile N*>(a);
+}
+
+__device__ __forceinline__ uint32_t block_max_u32(uint32_t v, unsigned long long* scratch) { return (uint32_t)block_max_u64(v, scratch); }
+
+// Sum over a block; every thread gets it (integers: any order gives the same).
+__device__ __forceinline__ unsigned long long block_sum_u64(unsigned long long v, unsigned long long* scratch) {
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
+  __syncthreads();
+  if ((threadIdx.x & 31) == 0) scratch[threadIdx.x >> 5] = v;
+  __syncthreads();
+  unsigned long long total = 0;
+  for (int i = 0; i < SAMPLE_THREADS / 32; ++i) total += scratch[i];
+  return total;
 }
 
 // The bin in which the sum from the highest bin down reaches `need` (bin 0 if it does not), and the sum above it.  One warp, eight
@@ -124,34 +176,66 @@ __device__ __forceinline__ void find_bin(const N* bins, N need, int& bin, N& abo
   above = cum;
 }
 
+// A row is looked over by the blocks of a cluster, each its part: they find the maximum, what top-p's masses add up to, and the
+// tokens that may still be drawn.  The first block then has all of those (it fetches the others' from their shared memory) and
+// goes on alone.  Rows of whom top-k asks for more than SAMPLE_SHARED_K, and what is left to be searched as a whole, are the first block's
+// from the start: the blocks' lists together would not fit, and such rows are rare.  (48 rows of 151,936, top-k 50, top-p 0.9: two blocks a
+// row 44 us, one 53; of 16 flat rows with top-p alone: eight 258, one 717; of one: 98 and 559.  Timed one by one.)
+constexpr int SAMPLE_SHARED_K = 256;
+// Up to this many gathered tokens every thread compares its token with all: thresholds are then a look at a list that lies in shared
+// memory and one reduction, where the digits of a key take four histograms with their barriers.
+constexpr int SAMPLE_FEW = 512;
+
 __global__ void __launch_bounds__(SAMPLE_THREADS)
 sample_kernel(const float* logits, long ld, int V, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
-              const unsigned long long* __restrict__ keys, int* __restrict__ out) {
+              const unsigned long long* __restrict__ keys, int* __restrict__ out, int blocks) {
   __shared__ unsigned long long scratch[32];
   __shared__ unsigned int hist[256];
-  __shared__ unsigned long long mass[256];
+  __shared__ unsigned long long mass[2][256], all_mass[256];      // (by turns: the other blocks read one while the next is made)
   __shared__ unsigned int s_prefix, s_remaining_k;
   __shared__ unsigned long long s_remaining_mass;
   __shared__ unsigned int s_ncand, s_short, s_gather;
+  __shared__ unsigned long long s_told[5];          // what a block tells the others: a maximum, masses, gathered masses, how many, a draw
+  __shared__ unsigned int s_bound;
   extern __shared__ unsigned long long cand_raw[];              // SAMPLE_CANDIDATES x (mass, key, index)
   unsigned long long* cand_mass = cand_raw;
   uint32_t* cand_key = reinterpret_cast<uint32_t*>(cand_raw + SAMPLE_CANDIDATES);
   uint32_t* cand_idx = cand_key + SAMPLE_CANDIDATES;
-  const int row = blockIdx.x, tid = threadIdx.x;
+  const int row = blockIdx.x / blocks, rank = blockIdx.x % blocks, tid = threadIdx.x;
+  pdl_wait();
   const float* l = logits + (size_t)row * ld;
   const float temp = temperature[row];
   const int k = top_k[row];
   const float p = top_p[row];
+  const unsigned long long key_row = keys[row];
+  const bool top_p_on = p > 0.f && p < 1.f;
+  // (the same for every block of the row, and so is every meeting below)
+  const int parts = k >= 1 && k < V && k > SAMPLE_SHARED_K && temp > 0.f ? 1 : blocks;
+  if (rank >= parts) return;
+  // what the blocks have told becomes every block's; a block's shared memory is read until the last meeting
+  auto meet = [&]() { if (parts > 1) cluster_sync_all(); };
+  auto most_of_all = [&](unsigned long long best) {
+    best = block_max_u64(best, scratch);
+    if (parts == 1) return best;
+    if (tid == 0) s_told[0] = best;
+    meet();
+    for (int r = 0; r < parts; ++r) {
+      const unsigned long long other = *in_block(&s_told[0], r);
+      best = other > best ? other : best;
+    }
+    return best;
+  };
 
   if (temp <= 0.f || k == 1) {  // greedy
     unsigned long long best = 0;
-    each_logit(l, V, [&](float x, int i) {
+    each_logit(l, V, rank, parts, [&](float x, int i) {
       const unsigned long long c = pack_candidate(x, i);
       best = c > best ? c : best;
     });
-    best = block_max_u64(best, scratch);
-    if (tid == 0) out[row] = (int)(0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull));
+    best = most_of_all(best);
+    if (tid == 0 && rank == 0) out[row] = (int)(0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull));
+    meet();
     return;
   }
   const float inv_t = 1.0f / temp;
@@ -160,8 +244,9 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
   // A token among the k largest is at least as large as the k-th largest of the threads' own maxima (k of them are tokens).  So
   // the first look at the row only takes maxima, the second gathers the tokens from that bound on into shared memory, and
   // everything after (the digits of the exact threshold, the maximum, top-p, the draw) runs over them alone: some
-  // -1024 ln(1 - k / 1024) tokens of a long row, 51 for k = 50, 2,839 for 960.  (48 rows of 151,936 with top-k 50 and top-p 0.9: 39 us;
-  // 139 by the histogram alone, which is bound by atomics to a handful of bins.)
+  // -1024 ln(1 - k / 1024) tokens of a long row, 51 for k = 50, 2,839 for 960.  The largest of the blocks' bounds is one for the whole
+  // row.  (48 rows of 151,936 with top-k 50 and top-p 0.9, a block each: 35 us; 139 by the histogram alone, which is bound by atomics to a
+  // handful of bins.)
   // More than SAMPLE_TOP_K asked for, or more than half of the threads' maxima equal to the bound (a masked vocabulary with fewer
   // than k tokens left: every masked token is at the bound): the first digit (sign and most of the exponent) is found by a histogram
   // over the row, and the tokens whose first digit is at least that of the k-th largest are gathered if they are few.
@@ -170,28 +255,69 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
   if (k >= 1 && k < V) {
     if (k <= SAMPLE_TOP_K) {
       uint32_t most = 0;
-      each_logit(l, V, [&](float x, int) { most = max(most, ordered_key(x * inv_t)); });
+      each_logit(l, V, rank, parts, [&](float x, int) { most = max(most, ordered_key(x * inv_t)); });
       uint32_t bound = 0;
       for (int bit = 31; bit >= 0; --bit) {
         const uint32_t higher = bound | (1u << bit);
         if (__syncthreads_count(most >= higher) >= k) bound = higher;
       }
       // (a bound of 0: fewer threads than that have a token, and the row is short)
-      if (__syncthreads_count(most == bound) <= SAMPLE_THREADS / 2 || bound == 0) {
-        if (tid == 0) s_ncand = 0;
-        __syncthreads();
-        each_logit(l, V, [&](float x, int i) {
+      const bool few = __syncthreads_count(most == bound) <= SAMPLE_THREADS / 2 && bound != 0;
+      // (a part of a row where many are at the bound, such as a masked one, gathers what is above it: the bound of the others decides)
+      if (!few) ++bound;
+      if (tid == 0) { s_ncand = few || parts > 1 ? 0u : (unsigned)SAMPLE_CANDIDATES + 1; s_bound = bound; }
+      __syncthreads();
+      if (few || parts > 1) {
+        each_logit(l, V, rank, parts, [&](float x, int i) {
           const uint32_t key = ordered_key(x * inv_t);
           if (key >= bound) {
             const unsigned pos = atomicAdd(&s_ncand, 1u);
             if (pos < (unsigned)SAMPLE_CANDIDATES) { cand_key[pos] = key; cand_idx[pos] = (uint32_t)i; }
           }
         });
-        __syncthreads();
-        gathered = s_ncand <= (unsigned)SAMPLE_CANDIDATES;
+      }
+      __syncthreads();
+      gathered = s_ncand <= (unsigned)SAMPLE_CANDIDATES;
+      if (parts > 1) {
+        meet();
+        if (rank == 0) {
+          for (int r = 1; r < parts; ++r) {
+            bound = max(bound, *in_block(&s_bound, r));
+            gathered = gathered && *in_block(&s_ncand, r) <= (unsigned)SAMPLE_CANDIDATES;
+          }
+          for (int r = 1; r < parts && gathered; ++r) {
+            const unsigned n = *in_block(&s_ncand, r);
+            const volatile uint32_t* key = in_block(cand_key, r);
+            const volatile uint32_t* idx = in_block(cand_idx, r);
+            for (unsigned c = tid; c < n; c += SAMPLE_THREADS) {
+              const uint32_t x = key[c];
+              if (x < bound) continue;
+              const unsigned pos = atomicAdd(&s_ncand, 1u);
+              if (pos < (unsigned)SAMPLE_CANDIDATES) { cand_key[pos] = x; cand_idx[pos] = idx[c]; }
+            }
+          }
+          __syncthreads();
+          gathered = gathered && s_ncand <= (unsigned)SAMPLE_CANDIDATES;
+          // every token from the largest bound on is there: if they are k, the k largest are among them
+          unsigned long long have = 0;
+          for (unsigned c = tid; gathered && c < s_ncand; c += SAMPLE_THREADS) have += cand_key[c] >= bound;
+          gathered = block_sum_u64(have, scratch) >= (unsigned long long)k && gathered;
+        }
+        meet();
+        if (rank > 0) return;
       }
     }
     __syncthreads();
+    const bool few_left = gathered && s_ncand <= (unsigned)SAMPLE_FEW;
+    if (few_left) {
+      // the largest key that at least k tokens reach
+      const unsigned n = s_ncand;
+      const uint32_t mine = (unsigned)tid < n ? cand_key[tid] : 0u;
+      unsigned reach = 0;
+      if ((unsigned)tid < n)
+        for (unsigned c = 0; c < n; ++c) reach += cand_key[c] >= mine;
+      thr = block_max_u32((unsigned)tid < n && reach >= (unsigned)k ? mine : 0u, scratch);
+    } else {
     if (tid == 0) { s_prefix = 0; s_remaining_k = (unsigned)k; s_gather = 0; }
     for (int pass = 0; pass < 4; ++pass) {
       const int shift = 24 - 8 * pass;
@@ -206,7 +332,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
           if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
         }
       } else {
-        each_logit(l, V, [&](float x, int) {
+        each_logit(l, V, 0, 1, [&](float x, int) {
           const uint32_t key = ordered_key(x * inv_t);
           if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
         });
@@ -226,7 +352,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       __syncthreads();
       if (pass == 0 && s_gather) {
         const uint32_t first = s_prefix >> 24;
-        each_logit(l, V, [&](float x, int i) {
+        each_logit(l, V, 0, 1, [&](float x, int i) {
           const uint32_t key = ordered_key(x * inv_t);
           if ((key >> 24) >= first) {
             const unsigned pos = atomicAdd(&s_ncand, 1u);
@@ -238,52 +364,52 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       }
     }
     thr = s_prefix;
+    }
   }
 
+  // the blocks that are still here share the row: all of them without a top-k, else the first alone
+  const int of = k >= 1 && k < V ? 1 : parts, now = rank;
   // ---- maximum of the scaled logits (always a survivor)
   unsigned long long best = 0;
   if (gathered) {
     const unsigned ncand = s_ncand;
     for (unsigned c = tid; c < ncand; c += SAMPLE_THREADS) {
-      const int i = (int)cand_idx[c];
-      const unsigned long long cnd = pack_candidate(l[i] * inv_t, i);
+      const unsigned long long cnd = ((unsigned long long)cand_key[c] << 32) | (unsigned long long)(0xFFFFFFFFu - cand_idx[c]);
       best = cnd > best ? cnd : best;
     }
   } else {
-    each_logit(l, V, [&](float x, int i) {
+    each_logit(l, V, now, of, [&](float x, int i) {
       const unsigned long long c = pack_candidate(x * inv_t, i);
       best = c > best ? c : best;
     });
   }
-  best = block_max_u64(best, scratch);
-  const int imax = (int)(0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull));
-  const float maxv = l[imax] * inv_t;
+  best = of > 1 ? most_of_all(best) : block_max_u64(best, scratch);
+  const float maxv = value_of((uint32_t)(best >> 32));
 
   // ---- top-p over the survivors
-  if (p > 0.f && p < 1.f) {
+  if (top_p_on) {
     unsigned long long z = 0;
     if (gathered) {
       const unsigned ncand = s_ncand;
       for (unsigned c = tid; c < ncand; c += SAMPLE_THREADS) {
-        const unsigned long long m = cand_key[c] >= thr ? fixed_mass(l[cand_idx[c]] * inv_t, maxv) : 0ull;
+        const unsigned long long m = cand_key[c] >= thr ? fixed_mass(value_of(cand_key[c]), maxv) : 0ull;
         cand_mass[c] = m;
         z += m;
       }
     } else {
-      each_logit(l, V, [&](float raw, int) {
+      each_logit(l, V, now, of, [&](float raw, int) {
         const float x = raw * inv_t;
         if (ordered_key(x) >= thr) z += fixed_mass(x, maxv);
       });
     }
-    // integer sum over the block: any order gives the same total
-#pragma unroll
-    for (int o = 16; o > 0; o >>= 1) z += __shfl_xor_sync(0xffffffffu, z, o);
-    __syncthreads();
-    if ((tid & 31) == 0) scratch[tid >> 5] = z;
-    __syncthreads();
+    unsigned long long total = block_sum_u64(z, scratch);
+    if (of > 1) {
+      if (tid == 0) s_told[1] = total;
+      meet();
+      total = 0;
+      for (int r = 0; r < of; ++r) total += *in_block(&s_told[1], r);
+    }
     if (tid == 0) {
-      unsigned long long total = 0;
-      for (int i = 0; i < SAMPLE_THREADS / 32; ++i) total += scratch[i];
       unsigned long long target = (unsigned long long)((double)p * (double)total);
       if (target < 1) target = 1;
       s_remaining_mass = target;
@@ -298,11 +424,9 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
     if (tid == 0) { s_short = gathered ? 1u : 0u; if (!gathered) s_ncand = 0; }
     __syncthreads();
     if (!gathered) {
-      unsigned long long total = 0;
-      for (int i = 0; i < SAMPLE_THREADS / 32; ++i) total += scratch[i];
       const unsigned long long floor_mass = (unsigned long long)((1.0 - (double)p) * (double)total / (double)V);
       if (floor_mass >= 1) {
-        each_logit(l, V, [&](float raw, int i) {
+        each_logit(l, V, now, of, [&](float raw, int i) {
           const float x = raw * inv_t;
           const uint32_t key = ordered_key(x);
           if (key < thr) return;
@@ -316,48 +440,90 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       }
     }
     __syncthreads();
-    const unsigned ncand = s_ncand;
-    if (!gathered && ncand <= (unsigned)SAMPLE_CANDIDATES) {
-      unsigned long long z2 = 0;
-      for (unsigned i = tid; i < ncand; i += SAMPLE_THREADS) z2 += cand_mass[i];
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) z2 += __shfl_xor_sync(0xffffffffu, z2, o);
-      __syncthreads();
-      if ((tid & 31) == 0) scratch[tid >> 5] = z2;
-      __syncthreads();
-      if (tid == 0) {
-        unsigned long long have = 0;
-        for (int i = 0; i < SAMPLE_THREADS / 32; ++i) have += scratch[i];
-        s_short = have >= s_remaining_mass ? 1u : 0u;
+    if (!gathered) {
+      unsigned n = s_ncand;
+      unsigned long long have = 0;
+      if (n <= (unsigned)SAMPLE_CANDIDATES)
+        for (unsigned i = tid; i < n; i += SAMPLE_THREADS) have += cand_mass[i];
+      have = block_sum_u64(have, scratch);
+      if (of > 1) {
+        if (tid == 0) { s_told[2] = have; s_told[3] = n; }
+        meet();
+        have = n = 0;
+        for (int r = 0; r < of; ++r) {
+          have += *in_block(&s_told[2], r);
+          n += (unsigned)min(*in_block(&s_told[3], r), (unsigned long long)SAMPLE_CANDIDATES + 1);
+        }
+      }
+      const bool enough = n <= (unsigned)SAMPLE_CANDIDATES && have >= s_remaining_mass;
+      if (tid == 0) s_short = enough ? 1u : 0u;
+      if (enough && of > 1) {
+        // the others' gathered tokens become the first block's
+        if (rank == 0) {
+          for (int r = 1; r < of; ++r) {
+            const unsigned more = (unsigned)*in_block(&s_told[3], r);
+            const volatile unsigned long long* m = in_block(cand_mass, r);
+            const volatile uint32_t* key = in_block(cand_key, r);
+            const volatile uint32_t* idx = in_block(cand_idx, r);
+            for (unsigned c = tid; c < more; c += SAMPLE_THREADS) {
+              const unsigned pos = atomicAdd(&s_ncand, 1u);
+              cand_mass[pos] = m[c]; cand_key[pos] = key[c]; cand_idx[pos] = idx[c];
+            }
+          }
+        }
+        meet();
+        if (rank > 0) return;
       }
       __syncthreads();
     }
+    const unsigned ncand = s_ncand;
     const bool short_way = s_short != 0;
+    if (short_way && ncand <= (unsigned)SAMPLE_FEW) {
+      // the largest key down to which the masses reach the target
+      const uint32_t mine = (unsigned)tid < ncand ? cand_key[tid] : 0u;
+      unsigned long long reach = 0;
+      if ((unsigned)tid < ncand)
+        for (unsigned c = 0; c < ncand; ++c) reach += cand_key[c] >= mine ? cand_mass[c] : 0ull;
+      const uint32_t at = block_max_u32((unsigned)tid < ncand && reach >= s_remaining_mass ? mine : 0u, scratch);
+      if (tid == 0) s_prefix = at;
+      __syncthreads();
+    } else
     for (int pass = 0; pass < 4; ++pass) {
       const int shift = 24 - 8 * pass;
-      if (tid < 256) mass[tid] = 0;
+      unsigned long long* bins = mass[pass & 1];
+      if (tid < 256) bins[tid] = 0;
       __syncthreads();
       const uint32_t prefix = s_prefix;
       const uint32_t mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
       if (short_way) {
         for (unsigned i = tid; i < ncand; i += SAMPLE_THREADS) {
           const uint32_t key = cand_key[i];
-          if ((key & mask) == prefix) atomicAdd(&mass[(key >> shift) & 255u], cand_mass[i]);
+          if ((key & mask) == prefix) atomicAdd(&bins[(key >> shift) & 255u], cand_mass[i]);
         }
-      } else
-      for (int base = 0; base < V; base += SAMPLE_THREADS) {
-        const int i = base + tid;
-        const float x = i < V ? l[i] * inv_t : 0.f;
-        const uint32_t key = ordered_key(x);
-        const bool in = i < V && key >= thr && (key & mask) == prefix;
-        warp_hist_mass(mass, (int)((key >> shift) & 255u), in ? fixed_mass(x, maxv) : 0ull, in);
+      } else {
+        each_logit_together(l, V, now, of, [&](float raw, int, bool there) {
+          const float x = there ? raw * inv_t : 0.f;
+          const uint32_t key = ordered_key(x);
+          const bool in = there && key >= thr && (key & mask) == prefix;
+          warp_hist_mass(bins, (int)((key >> shift) & 255u), in ? fixed_mass(x, maxv) : 0ull, in);
+        });
       }
       __syncthreads();
+      if (of > 1 && !short_way) {
+        meet();
+        if (tid < 256) {
+          unsigned long long sum = 0;
+          for (int r = 0; r < of; ++r) sum += *in_block(&bins[tid], r);
+          all_mass[tid] = sum;
+        }
+        bins = all_mass;
+        __syncthreads();
+      }
       if (tid < 32) {
         const unsigned long long need = s_remaining_mass;
         int b;
         unsigned long long cum;
-        find_bin(mass, need, b, cum);
+        find_bin(bins, need, b, cum);
         if (tid == 0) {
           s_remaining_mass = need - cum;
           s_prefix = prefix | ((uint32_t)b << shift);
@@ -369,23 +535,23 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
     thr = thr_p > thr ? thr_p : thr;
   }
 
-  // ---- Gumbel-max over the survivors
-  const unsigned long long key_row = keys[row];
+  // ---- Gumbel-max over the survivors (gathered ones are the first block's)
+  const int drawing = top_p_on && s_short != 0 ? 1 : of;
   best = 0;
-  if (gathered || (p > 0.f && p < 1.f && s_short != 0)) {
+  if (gathered || (top_p_on && s_short != 0)) {
     // the survivors are among the gathered tokens
     const unsigned ncand = s_ncand;
     for (unsigned c = tid; c < ncand; c += SAMPLE_THREADS) {
       if (cand_key[c] < thr) continue;
       const int i = (int)cand_idx[c];
-      const float x = l[i] * inv_t;
+      const float x = value_of(cand_key[c]);
       const float u = counter_uniform(key_row, (uint32_t)i);
       const float g = -logf(-logf(u));
       const unsigned long long cnd = pack_candidate(x + g, i);
       best = cnd > best ? cnd : best;
     }
   } else
-  each_logit(l, V, [&](float raw, int i) {
+  each_logit(l, V, now, drawing, [&](float raw, int i) {
     const float x = raw * inv_t;
     if (ordered_key(x) < thr) return;
     const float u = counter_uniform(key_row, (uint32_t)i);
@@ -393,7 +559,20 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
     const unsigned long long c = pack_candidate(x + g, i);
     best = c > best ? c : best;
   });
-  best = block_max_u64(best, scratch);
+  if (drawing > 1) {
+    // (another variable than the maximum's: a block may still read that one)
+    best = block_max_u64(best, scratch);
+    if (tid == 0) s_told[4] = best;
+    meet();
+    for (int r = 0; r < drawing; ++r) {
+      const unsigned long long other = *in_block(&s_told[4], r);
+      best = other > best ? other : best;
+    }
+    meet();
+    if (rank > 0) return;
+  } else {
+    best = block_max_u64(best, scratch);
+  }
   if (tid == 0) out[row] = (int)(0xFFFFFFFFu - (uint32_t)(best & 0xFFFFFFFFull));
 }
 
@@ -428,8 +607,11 @@ VOB_API int vob_sample(const float* logits, long ld, int R, int V, const float* 
     if (e != cudaSuccess) return (int)e;
     configured = true;
   }
-  sample_kernel<<<R, SAMPLE_THREADS, smem, stream>>>(logits, ld, V, temperature, top_k, top_p, keys, out);
-  return launch_status();
+  // blocks a row: as many (1, 2, 4, 8) as leave every block an SM, of at least four thousand tokens each
+  int blocks = 8;
+  while (blocks > 1 && ((long)R * blocks > sm_count() || V / blocks < 4 * SAMPLE_THREADS)) blocks /= 2;
+  return launch_kernel_cluster(sample_kernel, dim3((unsigned)(R * blocks)), SAMPLE_THREADS, smem, stream, (unsigned)blocks, logits, ld, V,
+                               temperature, top_k, top_p, keys, out, blocks);
 }
 
 // (row, token, count) triples: one per distinct token of a row's history; a triple must appear once.
