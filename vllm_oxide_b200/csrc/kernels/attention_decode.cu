@@ -201,6 +201,15 @@ template <bool EXTRAS, bool SHARED, bool DENSE> struct DecodeShape {
   static constexpr int SMEM = 1024 + DATA + (QUERIES ? 16 * Q_ROW_BYTES : 0) + 2 * STAGES * 8 + 32;
 };
 
+// A LATE kernel works beside the portions' attention of the same step, which it follows on the stream: it starts when every block of that one
+// has seen the kernels before it complete (attention_prefill_tc5_kernel: lead), needs nothing that it makes, writes other rows, and waits
+// for it at its own end only, so that who waits for this kernel waits for both.  The first look at what those kernels wrote is made past
+// this SM's L1, and by the copy engine behind a proxy fence.
+__device__ __forceinline__ void late_start() {
+  __threadfence();
+  asm volatile("fence.proxy.async;\n" ::: "memory");
+}
+
 template <bool EXTRAS, bool SHARED, bool DENSE>
 __global__ void __launch_bounds__(DT_THREADS, DecodeShape<EXTRAS, SHARED, DENSE>::BLOCKS)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
@@ -208,7 +217,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                             const int* __restrict__ context_lens, int nh, int kvh, int block_size, int window, float scale,
                             long num_pages, float* part_o, float* part_lse,
-                            int box_keys, int cluster, int* err, HeadEpilogue ep) {
+                            int box_keys, int cluster, int late, int* err, HeadEpilogue ep) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   using SHAPE = DecodeShape<EXTRAS, SHARED, DENSE>;
@@ -219,6 +228,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   uint64_t* empty = full + STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + STAGES);
   pdl_launch_dependents();
+  if (late) late_start();
   const int split = blockIdx.x, num_splits = gridDim.x, kh = blockIdx.y, b = blockIdx.z;
   const int t = cu_q[b];
   const int t_next = cu_q[b + 1], context = context_lens[b];
@@ -271,7 +281,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
           if (it >= STAGES) ok = mbar_wait(&empty[s], (unsigned)(((it / STAGES) - 1) & 1), abort_flag, err);
           if (ok) {
             const int tile_start = km.real(start + it * DEC_TILE);
-            if (!waited && tile_start + DEC_TILE > pos) { pdl_wait(); waited = true; }
+            if (!waited && tile_start + DEC_TILE > pos) { if (!late) pdl_wait(); waited = true; }
             mbar_expect_tx(&full[s], (unsigned)STAGE_BYTES);
             char* kt = smem + s * STAGE_BYTES;
             if (box_keys == DEC_TILE) {
@@ -316,7 +326,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     }
   } else {
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
-    pdl_wait();
+    if (!late) pdl_wait();
     const int g = lane >> 2, tq = lane & 3;
     uint32_t qf[QUERIES ? 1 : KSTEPS][4];
     if constexpr (QUERIES) {
@@ -383,10 +393,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       if (lane == 0) mbar_arrive(&empty[s]);
     }
   }
-  pdl_wait();             // (a no-op for threads that have waited) nothing is written before the kernels before are done
+  if (!late) pdl_wait();  // (a no-op for threads that have waited) nothing is written before the kernels before are done
   __syncthreads();        // every stage has been read (or given up): the merge may reuse the memory
   const bool aborted = *abort_flag != 0;
-  if (aborted && !cluster) return;
+  if (aborted && !cluster) { if (late) pdl_wait(); return; }
   float* wm = reinterpret_cast<float*>(smem);                 // [DEC_WARPS][16]
   float* wl = wm + DEC_WARPS * 16;
   float* wo = wl + DEC_WARPS * 16;                            // [DEC_WARPS][16][HD]
@@ -464,7 +474,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       if (d == 0) part_lse[p] = lse;
     }
   }
-  if (num_splits == 1 || !cluster) return;
+  if (num_splits == 1 || !cluster) { if (late) pdl_wait(); return; }
   // The blocks of a (request, kv head) form a thread-block cluster: each reads the others' results from their shared
   // memory and merges a share of the outputs (weights 2^(lse - max lse), in the order of the splits).  Every block
   // of the cluster comes to both barriers, also one that gave up (its log-sum-exp is -inf: weight zero).
@@ -507,6 +517,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   // nobody may leave while another block still reads its shared memory
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+  if (late) pdl_wait();   // it ends behind the kernel that it works beside
 }
 
 // ---- many decoding requests, one split each ---------------------------------------------------------------------------
@@ -529,13 +540,19 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
 constexpr int DI_MERGE_FLOATS(int G) { return 2 * DEC_WARPS * 16 + DEC_WARPS * G * HD; }
 constexpr int DI_DRAW_AHEAD = 2;                          // tiles before a pair's last at which the next pair is drawn
 constexpr int DI_QUEUE = 8;                               // entries; the producer is at most DT_STAGES + 1 pairs ahead
+// Pairs are given out with the longest requests first, so that the last to end are short ones: every block sorts up to DI_ORDERED
+// requests by their tiles (in 256 steps; equal ones stay in the batch's order, so every block finds the same), before the kernels ahead are done.
+// (224 requests of 40 to 1,152 keys, 8 x 2 heads of 128: 100 us, 111 in the order of the batch, both beside portions.)
+constexpr int DI_ORDERED = 1024, DI_BUCKETS = 256;
+// (from seven heads a key head on the sums' buffers leave no room for it beside a second block)
+constexpr int DI_ORDER_BYTES(int G) { return G <= 6 ? DI_BUCKETS * 4 + DI_ORDERED * 2 : 0; }
 
 __global__ void __launch_bounds__(DT_THREADS)
 attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                                   const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                                   const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                                   const int* __restrict__ context_lens, int num_requests, int nh, int kvh, int block_size,
-                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, int* err,
+                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, int late, int* err,
                                   HeadEpilogue ep) {
   // pairs_taken[0]: pairs given out beyond the first of each block; [1]: blocks that have left
   extern __shared__ __align__(1024) char smem_raw[];
@@ -549,8 +566,51 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
   uint64_t* full = reinterpret_cast<uint64_t*>(queue + DI_QUEUE);
   uint64_t* empty = full + DT_STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + DT_STAGES);
+  int* bucket_at = const_cast<int*>(reinterpret_cast<volatile int*>(abort_flag)) + 2;       // [DI_BUCKETS]
+  uint16_t* order = reinterpret_cast<uint16_t*>(bucket_at + DI_BUCKETS);                    // [num_requests], up to DI_ORDERED
+  const bool ordered = num_requests <= DI_ORDERED && DI_ORDER_BYTES(G) > 0;
   pdl_launch_dependents();
+  if (late) late_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (ordered && warp == 0) {
+    for (int i = lane; i < DI_BUCKETS; i += 32) bucket_at[i] = 0;
+    __syncwarp();
+    for (int pass = 0; pass < 2; ++pass) {           // how many a bucket has, then where each goes
+      for (int b0 = 0; b0 < num_requests; b0 += 32) {
+        const int b = b0 + lane;
+        int bucket = -1;
+        if (b < num_requests) {
+          const int pos = context_lens[b] - 1, start = first_key(pos, window, ep) & ~(box_keys - 1);
+          const int tiles = cu_q[b + 1] - cu_q[b] == 1 ? (pos + 1 - start + DEC_TILE - 1) / DEC_TILE : 0;
+          bucket = DI_BUCKETS - 1 - max(0, min(DI_BUCKETS - 1, tiles));
+        }
+        const unsigned same = __match_any_sync(0xffffffffu, bucket);
+        const int rank = __popc(same & ((1u << lane) - 1)), at = bucket >= 0 ? bucket_at[bucket] : 0;
+        __syncwarp();
+        if (bucket >= 0) {
+          if (rank == 0) bucket_at[bucket] = at + __popc(same);
+          if (pass) order[at + rank] = (uint16_t)b;
+        }
+        __syncwarp();
+      }
+      if (pass == 0) {
+        int mine[DI_BUCKETS / 32], sum = 0;
+#pragma unroll
+        for (int i = 0; i < DI_BUCKETS / 32; ++i) { mine[i] = sum; sum += bucket_at[lane * (DI_BUCKETS / 32) + i]; }
+        int before = sum;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+          const int v = __shfl_up_sync(0xffffffffu, before, d);
+          if (lane >= d) before += v;
+        }
+        before -= sum;
+        __syncwarp();
+#pragma unroll
+        for (int i = 0; i < DI_BUCKETS / 32; ++i) bucket_at[lane * (DI_BUCKETS / 32) + i] = before + mine[i];
+        __syncwarp();
+      }
+    }
+  }
   if (threadIdx.x == 0) {
     for (int s = 0; s < DT_STAGES; ++s) { mbar_init(&full[s], 1); mbar_init(&empty[s], DEC_WARPS); }
     *abort_flag = 0;
@@ -564,7 +624,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
 
   if (warp == DEC_WARPS) {
     // ------------------------------------------------ producer: lane 0 issues, all lanes look pages up
-    bool ok = true, waited = false;                   // `waited`: this warp has waited for the kernels before this one
+    bool ok = true, waited = late != 0;               // `waited`: this warp has waited for the kernels before this one
     long ring = 0;                                    // stages armed so far, over all pairs: stage = ring % DT_STAGES
     int pairs = 0;                                    // pairs announced to the consumers
     int item = blockIdx.x;
@@ -574,7 +634,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       // yet draws after its tiles: the counter is this launch's only after the launches before it are done).
       int next = -1;
       bool drawn = false;
-      const int b = item / kvh, kh = item % kvh;
+      const int b = ordered ? order[item / kvh] : item / kvh, kh = item % kvh;
       const int t = cu_q[b];
       if (cu_q[b + 1] - t == 1) {                     // a decoding request (the others are the prefill kernel's)
         const int pos = context_lens[b] - 1;
@@ -664,7 +724,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
     // Every pair, and the entry that ends the list, takes a warp through the same two barriers, also a warp whose wait
     // ran out (it has raised the flag before it arrives); after the second barrier all four see the flag and leave.
-    pdl_wait();
+    if (!late) pdl_wait();
     const int g = lane >> 2, tq = lane & 3;
     const float sc = scale * LOG2E;
     long ring = 0;
@@ -772,6 +832,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       __threadfence();
     }
   }
+  if (late) pdl_wait();
 }
 #endif  // VOB_HD % 64 == 0
 
@@ -824,7 +885,7 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
                                    const int* cu_q, const int* context_lens, int num_requests, int nh, int kvh,
                                    int block_size, int window, float scale, long num_pages, int num_splits, float* scratch,
                                    unsigned* pairs_counter, int* err, cudaStream_t stream,
-                                   HeadEpilogue ep = head_options(0, nullptr, nullptr, 0, 0.f, 1.f, 0, 1)) {
+                                   HeadEpilogue ep = head_options(0, nullptr, nullptr, 0, 0.f, 1.f, 0, 1), int late = 0) {
   if (num_requests <= 0) return 0;
   if (kvh <= 0 || nh % kvh || nh / kvh > 16 || block_size <= 0 || num_splits < 1 || num_splits > 65535) return VOB_UNSUPPORTED;
   static bool configured = false;
@@ -875,7 +936,7 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
     // walk one range of keys and know no bias)
     if (num_splits == 1 && pairs_counter && !extras) {
       const int G = nh / kvh;
-      const int items_smem = 1024 + DT_STAGES * DT_STAGE_BYTES + DI_MERGE_FLOATS(G) * 4 + DI_QUEUE * 16 + 2 * DT_STAGES * 8 + 32;
+      const int items_smem = 1024 + DT_STAGES * DT_STAGE_BYTES + DI_MERGE_FLOATS(G) * 4 + DI_QUEUE * 16 + 2 * DT_STAGES * 8 + 32 + DI_ORDER_BYTES(G);
       static int resident_of[17] = {0};      // blocks that fit the GPU at once, by heads per kv head (0: not asked yet)
       if (!resident_of[G]) {
         static int items_configured = 0;
@@ -893,19 +954,19 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
         return launch_kernel(attention_decode_tma_items_kernel, dim3(resident_of[G]), DT_THREADS, items_smem, stream,
                              *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride,
                              (__nv_bfloat16*)out, block_tables, table_stride, cu_q, context_lens, num_requests, nh, kvh,
-                             block_size, window, scale, num_pages, box_keys, pairs_counter, err, ep);
+                             block_size, window, scale, num_pages, box_keys, pairs_counter, late, err, ep);
     }
     // up to 8 splits: the blocks of a (request, kv head) are a cluster and merge through shared memory
     if (num_splits > 1 && num_splits <= 8 && g_decode_cluster_merge)
       return launch_kernel_cluster(kernel, grid, DT_THREADS, tma_smem, stream, (unsigned)num_splits,
                                    *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride,
                                    (__nv_bfloat16*)out, block_tables, table_stride, cu_q, context_lens, nh, kvh, block_size,
-                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, err, ep);
+                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, late, err, ep);
     if (num_splits > 1 && !scratch) return VOB_BAD_ARGUMENT;
     rc = launch_kernel(kernel, grid, DT_THREADS, tma_smem, stream, *(const CUtensorMap*)map_k,
                        *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables,
                        table_stride, cu_q, context_lens, nh, kvh, block_size, window, scale, num_pages, part_o, part_lse,
-                       box_keys, 0, err, ep);
+                       box_keys, 0, late, err, ep);
     if (rc || num_splits == 1) return rc;
     return launch_kernel(attention_decode_combine_kernel, dim3(nh, num_requests), HD < 128 ? 64 : 128, 0, stream,
                          (const float*)part_o, (const float*)part_lse, (__nv_bfloat16*)out, cu_q, nh, num_splits, ep);
@@ -955,21 +1016,21 @@ VOB_API int vob_attention_decode_tma(const void* map_k, const void* map_v, const
 // keys of its own block of `chunk` positions; `window` is then not looked at), `value_div` > 1 (the value plane has
 // kvh / value_div heads and key head k reads value head k / value_div), `out_float` (out is float), `keep_first` > 0 (the
 // keys at positions below it are seen whatever the window) and `dist_bias` (float [nh, dist_rows]: a bias by the distance
-// between query and key).
+// between query and key).  `late`: the launch before it on this stream is vob_attention_prefill_tc5 with `lead`, for the same step.
 VOB_API int vob_attention_decode_ex(const void* map_k, const void* map_v, const void* q, long q_stride, void* out,
                                     const void* kcache, const void* vcache, const int* block_tables, int table_stride,
                                     const int* cu_q, const int* context_lens, int num_requests, int nh, int kvh,
                                     int block_size, int window, float scale, long num_pages, int num_splits,
                                     float* scratch, unsigned* pairs_counter, int sink, const float* sinks, const void* gate, long gate_stride,
                                     float softcap, int chunk, int value_div, int out_float, int keep_first,
-                                    const float* dist_bias, int dist_rows, int* err, cudaStream_t stream) {
+                                    const float* dist_bias, int dist_rows, int late, int* err, cudaStream_t stream) {
   if (value_div > 1 && kvh % value_div) return VOB_BAD_ARGUMENT;
   if (keep_first < 0 || (dist_bias && dist_rows <= 0)) return VOB_BAD_ARGUMENT;
   return attention_decode_launch(map_k, map_v, q, q_stride, out, kcache, vcache, block_tables, table_stride, cu_q,
                                  context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, num_splits,
                                  scratch, pairs_counter, err, stream,
                                  head_options(sink, sinks, gate, gate_stride, softcap, scale, chunk, value_div, out_float, keep_first,
-                                              dist_bias, dist_rows));
+                                              dist_bias, dist_rows), late);
 }
 
 VOB_API int vob_attention_decode_has_tma() { return VOB_HD % 64 == 0 ? 1 : 0; }

@@ -968,14 +968,15 @@ def attention_decode_scratch_floats(head_dim: int, num_requests: int, nh: int, n
 def attention_decode(q, q_stride, out, kcache, vcache, block_tables, cu_q, context_lens, num_requests, nh, kvh, hd,
                      window: int, scale: float, num_splits: int, scratch, err, use_tma: bool = True, pairs=None,
                      sink: bool = False, gate=None, gate_stride: int = 0, softcap: float = 0.0, chunk: int = 0,
-                     value_div: int = 1, keep_first: int = 0, dist_bias=None) -> None:
+                     value_div: int = 1, keep_first: int = 0, dist_bias=None, late: bool = False) -> None:
     """Requests that bring exactly one token; the others are skipped.  `pairs`: two int32 zeros on the device that belong
     to this caller (`decode_pairs_counter`); with it, one split and more (request, kv head) pairs than blocks fit the GPU
     run as persistent blocks that draw their pairs from it (the kernel leaves it at zero), without it as one block per
     pair.  Same bits either way.  `sink`, `gate`, `gate_stride`, `softcap`, `chunk`: as for paged_attention_generic.
     `value_div` > 1: `vcache` has kvh // value_div heads, and key head k reads value head k // value_div.  `out` is
     bfloat16 or float32.  `keep_first`, `dist_bias`: as for paged_attention_generic (with either, a block a pair).  A float tensor
-    [nh] as `sink` as there."""
+    [nh] as `sink` as there.  `late`: the launch before this one on the stream is `attention_prefill` with `lead` for the same step, and
+    has said that it leads; the two then run beside each other."""
     sink, sinks = _sinks(sink, nh)
     _cuda(q, out, kcache, vcache, block_tables, cu_q, context_lens, scratch, pairs, gate, dist_bias)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape[0] == nh)
@@ -993,7 +994,7 @@ def attention_decode(q, q_stride, out, kcache, vcache, block_tables, cu_q, conte
         block_tables.shape[-1], _p(cu_q), _p(context_lens), num_requests, nh, kvh, kcache.shape[2], window,
         ctypes.c_float(scale), ctypes.c_long(kcache.shape[0]), num_splits, _p(scratch), _p(pairs if map_k is not None else None),
         sink, sinks, _p(gate), ctypes.c_long(gate_stride), ctypes.c_float(softcap), int(chunk), int(value_div), int(out.dtype == torch.float32),
-        int(keep_first), _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[1], _p(err), _stream()),
+        int(keep_first), _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[1], int(bool(late)), _p(err), _stream()),
         "attention_decode_window_bias" if keep_first or dist_bias is not None else
         ("attention_decode_tma" if map_k is not None else "attention_decode"))
 
@@ -1008,14 +1009,15 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
                       hd, window: int, scale: float, err, use_tma: bool = True, use_tc5: bool = True,
                       query_tiles: int = 2, tiles_by_tma: bool = True, sink: bool = False, gate=None, gate_stride: int = 0,
                       softcap: float = 0.0, chunk: int = 0, value_div: int = 1, keep_first: int = 0, dist_bias=None,
-                      portions: int = 0, portion_tokens: int = 0) -> None:
+                      portions: int = 0, portion_tokens: int = 0, lead: bool = False) -> bool:
     """Requests that bring more than one token; the others are skipped.  `portions` and `portion_tokens`: how many such requests there
     are and their tokens, where the caller knows (the tcgen05 kernel then launches no block for the other requests).  Head sizes 64,
     128, 192 and 256 run on the tcgen05 tensor cores (`use_tc5`; `tiles_by_tma` False makes that kernel bring its query tiles in by
     cp.async and store its output row by row also where TMA could).  Their calls with a query stride that is no multiple of 8, and for
     heads of 192 and 256 also those with addresses or a scale that the kernel does not take, run on mma.sync with TMA copies
     (`use_tma`); other head sizes with cp.async.  `sink`, `gate`, `gate_stride`, `softcap`, `chunk`: as for paged_attention_generic;
-    `value_div`: as for attention_decode.  `keep_first`, `dist_bias`: as for paged_attention_generic; all three kernels take them."""
+    `value_div`: as for attention_decode.  `keep_first`, `dist_bias`: as for paged_attention_generic; all three kernels take them.
+    `lead`: the next launch on the stream will be `attention_decode` for the same step; the answer says whether it may be `late`."""
     _cuda(q, out, kcache, vcache, block_tables, cu_q, context_lens, gate, dist_bias)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape[0] == nh)
     assert q.dtype == torch.bfloat16 and kcache.dtype == torch.bfloat16 and (gate is None or gate.dtype == torch.bfloat16)
@@ -1042,9 +1044,9 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
                 map_k, map_v, map_q, map_o, _p(q), ctypes.c_long(q_stride), _p(out), _p(block_tables), block_tables.shape[-1], _p(cu_q),
                 _p(context_lens), num_requests, max_q, ctypes.c_long(portion_tokens), portions, nh, kvh, bs, window,
                 ctypes.c_float(scale), ctypes.c_long(kcache.shape[0]), query_tiles if hd <= 128 else 1, *extras, int(keep_first), _p(dist_bias),
-                0 if dist_bias is None else dist_bias.shape[1], int(kcache.data_ptr() == vcache.data_ptr() and value_div == 1), _p(err),
-                _stream()), "attention_prefill_window_bias" if keep_first or dist_bias is not None else "attention_prefill_tc5")
-            return
+                0 if dist_bias is None else dist_bias.shape[1], int(kcache.data_ptr() == vcache.data_ptr() and value_div == 1), int(bool(lead)),
+                _p(err), _stream()), "attention_prefill_window_bias" if keep_first or dist_bias is not None else "attention_prefill_tc5")
+            return bool(lead) and max_q > 1 and num_requests > 0
     _check(L.vob_attention_prefill_ex(
         map_k, map_v, _p(q), ctypes.c_long(q_stride), _p(out), _p(kcache), _p(vcache), _p(block_tables),
         block_tables.shape[-1], _p(cu_q), _p(context_lens), num_requests, max_q, nh, kvh, kcache.shape[2], window,
@@ -1052,6 +1054,7 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
         0 if dist_bias is None else dist_bias.shape[1], _p(err), _stream()),
         ("attention_prefill_window_bias" if keep_first or dist_bias is not None else
          ("attention_prefill_tma" if map_k is not None else "attention_prefill")))
+    return False
 
 
 def gemm_f32(a, w, out, bias=None) -> None:

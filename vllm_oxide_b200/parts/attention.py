@@ -239,6 +239,14 @@ def paged_attend(q, q_stride, out, keys, values, group: int, ctx, T: int, nh: in
                                         dist_bias=dist_bias)
         return values.shape[3] if own_values else (hd if value_dim is None else value_dim)
     B = ctx.launch_requests
+    late = False
+    if ctx.max_q > 1:
+        # the portions first: bound by their products and often by few blocks, where decoding is bound by memory; the two run side by side
+        late = kernels.attention_prefill(q, q_stride, out, keys, values, tables, ctx.cu_q, ctx.context_lens, B,
+                                         ctx.max_q, nh, kvh, hd, window, scale, ctx.err, sink=sink, gate=gate, gate_stride=gate_stride,
+                                         softcap=softcap, chunk=chunk, value_div=value_div, keep_first=keep_first, dist_bias=dist_bias,
+                                         portions=ctx.num_requests - ctx.num_decode, portion_tokens=ctx.num_tokens - ctx.num_decode,
+                                         lead=ctx.num_decode > 0)
     if ctx.num_decode > 0:
         n_keys = min(ctx.max_context, chunk or (window + keep_first if window else 0) or ctx.max_context)
         splits = decode_splits(B, kvh, n_keys, kernels.sm_count())
@@ -247,12 +255,7 @@ def paged_attend(q, q_stride, out, keys, values, group: int, ctx, T: int, nh: in
         kernels.attention_decode(q, q_stride, out, keys, values, tables, ctx.cu_q, ctx.context_lens, B, nh,
                                  kvh, hd, window, scale, splits, scratch, ctx.err, pairs=pairs, sink=sink, gate=gate,
                                  gate_stride=gate_stride, softcap=softcap, chunk=chunk, value_div=value_div,
-                                 keep_first=keep_first, dist_bias=dist_bias)
-    if ctx.max_q > 1:
-        kernels.attention_prefill(q, q_stride, out, keys, values, tables, ctx.cu_q, ctx.context_lens, B,
-                                  ctx.max_q, nh, kvh, hd, window, scale, ctx.err, sink=sink, gate=gate, gate_stride=gate_stride,
-                                  softcap=softcap, chunk=chunk, value_div=value_div, keep_first=keep_first, dist_bias=dist_bias,
-                                  portions=ctx.num_requests - ctx.num_decode, portion_tokens=ctx.num_tokens - ctx.num_decode)
+                                 keep_first=keep_first, dist_bias=dist_bias, late=late)
     return hd
 
 
