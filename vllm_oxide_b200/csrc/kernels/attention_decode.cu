@@ -542,7 +542,7 @@ constexpr int DI_DRAW_AHEAD = 2;                          // tiles before a pair
 constexpr int DI_QUEUE = 8;                               // entries; the producer is at most DT_STAGES + 1 pairs ahead
 // Pairs are given out with the longest requests first, so that the last to end are short ones: every block sorts up to DI_ORDERED
 // requests by their tiles (in 256 steps; equal ones stay in the batch's order, so every block finds the same), before the kernels ahead are done.
-// (224 requests of 40 to 1,152 keys, 8 x 2 heads of 128: 100 us, 111 in the order of the batch, both beside portions.)
+// (224 requests of 40 to 1,152 keys, 8 x 2 heads of 128, and five portions: with the late start 136 us a layer, 143 without either.)
 constexpr int DI_ORDERED = 1024, DI_BUCKETS = 256;
 // (from seven heads a key head on the sums' buffers leave no room for it beside a second block)
 constexpr int DI_ORDER_BYTES(int G) { return G <= 6 ? DI_BUCKETS * 4 + DI_ORDERED * 2 : 0; }
@@ -902,8 +902,8 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
   int rc;
 #if VOB_HD % 64 == 0
   const int extras = ep.keep_first || ep.dist_bias;
-  // Heads of 192 leave one block of this kernel on an SM (its registers), two of the cp.async kernel, which answers these calls where there
-  // are more blocks than SMs (24 requests of 600 keys, 4 heads, 3 splits: 21 us, 29 here; 40, 1 head, 4 splits: 23 and 30; 8 requests, 4
+  // Heads of 192 left one block of this kernel on an SM when this was measured (since then two: DecodeShape), two of the cp.async kernel, which
+  // answers these calls where there are more blocks than SMs (24 requests of 600 keys, 4 heads, 3 splits: 21 us, 29 here; 40, 1 head, 4 splits: 23 and 30; 8 requests, 4
   // splits, fit: 14 and 9).
   const bool second_places = HD == 192 && extras && (long)num_splits * kvh * num_requests > sm_count() && (num_splits == 1 || scratch);
   if (map_k && map_v && block_size % 16 == 0 && !second_places) {
