@@ -205,19 +205,21 @@ template <bool EXTRAS, bool SHARED, bool DENSE> struct DecodeShape {
 // has seen the kernels before it complete (attention_prefill_tc5_kernel: lead), needs nothing that it makes, writes other rows, and waits
 // for it at its own end only, so that who waits for this kernel waits for both.  The first look at what those kernels wrote is made past
 // this SM's L1, and by the copy engine behind a proxy fence.
+// (An instance of its own: a flag that is looked at while the kernel runs costs a step without portions 4 to 8 us of 28 layers: Qwen3-0.6B,
+// 1, 4 and 8 requests, 725, 897 and 904 us with the flag, 721, 890 and 900 without.)
 __device__ __forceinline__ void late_start() {
   __threadfence();
   asm volatile("fence.proxy.async;\n" ::: "memory");
 }
 
-template <bool EXTRAS, bool SHARED, bool DENSE>
+template <bool EXTRAS, bool SHARED, bool DENSE, bool LATE>
 __global__ void __launch_bounds__(DT_THREADS, DecodeShape<EXTRAS, SHARED, DENSE>::BLOCKS)
 attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                             const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                             const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                             const int* __restrict__ context_lens, int nh, int kvh, int block_size, int window, float scale,
                             long num_pages, float* part_o, float* part_lse,
-                            int box_keys, int cluster, int late, int* err, HeadEpilogue ep) {
+                            int box_keys, int cluster, int* err, HeadEpilogue ep) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   using SHAPE = DecodeShape<EXTRAS, SHARED, DENSE>;
@@ -228,7 +230,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   uint64_t* empty = full + STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + STAGES);
   pdl_launch_dependents();
-  if (late) late_start();
+  if (LATE) late_start();
   const int split = blockIdx.x, num_splits = gridDim.x, kh = blockIdx.y, b = blockIdx.z;
   const int t = cu_q[b];
   const int t_next = cu_q[b + 1], context = context_lens[b];
@@ -281,7 +283,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
           if (it >= STAGES) ok = mbar_wait(&empty[s], (unsigned)(((it / STAGES) - 1) & 1), abort_flag, err);
           if (ok) {
             const int tile_start = km.real(start + it * DEC_TILE);
-            if (!waited && tile_start + DEC_TILE > pos) { if (!late) pdl_wait(); waited = true; }
+            if (!waited && tile_start + DEC_TILE > pos) { if (!LATE) pdl_wait(); waited = true; }
             mbar_expect_tx(&full[s], (unsigned)STAGE_BYTES);
             char* kt = smem + s * STAGE_BYTES;
             if (box_keys == DEC_TILE) {
@@ -326,7 +328,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     }
   } else {
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
-    if (!late) pdl_wait();
+    if (!LATE) pdl_wait();
     const int g = lane >> 2, tq = lane & 3;
     uint32_t qf[QUERIES ? 1 : KSTEPS][4];
     if constexpr (QUERIES) {
@@ -393,10 +395,10 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       if (lane == 0) mbar_arrive(&empty[s]);
     }
   }
-  if (!late) pdl_wait();  // (a no-op for threads that have waited) nothing is written before the kernels before are done
+  if (!LATE) pdl_wait();  // (a no-op for threads that have waited) nothing is written before the kernels before are done
   __syncthreads();        // every stage has been read (or given up): the merge may reuse the memory
   const bool aborted = *abort_flag != 0;
-  if (aborted && !cluster) { if (late) pdl_wait(); return; }
+  if (aborted && !cluster) { if (LATE) pdl_wait(); return; }
   float* wm = reinterpret_cast<float*>(smem);                 // [DEC_WARPS][16]
   float* wl = wm + DEC_WARPS * 16;
   float* wo = wl + DEC_WARPS * 16;                            // [DEC_WARPS][16][HD]
@@ -474,7 +476,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       if (d == 0) part_lse[p] = lse;
     }
   }
-  if (num_splits == 1 || !cluster) { if (late) pdl_wait(); return; }
+  if (num_splits == 1 || !cluster) { if (LATE) pdl_wait(); return; }
   // The blocks of a (request, kv head) form a thread-block cluster: each reads the others' results from their shared
   // memory and merges a share of the outputs (weights 2^(lse - max lse), in the order of the splits).  Every block
   // of the cluster comes to both barriers, also one that gave up (its log-sum-exp is -inf: weight zero).
@@ -517,7 +519,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   // nobody may leave while another block still reads its shared memory
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-  if (late) pdl_wait();   // it ends behind the kernel that it works beside
+  if (LATE) pdl_wait();   // it ends behind the kernel that it works beside
 }
 
 // ---- many decoding requests, one split each ---------------------------------------------------------------------------
@@ -547,12 +549,13 @@ constexpr int DI_ORDERED = 1024, DI_BUCKETS = 256;
 // (from seven heads a key head on the sums' buffers leave no room for it beside a second block)
 constexpr int DI_ORDER_BYTES(int G) { return G <= 6 ? DI_BUCKETS * 4 + DI_ORDERED * 2 : 0; }
 
+template <bool LATE>
 __global__ void __launch_bounds__(DT_THREADS)
 attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const __grid_constant__ CUtensorMap tmV,
                                   const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                                   const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                                   const int* __restrict__ context_lens, int num_requests, int nh, int kvh, int block_size,
-                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, int late, int* err,
+                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, int* err,
                                   HeadEpilogue ep) {
   // pairs_taken[0]: pairs given out beyond the first of each block; [1]: blocks that have left
   extern __shared__ __align__(1024) char smem_raw[];
@@ -570,7 +573,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
   uint16_t* order = reinterpret_cast<uint16_t*>(bucket_at + DI_BUCKETS);                    // [num_requests], up to DI_ORDERED
   const bool ordered = num_requests <= DI_ORDERED && DI_ORDER_BYTES(G) > 0;
   pdl_launch_dependents();
-  if (late) late_start();
+  if (LATE) late_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (ordered && warp == 0) {
     for (int i = lane; i < DI_BUCKETS; i += 32) bucket_at[i] = 0;
@@ -624,7 +627,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
 
   if (warp == DEC_WARPS) {
     // ------------------------------------------------ producer: lane 0 issues, all lanes look pages up
-    bool ok = true, waited = late != 0;               // `waited`: this warp has waited for the kernels before this one
+    bool ok = true, waited = LATE;                    // `waited`: this warp has waited for the kernels before this one
     long ring = 0;                                    // stages armed so far, over all pairs: stage = ring % DT_STAGES
     int pairs = 0;                                    // pairs announced to the consumers
     int item = blockIdx.x;
@@ -724,7 +727,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
     // Every pair, and the entry that ends the list, takes a warp through the same two barriers, also a warp whose wait
     // ran out (it has raised the flag before it arrives); after the second barrier all four see the flag and leave.
-    if (!late) pdl_wait();
+    if (!LATE) pdl_wait();
     const int g = lane >> 2, tq = lane & 3;
     const float sc = scale * LOG2E;
     long ring = 0;
@@ -832,7 +835,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       __threadfence();
     }
   }
-  if (late) pdl_wait();
+  if (LATE) pdl_wait();
 }
 #endif  // VOB_HD % 64 == 0
 
@@ -911,13 +914,13 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
     const bool shared = HD >= 192 && kcache == vcache && ep.value_div == 1;
     const bool dense = HD == 128 && extras && (long)num_splits * kvh * num_requests > 2 * sm_count();
     const int form = extras + 2 * shared + 4 * dense;
-    static bool tma_configured[8] = {};
-    auto kernel = attention_decode_tma_kernel<false, false, false>;
+    static bool tma_configured[2][8] = {};
+    auto kernel = late ? attention_decode_tma_kernel<false, false, false, true> : attention_decode_tma_kernel<false, false, false, false>;
     int tma_smem = DecodeShape<false, false, false>::SMEM;
-#define VOB_FORM(X, S, D)                              \
-  if (form == (X) + 2 * (S) + 4 * (D)) {               \
-    kernel = attention_decode_tma_kernel<X, S, D>;     \
-    tma_smem = DecodeShape<X, S, D>::SMEM;             \
+#define VOB_FORM(X, S, D)                                                                                        \
+  if (form == (X) + 2 * (S) + 4 * (D)) {                                                                         \
+    kernel = late ? attention_decode_tma_kernel<X, S, D, true> : attention_decode_tma_kernel<X, S, D, false>;    \
+    tma_smem = DecodeShape<X, S, D>::SMEM;                                                                       \
   }
     VOB_FORM(true, false, false)
 #if VOB_HD >= 192
@@ -926,10 +929,10 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
     VOB_FORM(true, false, true)
 #endif
 #undef VOB_FORM
-    if (!tma_configured[form]) {
+    if (!tma_configured[late != 0][form]) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
       if (e != cudaSuccess) return (int)e;
-      tma_configured[form] = true;
+      tma_configured[late != 0][form] = true;
     }
     const int box_keys = block_size % DEC_TILE == 0 ? DEC_TILE : RUN_KEYS;
     // one split and more (request, kv head) pairs than blocks fit the GPU: persistent blocks, the producer ahead across pairs (they
@@ -937,36 +940,38 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
     if (num_splits == 1 && pairs_counter && !extras) {
       const int G = nh / kvh;
       const int items_smem = 1024 + DT_STAGES * DT_STAGE_BYTES + DI_MERGE_FLOATS(G) * 4 + DI_QUEUE * 16 + 2 * DT_STAGES * 8 + 32 + DI_ORDER_BYTES(G);
-      static int resident_of[17] = {0};      // blocks that fit the GPU at once, by heads per kv head (0: not asked yet)
-      if (!resident_of[G]) {
-        static int items_configured = 0;
-        if (items_configured < items_smem) {
-          cudaError_t e = cudaFuncSetAttribute(attention_decode_tma_items_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, items_smem);
+      auto items_kernel = late ? attention_decode_tma_items_kernel<true> : attention_decode_tma_items_kernel<false>;
+      static int resident_of[2][17] = {};      // blocks that fit the GPU at once, by heads per kv head (0: not asked yet)
+      int& resident = resident_of[late != 0][G];
+      if (!resident) {
+        static int items_configured[2] = {};
+        if (items_configured[late != 0] < items_smem) {
+          cudaError_t e = cudaFuncSetAttribute(items_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, items_smem);
           if (e != cudaSuccess) return (int)e;
-          items_configured = items_smem;
+          items_configured[late != 0] = items_smem;
         }
         int per_sm = 0;
-        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, attention_decode_tma_items_kernel, DT_THREADS, items_smem);
+        cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, items_kernel, DT_THREADS, items_smem);
         if (e != cudaSuccess) return (int)e;
-        resident_of[G] = (per_sm > 0 ? per_sm : 1) * sm_count();
+        resident = (per_sm > 0 ? per_sm : 1) * sm_count();
       }
-      if ((long)num_requests * kvh > resident_of[G])
-        return launch_kernel(attention_decode_tma_items_kernel, dim3(resident_of[G]), DT_THREADS, items_smem, stream,
-                             *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride,
-                             (__nv_bfloat16*)out, block_tables, table_stride, cu_q, context_lens, num_requests, nh, kvh,
-                             block_size, window, scale, num_pages, box_keys, pairs_counter, late, err, ep);
+      if ((long)num_requests * kvh > resident)
+        return launch_kernel(items_kernel, dim3(resident), DT_THREADS, items_smem, stream, *(const CUtensorMap*)map_k,
+                             *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables,
+                             table_stride, cu_q, context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, box_keys,
+                             pairs_counter, err, ep);
     }
     // up to 8 splits: the blocks of a (request, kv head) are a cluster and merge through shared memory
     if (num_splits > 1 && num_splits <= 8 && g_decode_cluster_merge)
       return launch_kernel_cluster(kernel, grid, DT_THREADS, tma_smem, stream, (unsigned)num_splits,
                                    *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride,
                                    (__nv_bfloat16*)out, block_tables, table_stride, cu_q, context_lens, nh, kvh, block_size,
-                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, late, err, ep);
+                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, err, ep);
     if (num_splits > 1 && !scratch) return VOB_BAD_ARGUMENT;
     rc = launch_kernel(kernel, grid, DT_THREADS, tma_smem, stream, *(const CUtensorMap*)map_k,
                        *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables,
                        table_stride, cu_q, context_lens, nh, kvh, block_size, window, scale, num_pages, part_o, part_lse,
-                       box_keys, 0, late, err, ep);
+                       box_keys, 0, err, ep);
     if (rc || num_splits == 1) return rc;
     return launch_kernel(attention_decode_combine_kernel, dim3(nh, num_requests), HD < 128 ? 64 : 128, 0, stream,
                          (const float*)part_o, (const float*)part_lse, (__nv_bfloat16*)out, cu_q, nh, num_splits, ep);
