@@ -202,14 +202,21 @@ template <bool EXTRAS, bool SHARED, bool DENSE> struct DecodeShape {
 };
 
 // A LATE kernel works beside the portions' attention of the same step, which it follows on the stream: it starts when every block of that one
-// has seen the kernels before it complete (attention_prefill_tc5_kernel: lead), needs nothing that it makes, writes other rows, and waits
-// for it at its own end only, so that who waits for this kernel waits for both.  The first look at what those kernels wrote is made past
-// this SM's L1, and by the copy engine behind a proxy fence.
+// has seen the kernels before it complete (attention_prefill_tc5_kernel: lead), learns of that itself by the ticket (wait_for_lead) where the
+// plain kernel waits for those kernels, needs nothing that the leading kernel makes, writes other rows, and waits for it at its own
+// end, so that who waits for this kernel waits for both.
 // (An instance of its own: a flag that is looked at while the kernel runs costs a step without portions 4 to 8 us of 28 layers: Qwen3-0.6B,
 // 1, 4 and 8 requests, 725, 897 and 904 us with the flag, 721, 890 and 900 without.)
-__device__ __forceinline__ void late_start() {
-  __threadfence();
-  asm volatile("fence.proxy.async;\n" ::: "memory");
+template <bool LATE>
+__device__ __forceinline__ void wait_for_inputs(const Handover& lead, int* err) {
+  if (LATE) wait_for_lead(lead, err);
+  else pdl_wait();
+}
+// The same for a whole warp, one lane of which looks (every thread of 296 blocks at one word: 2.7 us a layer).
+template <bool LATE>
+__device__ __forceinline__ void warp_wait_for_inputs(const Handover& lead, int lane, int* err) {
+  if (!LATE || lane == 0) wait_for_inputs<LATE>(lead, err);
+  if (LATE) __syncwarp();
 }
 
 template <bool EXTRAS, bool SHARED, bool DENSE, bool LATE>
@@ -219,7 +226,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
                             const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                             const int* __restrict__ context_lens, int nh, int kvh, int block_size, int window, float scale,
                             long num_pages, float* part_o, float* part_lse,
-                            int box_keys, int cluster, int* err, HeadEpilogue ep) {
+                            int box_keys, int cluster, Handover lead, int* err, HeadEpilogue ep) {
   extern __shared__ __align__(1024) char smem_raw[];
   char* smem = reinterpret_cast<char*>(((uintptr_t)smem_raw + 1023) & ~(uintptr_t)1023);
   using SHAPE = DecodeShape<EXTRAS, SHARED, DENSE>;
@@ -230,7 +237,6 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   uint64_t* empty = full + STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + STAGES);
   pdl_launch_dependents();
-  if (LATE) late_start();
   const int split = blockIdx.x, num_splits = gridDim.x, kh = blockIdx.y, b = blockIdx.z;
   const int t = cu_q[b];
   const int t_next = cu_q[b + 1], context = context_lens[b];
@@ -283,7 +289,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
           if (it >= STAGES) ok = mbar_wait(&empty[s], (unsigned)(((it / STAGES) - 1) & 1), abort_flag, err);
           if (ok) {
             const int tile_start = km.real(start + it * DEC_TILE);
-            if (!waited && tile_start + DEC_TILE > pos) { if (!LATE) pdl_wait(); waited = true; }
+            if (!waited && tile_start + DEC_TILE > pos) { wait_for_inputs<LATE>(lead, err); waited = true; }
             mbar_expect_tx(&full[s], (unsigned)STAGE_BYTES);
             char* kt = smem + s * STAGE_BYTES;
             if (box_keys == DEC_TILE) {
@@ -328,7 +334,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
     }
   } else {
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
-    if (!LATE) pdl_wait();
+    warp_wait_for_inputs<LATE>(lead, lane, err);
     const int g = lane >> 2, tq = lane & 3;
     uint32_t qf[QUERIES ? 1 : KSTEPS][4];
     if constexpr (QUERIES) {
@@ -555,7 +561,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
                                   const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                                   const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                                   const int* __restrict__ context_lens, int num_requests, int nh, int kvh, int block_size,
-                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, int* err,
+                                  int window, float scale, long num_pages, int box_keys, unsigned* pairs_taken, Handover lead, int* err,
                                   HeadEpilogue ep) {
   // pairs_taken[0]: pairs given out beyond the first of each block; [1]: blocks that have left
   extern __shared__ __align__(1024) char smem_raw[];
@@ -573,7 +579,6 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
   uint16_t* order = reinterpret_cast<uint16_t*>(bucket_at + DI_BUCKETS);                    // [num_requests], up to DI_ORDERED
   const bool ordered = num_requests <= DI_ORDERED && DI_ORDER_BYTES(G) > 0;
   pdl_launch_dependents();
-  if (LATE) late_start();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   if (ordered && warp == 0) {
     for (int i = lane; i < DI_BUCKETS; i += 32) bucket_at[i] = 0;
@@ -627,7 +632,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
 
   if (warp == DEC_WARPS) {
     // ------------------------------------------------ producer: lane 0 issues, all lanes look pages up
-    bool ok = true, waited = LATE;                    // `waited`: this warp has waited for the kernels before this one
+    bool ok = true, waited = false;             // `waited`: this warp has waited for the kernels before this one
     long ring = 0;                                    // stages armed so far, over all pairs: stage = ring % DT_STAGES
     int pairs = 0;                                    // pairs announced to the consumers
     int item = blockIdx.x;
@@ -662,7 +667,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
             if (ok) {
               const int tile_start = start + it * DEC_TILE;
               // only the tile that holds this step's key waits for the kernels before this one (once for the block)
-              if (!waited && tile_start + DEC_TILE > pos) { pdl_wait(); waited = true; }
+              if (!waited && tile_start + DEC_TILE > pos) { wait_for_inputs<LATE>(lead, err); waited = true; }
               if (it == 0) queue[pairs % DI_QUEUE] = make_int4(item, t, pos, 0);   // before the arrival below releases it
               mbar_expect_tx(&full[s], (unsigned)DT_STAGE_BYTES);
               char* kt = smem + s * DT_STAGE_BYTES;
@@ -700,7 +705,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       }
       if (!ok) break;
       if (!drawn && lane == 0) {
-        if (!waited) pdl_wait();
+        if (!waited) wait_for_inputs<LATE>(lead, err);
         next = (int)min((unsigned)num_items, gridDim.x + atomicAdd(&pairs_taken[0], 1u));
       }
       waited = true;
@@ -727,7 +732,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
     // ------------------------------------------------ consumers: warp w takes keys 16w..16w+15 of every tile
     // Every pair, and the entry that ends the list, takes a warp through the same two barriers, also a warp whose wait
     // ran out (it has raised the flag before it arrives); after the second barrier all four see the flag and leave.
-    if (!LATE) pdl_wait();
+    warp_wait_for_inputs<LATE>(lead, lane, err);
     const int g = lane >> 2, tq = lane & 3;
     const float sc = scale * LOG2E;
     long ring = 0;
@@ -888,8 +893,9 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
                                    const int* cu_q, const int* context_lens, int num_requests, int nh, int kvh,
                                    int block_size, int window, float scale, long num_pages, int num_splits, float* scratch,
                                    unsigned* pairs_counter, int* err, cudaStream_t stream,
-                                   HeadEpilogue ep = head_options(0, nullptr, nullptr, 0, 0.f, 1.f, 0, 1), int late = 0) {
+                                   HeadEpilogue ep = head_options(0, nullptr, nullptr, 0, 0.f, 1.f, 0, 1), Handover lead = Handover{nullptr, 0}) {
   if (num_requests <= 0) return 0;
+  const bool late = lead.word != nullptr;
   if (kvh <= 0 || nh % kvh || nh / kvh > 16 || block_size <= 0 || num_splits < 1 || num_splits > 65535) return VOB_UNSUPPORTED;
   static bool configured = false;
   const int merge_bytes = (2 * DEC_WARPS * 16 + DEC_WARPS * 16 * HD) * (int)sizeof(float);
@@ -929,10 +935,10 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
     VOB_FORM(true, false, true)
 #endif
 #undef VOB_FORM
-    if (!tma_configured[late != 0][form]) {
+    if (!tma_configured[late][form]) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
       if (e != cudaSuccess) return (int)e;
-      tma_configured[late != 0][form] = true;
+      tma_configured[late][form] = true;
     }
     const int box_keys = block_size % DEC_TILE == 0 ? DEC_TILE : RUN_KEYS;
     // one split and more (request, kv head) pairs than blocks fit the GPU: persistent blocks, the producer ahead across pairs (they
@@ -942,13 +948,13 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
       const int items_smem = 1024 + DT_STAGES * DT_STAGE_BYTES + DI_MERGE_FLOATS(G) * 4 + DI_QUEUE * 16 + 2 * DT_STAGES * 8 + 32 + DI_ORDER_BYTES(G);
       auto items_kernel = late ? attention_decode_tma_items_kernel<true> : attention_decode_tma_items_kernel<false>;
       static int resident_of[2][17] = {};      // blocks that fit the GPU at once, by heads per kv head (0: not asked yet)
-      int& resident = resident_of[late != 0][G];
+      int& resident = resident_of[late][G];
       if (!resident) {
         static int items_configured[2] = {};
-        if (items_configured[late != 0] < items_smem) {
+        if (items_configured[late] < items_smem) {
           cudaError_t e = cudaFuncSetAttribute(items_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, items_smem);
           if (e != cudaSuccess) return (int)e;
-          items_configured[late != 0] = items_smem;
+          items_configured[late] = items_smem;
         }
         int per_sm = 0;
         cudaError_t e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, items_kernel, DT_THREADS, items_smem);
@@ -959,19 +965,19 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
         return launch_kernel(items_kernel, dim3(resident), DT_THREADS, items_smem, stream, *(const CUtensorMap*)map_k,
                              *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables,
                              table_stride, cu_q, context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, box_keys,
-                             pairs_counter, err, ep);
+                             pairs_counter, lead, err, ep);
     }
     // up to 8 splits: the blocks of a (request, kv head) are a cluster and merge through shared memory
     if (num_splits > 1 && num_splits <= 8 && g_decode_cluster_merge)
       return launch_kernel_cluster(kernel, grid, DT_THREADS, tma_smem, stream, (unsigned)num_splits,
                                    *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride,
                                    (__nv_bfloat16*)out, block_tables, table_stride, cu_q, context_lens, nh, kvh, block_size,
-                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, err, ep);
+                                   window, scale, num_pages, part_o, part_lse, box_keys, 1, lead, err, ep);
     if (num_splits > 1 && !scratch) return VOB_BAD_ARGUMENT;
     rc = launch_kernel(kernel, grid, DT_THREADS, tma_smem, stream, *(const CUtensorMap*)map_k,
                        *(const CUtensorMap*)map_v, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables,
                        table_stride, cu_q, context_lens, nh, kvh, block_size, window, scale, num_pages, part_o, part_lse,
-                       box_keys, 0, err, ep);
+                       box_keys, 0, lead, err, ep);
     if (rc || num_splits == 1) return rc;
     return launch_kernel(attention_decode_combine_kernel, dim3(nh, num_requests), HD < 128 ? 64 : 128, 0, stream,
                          (const float*)part_o, (const float*)part_lse, (__nv_bfloat16*)out, cu_q, nh, num_splits, ep);
@@ -1021,22 +1027,26 @@ VOB_API int vob_attention_decode_tma(const void* map_k, const void* map_v, const
 // keys of its own block of `chunk` positions; `window` is then not looked at), `value_div` > 1 (the value plane has
 // kvh / value_div heads and key head k reads value head k / value_div), `out_float` (out is float), `keep_first` > 0 (the
 // keys at positions below it are seen whatever the window) and `dist_bias` (float [nh, dist_rows]: a bias by the distance
-// between query and key).  `late`: the launch before it on this stream is vob_attention_prefill_tc5 with `lead`, for the same step.
+// between query and key).  `lead_word` (may be null) and `lead_ticket`: the launch before this one on the stream is
+// vob_attention_prefill_tc5 with the same two, for the same step.
 VOB_API int vob_attention_decode_ex(const void* map_k, const void* map_v, const void* q, long q_stride, void* out,
                                     const void* kcache, const void* vcache, const int* block_tables, int table_stride,
                                     const int* cu_q, const int* context_lens, int num_requests, int nh, int kvh,
                                     int block_size, int window, float scale, long num_pages, int num_splits,
                                     float* scratch, unsigned* pairs_counter, int sink, const float* sinks, const void* gate, long gate_stride,
                                     float softcap, int chunk, int value_div, int out_float, int keep_first,
-                                    const float* dist_bias, int dist_rows, int late, int* err, cudaStream_t stream) {
+                                    const float* dist_bias, int dist_rows, unsigned* lead_word, unsigned lead_ticket, int* err, cudaStream_t stream) {
   if (value_div > 1 && kvh % value_div) return VOB_BAD_ARGUMENT;
   if (keep_first < 0 || (dist_bias && dist_rows <= 0)) return VOB_BAD_ARGUMENT;
   return attention_decode_launch(map_k, map_v, q, q_stride, out, kcache, vcache, block_tables, table_stride, cu_q,
                                  context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, num_splits,
                                  scratch, pairs_counter, err, stream,
                                  head_options(sink, sinks, gate, gate_stride, softcap, scale, chunk, value_div, out_float, keep_first,
-                                              dist_bias, dist_rows), late);
+                                              dist_bias, dist_rows), Handover{lead_word, lead_ticket});
 }
+
+// For tests: how often this file's waits try before they give up (0: as often as ever).
+VOB_API int vob_attention_decode_set_wait_limit(unsigned tries) { return set_wait_limit(tries, 0); }
 
 VOB_API int vob_attention_decode_has_tma() { return VOB_HD % 64 == 0 ? 1 : 0; }
 VOB_API int vob_attention_decode_box_keys(int block_size) { return block_size % DEC_TILE == 0 ? DEC_TILE : RUN_KEYS; }

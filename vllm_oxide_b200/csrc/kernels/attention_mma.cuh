@@ -405,4 +405,26 @@ struct WarpPages {
   __device__ __forceinline__ int page(int it, int run) const { return __shfl_sync(0xffffffffu, cur, ((it & 7) << 2) + run); }
 };
 
+// Attention of a step's portions that leads, and of its decoding requests that is late (attention_decode.cu): the two run beside each other.
+// The late kernel may start before the leading one has ended, so it learns from a word in device memory, not from the order of
+// launches, that the kernels before both are done: the first block of the leading kernel, behind its own wait for them, writes the launch's
+// ticket with release, and a thread of the late kernel that needs what they wrote reads it with acquire first.  A ticket is used once.
+struct Handover {
+  unsigned* word;        // null: neither leads nor is late
+  unsigned ticket;
+};
+__device__ __forceinline__ void give_lead(const Handover& h) {
+  __threadfence();
+  asm volatile("st.release.gpu.global.u32 [%0], %1;\n" ::"l"(h.word), "r"(h.ticket) : "memory");
+}
+// (The late kernel starts when every block of the leading one has come past that write or is about to: the wait is short, and bounded
+// all the same.)  The proxy fence is for who goes on with copies by the copy engine.
+__device__ __forceinline__ void wait_for_lead(const Handover& h, int* err) {
+  const unsigned limit = vob_wait_limit;
+  unsigned seen = h.ticket + 1;
+  for (unsigned i = 0; i < limit && seen != h.ticket; ++i) asm volatile("ld.acquire.gpu.global.u32 %0, [%1];\n" : "=r"(seen) : "l"(h.word) : "memory");
+  if (seen != h.ticket) atomicOr(err, VOB_ERR_TIMEOUT_BITS);
+  asm volatile("fence.proxy.async;\n" ::: "memory");
+}
+
 }  // namespace vob

@@ -111,7 +111,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
                              const __nv_bfloat16* q, long q_stride, __nv_bfloat16* out,
                              const int* __restrict__ block_tables, int table_stride, const int* __restrict__ cu_q,
                              const int* __restrict__ context_lens, int num_requests, int nh, int kvh, int block_size,
-                             int window, float scale, long num_pages, int box_keys, int lead, int* err, HeadEpilogue ep) {
+                             int window, float scale, long num_pages, int box_keys, Handover lead, int* err, HeadEpilogue ep) {
   using C = F5<NQ, ONE_PLANE>;
   constexpr int ST = C::STAGES, F5_STAGE_BYTES = C::STAGE_BYTES;
   constexpr int V_OFF = ONE_PLANE ? 0 : F5_KV_BYTES;        // where a stage's values lie
@@ -131,7 +131,7 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(o_staged + NQ);
   volatile int* abort_flag = reinterpret_cast<volatile int*>(tmem_slot + 1);
 
-  if (!lead) pdl_launch_dependents();
+  if (!lead.word) pdl_launch_dependents();
   // blockIdx.x = row block * kv heads + kv head: the blocks of all heads that see a request's most keys start first
   const int kh = blockIdx.x % kvh;
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
@@ -140,7 +140,11 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
   // left are zeros that nobody reads).  So a tile never ends inside a token, and one box of a tensor map is a tile.
   const int TT = F5_ROWS / G, TR = TT * G;
   PortionBlock at;
-  if (!find_portion(cu_q, num_requests, (int)blockIdx.x / kvh, NQ * TT, lane, at)) { pdl_wait(); return; }     // nothing left (uniform)
+  if (!find_portion(cu_q, num_requests, (int)blockIdx.x / kvh, NQ * TT, lane, at)) {      // nothing left (uniform)
+    pdl_wait();
+    if (lead.word && blockIdx.x == 0 && threadIdx.x == 0) give_lead(lead);
+    return;
+  }
   const int b = at.b, t0 = at.t0, n = at.n, tok_base = at.tok_base;
   const int ctx = context_lens[b];
   const int first_pos = ctx - n;
@@ -188,9 +192,12 @@ attention_prefill_tc5_kernel(const __grid_constant__ CUtensorMap tmK, const __gr
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   __syncthreads();                              // the barriers are there: the producer starts on the first keys and values
   pdl_wait();                                   // the kernels before this one wrote q and this portion's keys and values
-  // `lead`: the decode kernel that follows works beside this one and waits for nothing before its end (attention_decode.cu: late), so it
-  // may start when the kernels before this one are done
-  if (lead) pdl_launch_dependents();
+  // `lead`: the decode kernel that follows works beside this one (attention_decode.cu: LATE) and may start when the kernels before this one
+  // are done
+  if (lead.word) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) give_lead(lead);
+    pdl_launch_dependents();
+  }
   uint32_t tmem_base = 0;
   if (warp != 4 * NQ) {
     if (warp == 4 * NQ + 1) t5_alloc(tmem_slot, C::TMEM_COLS);
@@ -610,13 +617,16 @@ VOB_API int vob_attention_prefill_has_tc5() {
 // `query_tiles` is 1 or, for heads of up to 128, 2: how many tiles of 128 query rows a block takes.  `sink`: the softmax has a
 // silent extra entry of score 0, or (`sinks`, float [nh] or null) of the head's own score; `gate` (bfloat16, may be null): head h of token t is multiplied by
 // sigmoid(gate[t * gate_stride + h]).  `softcap`, `chunk`, `value_div`, `out_float`, `keep_first`, `dist_bias`: as for
-// vob_attention_prefill_ex.  `lead`: the next launch on the stream is vob_attention_decode_ex with `late`, for the same step.
+// vob_attention_prefill_ex.  `lead_word` (may be
+// null) and `lead_ticket`: the next launch on the stream is vob_attention_decode_ex with the same two, for the same step; the word, four
+// bytes of device memory, belongs to this stream, and no two launches on it have the same ticket.
 VOB_API int vob_attention_prefill_tc5(const void* map_k, const void* map_v, const void* map_q, const void* map_o, const void* q, long q_stride, void* out,
                                       const int* block_tables, int table_stride, const int* cu_q, const int* context_lens,
                                       int num_requests, int max_q, long portion_tokens, int portions, int nh, int kvh, int block_size, int window, float scale,
                                       long num_pages, int query_tiles, int sink, const float* sinks, const void* gate, long gate_stride,
                                       float softcap, int chunk, int value_div, int out_float, int keep_first,
-                                      const float* dist_bias, int dist_rows, int one_plane, int lead, int* err, cudaStream_t stream) {
+                                      const float* dist_bias, int dist_rows, int one_plane, unsigned* lead_word, unsigned lead_ticket, int* err,
+                                      cudaStream_t stream) {
 #if VOB_HD % 64 == 0
   const HeadEpilogue ep = head_options(sink, sinks, gate, gate_stride, softcap, scale, chunk, value_div, out_float, keep_first, dist_bias,
                                        dist_rows);
@@ -652,7 +662,8 @@ VOB_API int vob_attention_prefill_tc5(const void* map_k, const void* map_v, cons
                          F5<NN, PP>::SMEM_BYTES, stream, *(const CUtensorMap*)map_k, *(const CUtensorMap*)map_v,            \
                          *(const CUtensorMap*)(q_by_tma ? map_q : map_k), q_by_tma, *(const CUtensorMap*)(o_by_tma ? map_o : map_k), \
                          o_by_tma, (const __nv_bfloat16*)q, q_stride, (__nv_bfloat16*)out, block_tables, table_stride, cu_q, \
-                         context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, box_keys, lead, err, ep); \
+                         context_lens, num_requests, nh, kvh, block_size, window, scale, num_pages, box_keys, \
+                         Handover{lead_word, lead_ticket}, err, ep);                                                        \
   } while (0)
 #if VOB_HD <= 128
   if (query_tiles == 2) VOB_F5(2, false);

@@ -976,7 +976,7 @@ def attention_decode(q, q_stride, out, kcache, vcache, block_tables, cu_q, conte
     `value_div` > 1: `vcache` has kvh // value_div heads, and key head k reads value head k // value_div.  `out` is
     bfloat16 or float32.  `keep_first`, `dist_bias`: as for paged_attention_generic (with either, a block a pair).  A float tensor
     [nh] as `sink` as there.  `late`: the launch before this one on the stream is `attention_prefill` with `lead` for the same step, and
-    has said that it leads; the two then run beside each other."""
+    has said that it leads; the two then run beside each other.  Refused where no such launch is outstanding on the stream."""
     sink, sinks = _sinks(sink, nh)
     _cuda(q, out, kcache, vcache, block_tables, cu_q, context_lens, scratch, pairs, gate, dist_bias)
     assert dist_bias is None or (dist_bias.dtype == torch.float32 and dist_bias.is_contiguous() and dist_bias.shape[0] == nh)
@@ -994,9 +994,63 @@ def attention_decode(q, q_stride, out, kcache, vcache, block_tables, cu_q, conte
         block_tables.shape[-1], _p(cu_q), _p(context_lens), num_requests, nh, kvh, kcache.shape[2], window,
         ctypes.c_float(scale), ctypes.c_long(kcache.shape[0]), num_splits, _p(scratch), _p(pairs if map_k is not None else None),
         sink, sinks, _p(gate), ctypes.c_long(gate_stride), ctypes.c_float(softcap), int(chunk), int(value_div), int(out.dtype == torch.float32),
-        int(keep_first), _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[1], int(bool(late)), _p(err), _stream()),
+        int(keep_first), _p(dist_bias), 0 if dist_bias is None else dist_bias.shape[1], *_late_handover(late), _p(err), _stream()),
         "attention_decode_window_bias" if keep_first or dist_bias is not None else
         ("attention_decode_tma" if map_k is not None else "attention_decode"))
+
+
+def attention_decode_set_wait_limit(head_dim: int, tries: int) -> None:
+    """For tests: how often the waits of decode attention try before they give up (0: as often as ever)."""
+    L = attention_lib(head_dim)
+    code = L.vob_attention_decode_set_wait_limit(ctypes.c_uint(tries))
+    if code != 0:
+        raise KernelError(f"attention_decode_set_wait_limit: {lib().vob_error_string(code).decode()}")
+
+
+class _Handover:
+    """The word in device memory through which an `attention_prefill` that leads lets the `attention_decode` behind it start, one for a stream:
+    every pair of launches has a ticket of its own, and the word holds the last one given."""
+
+    def __init__(self, device):
+        self.word, self.ticket, self.outstanding = torch.zeros(1, dtype=torch.int32, device=device), 0, False
+
+
+MAX_HANDOVERS = 64      # streams that have one; a step on any further stream runs its two kernels one after the other
+_handovers = {}         # (device, stream handle) -> _Handover
+
+
+def _handover_key():
+    # (asked for twice a layer of an eager step, which the host may hold up: the handle alone, without a Stream object)
+    index = torch.cuda.current_device()
+    return index, torch._C._cuda_getCurrentRawStream(index)
+
+
+def _next_handover(device) -> Optional[_Handover]:
+    """The current stream's, with a new ticket; None while the stream is captured (a replay would use a ticket twice)."""
+    if torch.cuda.is_current_stream_capturing():
+        return None
+    key = _handover_key()
+    h = _handovers.get(key)
+    if h is None:
+        if len(_handovers) >= MAX_HANDOVERS:
+            return None
+        h = _handovers.setdefault(key, _Handover(device))
+    h.ticket, h.outstanding = h.ticket % 0x7fffffff + 1, False
+    return h
+
+
+def _handover_args(h: Optional[_Handover]):
+    return (_p(h.word), ctypes.c_uint(h.ticket)) if h is not None else (None, ctypes.c_uint(0))
+
+
+def _late_handover(late: bool):
+    if not late:
+        return _handover_args(None)
+    h = _handovers.get(_handover_key())
+    if h is None or not h.outstanding:
+        raise KernelError("attention_decode cannot be late: no attention_prefill that leads is outstanding on this stream")
+    h.outstanding = False
+    return _handover_args(h)
 
 
 def decode_pairs_counter(device) -> torch.Tensor:
@@ -1040,13 +1094,16 @@ def attention_prefill(q, q_stride, out, kcache, vcache, block_tables, cu_q, cont
             map_q = tensor_map_heads(q, q_stride, nh, hd, box_heads, 128 // box_heads) if box_heads > 0 else None
             map_o = (tensor_map_heads(out, nh * hd, nh, hd, box_heads, 128 // box_heads)
                      if box_heads > 0 and out.is_contiguous() and out.data_ptr() % 16 == 0 and out.dtype == torch.bfloat16 else None)
+            handover = _next_handover(q.device) if lead and max_q > 1 and num_requests > 0 else None
             _check(L.vob_attention_prefill_tc5(
                 map_k, map_v, map_q, map_o, _p(q), ctypes.c_long(q_stride), _p(out), _p(block_tables), block_tables.shape[-1], _p(cu_q),
                 _p(context_lens), num_requests, max_q, ctypes.c_long(portion_tokens), portions, nh, kvh, bs, window,
                 ctypes.c_float(scale), ctypes.c_long(kcache.shape[0]), query_tiles if hd <= 128 else 1, *extras, int(keep_first), _p(dist_bias),
-                0 if dist_bias is None else dist_bias.shape[1], int(kcache.data_ptr() == vcache.data_ptr() and value_div == 1), int(bool(lead)),
-                _p(err), _stream()), "attention_prefill_window_bias" if keep_first or dist_bias is not None else "attention_prefill_tc5")
-            return bool(lead) and max_q > 1 and num_requests > 0
+                0 if dist_bias is None else dist_bias.shape[1], int(kcache.data_ptr() == vcache.data_ptr() and value_div == 1),
+                *_handover_args(handover), _p(err), _stream()), "attention_prefill_window_bias" if keep_first or dist_bias is not None else "attention_prefill_tc5")
+            if handover is not None:
+                handover.outstanding = True
+            return handover is not None
     _check(L.vob_attention_prefill_ex(
         map_k, map_v, _p(q), ctypes.c_long(q_stride), _p(out), _p(kcache), _p(vcache), _p(block_tables),
         block_tables.shape[-1], _p(cu_q), _p(context_lens), num_requests, max_q, nh, kvh, kcache.shape[2], window,
