@@ -204,7 +204,7 @@ template <bool EXTRAS, bool SHARED, bool DENSE> struct DecodeShape {
 // A LATE kernel works beside the portions' attention of the same step, which it follows on the stream: it starts when every block of that one
 // has seen the kernels before it complete (attention_prefill_tc5_kernel: lead), learns of that itself by the ticket (wait_for_lead) where the
 // plain kernel waits for those kernels, needs nothing that the leading kernel makes, writes other rows, and waits for it at its own
-// end, so that who waits for this kernel waits for both.
+// end, so that who waits for this kernel waits for both: its first block does, and the others leave their SMs to blocks that have not begun.
 // (An instance of its own: a flag that is looked at while the kernel runs costs a step without portions 4 to 8 us of 28 layers: Qwen3-0.6B,
 // 1, 4 and 8 requests, 725, 897 and 904 us with the flag, 721, 890 and 900 without.)
 template <bool LATE>
@@ -212,11 +212,15 @@ __device__ __forceinline__ void wait_for_inputs(const Handover& lead, int* err) 
   if (LATE) wait_for_lead(lead, err);
   else pdl_wait();
 }
-// The same for a whole warp, one lane of which looks (every thread of 296 blocks at one word: 2.7 us a layer).
+// The same for a whole warp, one lane of which looks (by every thread of 296 blocks the ticket costs 2.7 us a layer, so 1.7).
 template <bool LATE>
 __device__ __forceinline__ void warp_wait_for_inputs(const Handover& lead, int lane, int* err) {
   if (!LATE || lane == 0) wait_for_inputs<LATE>(lead, err);
   if (LATE) __syncwarp();
+}
+// The last thing that a thread of a late kernel does.
+__device__ __forceinline__ void end_behind_lead() {
+  if (blockIdx.x == 0 && blockIdx.y == 0 && blockIdx.z == 0) pdl_wait();
 }
 
 template <bool EXTRAS, bool SHARED, bool DENSE, bool LATE>
@@ -254,7 +258,11 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   // before this step's kernels began; the kernels of this step write this token's query, key and value only.
   // So the producer waits for the kernels before this one only when it comes to the tile that holds the new key,
   // and the consumers wait before they read the query: the older tiles stream in while those kernels still run.
-  if (t_next - t != 1) { pdl_wait(); return; }         // not a decoding request (uniform for the block)
+  if (t_next - t != 1) {                               // not a decoding request (uniform for the block)
+    if (LATE) end_behind_lead();
+    else pdl_wait();
+    return;
+  }
   const int G = nh / kvh;
   const int pos = context - 1;
   const int lo = first_key(pos, window, ep);
@@ -404,7 +412,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   if (!LATE) pdl_wait();  // (a no-op for threads that have waited) nothing is written before the kernels before are done
   __syncthreads();        // every stage has been read (or given up): the merge may reuse the memory
   const bool aborted = *abort_flag != 0;
-  if (aborted && !cluster) { if (LATE) pdl_wait(); return; }
+  if (aborted && !cluster) { if (LATE) end_behind_lead(); return; }
   float* wm = reinterpret_cast<float*>(smem);                 // [DEC_WARPS][16]
   float* wl = wm + DEC_WARPS * 16;
   float* wo = wl + DEC_WARPS * 16;                            // [DEC_WARPS][16][HD]
@@ -482,7 +490,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
       if (d == 0) part_lse[p] = lse;
     }
   }
-  if (num_splits == 1 || !cluster) { if (LATE) pdl_wait(); return; }
+  if (num_splits == 1 || !cluster) { if (LATE) end_behind_lead(); return; }
   // The blocks of a (request, kv head) form a thread-block cluster: each reads the others' results from their shared
   // memory and merges a share of the outputs (weights 2^(lse - max lse), in the order of the splits).  Every block
   // of the cluster comes to both barriers, also one that gave up (its log-sum-exp is -inf: weight zero).
@@ -525,7 +533,7 @@ attention_decode_tma_kernel(const __grid_constant__ CUtensorMap tmK, const __gri
   // nobody may leave while another block still reads its shared memory
   asm volatile("barrier.cluster.arrive.release.aligned;\n" ::: "memory");
   asm volatile("barrier.cluster.wait.acquire.aligned;\n" ::: "memory");
-  if (LATE) pdl_wait();   // it ends behind the kernel that it works beside
+  if (LATE) end_behind_lead();
 }
 
 // ---- many decoding requests, one split each ---------------------------------------------------------------------------
@@ -840,7 +848,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       __threadfence();
     }
   }
-  if (LATE) pdl_wait();
+  if (LATE) end_behind_lead();
 }
 #endif  // VOB_HD % 64 == 0
 
