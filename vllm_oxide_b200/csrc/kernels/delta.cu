@@ -173,14 +173,56 @@ short_conv_pairs_kernel(const T* x, long x_stride, const float* __restrict__ w, 
   const int req = token_req[t_first];
   const bool one = t_first + CONV_TOKENS <= num_tokens && req >= 0 && req == token_req[min(t_first + CONV_TOKENS, num_tokens) - 1];
   const int j = one ? t_first - cu_q[req] : 0, slot = one ? state_slots[req] : 0;
-  pdl_wait();
+  int place[CONV_TOKENS], slot_of[CONV_TOKENS];      // of several portions: a token's place in its own (-1: none) and its slot
   if (!one) {
 #pragma unroll
-    for (int e = 0; e < 2; ++e) {
-      const float all[DELTA_MAX_TAPS] = {wt[e][0], wt[e][1], wt[e][2], wt[e][3]};
-      conv_walk<T, TO>(x, x_stride, state, state_stride, conv_off, token_req, cu_q, state_slots, all, wt[e][3], b_in[e], b_out[e], out, t_first,
-                       num_tokens, CONV_TOKENS, c + e, C, 4, num_slots, act, err);
+    for (int k = 0; k < CONV_TOKENS; ++k) {
+      const int r = t_first + k < num_tokens ? token_req[t_first + k] : -1;
+      place[k] = r >= 0 ? t_first + k - cu_q[r] : -1;
+      slot_of[k] = r >= 0 ? state_slots[r] : 0;
     }
+  }
+  pdl_wait();
+  if (!one) {
+    // portions' edges, and every block of a step of short ones: all rows are asked for at once here too, a token then takes its inputs before
+    // its portion's start from its slot
+    typename P::Raw rows[3 + CONV_TOKENS];
+#pragma unroll
+    for (int s = 0; s < 3 + CONV_TOKENS; ++s)
+      if (s < 3 ? place[0] >= 3 - s : place[s - 3 < 0 ? 0 : s - 3] >= 0)
+        rows[s] = *reinterpret_cast<const typename P::Raw*>(x + (size_t)(t_first - 3 + s) * x_stride + c);
+    float o[CONV_TOKENS][2];
+    bool bad = false;
+#pragma unroll
+    for (int k = 0; k < CONV_TOKENS; ++k) {
+      if (place[k] < 0) continue;
+      if (slot_of[k] < 0 || slot_of[k] >= num_slots) {
+        bad = true;
+        place[k] = -1;
+        continue;
+      }
+      const float* st = state + (size_t)slot_of[k] * state_stride + conv_off;
+      o[k][0] = b_out[0];
+      o[k][1] = b_out[1];
+#pragma unroll
+      for (int s = 0; s < 4; ++s) {
+        float v[2];
+        if (place[k] >= 3 - s) {
+          const float2 r = P::get(rows[k + s]);
+          v[0] = r.x + b_in[0];
+          v[1] = r.y + b_in[1];
+        } else {
+          v[0] = st[(size_t)(place[k] + s) * C + c];
+          v[1] = st[(size_t)(place[k] + s) * C + c + 1];
+        }
+        o[k][0] = fmaf(wt[0][s], v[0], o[k][0]);
+        o[k][1] = fmaf(wt[1][s], v[1], o[k][1]);
+      }
+    }
+#pragma unroll
+    for (int k = 0; k < CONV_TOKENS; ++k)
+      if (place[k] >= 0) Pair2<TO>::put(out + (size_t)(t_first + k) * C + c, act ? silu_f(o[k][0]) : o[k][0], act ? silu_f(o[k][1]) : o[k][1]);
+    if (bad) atomicOr(err, VOB_ERR_SLOT);
     return;
   }
   if (slot < 0 || slot >= num_slots) {
