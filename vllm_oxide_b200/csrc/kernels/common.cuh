@@ -210,6 +210,21 @@ inline int launch_kernel_cluster(void (*kernel)(KArgs...), dim3 grid, dim3 block
   return (int)cudaGetLastError();
 }
 
+// How many clusters of `cluster_x` blocks of this kernel the device holds at once (0: it cannot be told).  Clusters lie inside a GPC, so
+// these are fewer than the SMs would give.
+template <typename... KArgs>
+inline int resident_clusters(void (*kernel)(KArgs...), int threads, size_t smem, unsigned cluster_x) {
+  cudaLaunchConfig_t cfg = {};
+  cfg.gridDim = dim3(cluster_x); cfg.blockDim = dim3(threads); cfg.dynamicSmemBytes = smem;
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = cluster_x; attr[0].val.clusterDim.y = 1; attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr; cfg.numAttrs = 1;
+  int n = 0;
+  if (cudaOccupancyMaxActiveClusters(&n, kernel, &cfg) != cudaSuccess) { cudaGetLastError(); return 0; }
+  return n;
+}
+
 // The number of SMs of the current device (asked once; launch shapes are derived from it, never from a literal).
 inline int sm_count() {
   static int sms = 0;

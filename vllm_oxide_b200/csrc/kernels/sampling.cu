@@ -13,6 +13,8 @@
 //     keeps a prefix of its sort, which is the same set unless equal logits straddle the
 //     boundary).  Probability mass is summed as 40-bit fixed point integers, so the set does
 //     not depend on the order of summation.
+#include <initializer_list>
+
 #include "cluster.cuh"
 
 namespace vob {
@@ -186,7 +188,10 @@ constexpr int SAMPLE_SHARED_K = 256;
 // memory and one reduction, where the digits of a key take four histograms with their barriers.
 constexpr int SAMPLE_FEW = 512;
 
-__global__ void __launch_bounds__(SAMPLE_THREADS)
+// MANY rows, more than there are SMs, a block each: two blocks share an SM, with 32 registers a thread.  (Top-k 50 and top-p 0.9, 149 rows of
+// 151,936 tokens 66 us, 82 in two rounds; 229: 78 and 86; 229 of 32,768: 39 and 45.)
+template <bool MANY>
+__global__ void __launch_bounds__(SAMPLE_THREADS, MANY ? 2 : 1)
 sample_kernel(const float* logits, long ld, int V, const float* __restrict__ temperature,
               const int* __restrict__ top_k, const float* __restrict__ top_p,
               const unsigned long long* __restrict__ keys, int* __restrict__ out, int blocks) {
@@ -281,15 +286,18 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       if (parts > 1) {
         meet();
         if (rank == 0) {
-          for (int r = 1; r < parts; ++r) {
-            bound = max(bound, *in_block(&s_bound, r));
-            gathered = gathered && *in_block(&s_ncand, r) <= (unsigned)SAMPLE_CANDIDATES;
-          }
-          for (int r = 1; r < parts && gathered; ++r) {
-            const unsigned n = *in_block(&s_ncand, r);
+          // a lane asks a block how it went, then some warps a block fetch its tokens: one behind the other these are a chain of latencies
+          // (8 rows of 32,768, top-k 50: 31 us and 35)
+          const int lane = tid & 31, r = (tid >> 5) % parts;
+          const unsigned has = lane < parts ? *in_block(&s_ncand, lane) : 0u, from = lane < parts ? *in_block(&s_bound, lane) : 0u;
+          bound = __reduce_max_sync(0xffffffffu, from);
+          gathered = __all_sync(0xffffffffu, has <= (unsigned)SAMPLE_CANDIDATES);
+          const unsigned n = gathered && r > 0 ? __shfl_sync(0xffffffffu, has, r) : 0u;
+          __syncthreads();      // (this block's own count grows from here on)
+          if (n > 0) {
             const volatile uint32_t* key = in_block(cand_key, r);
             const volatile uint32_t* idx = in_block(cand_idx, r);
-            for (unsigned c = tid; c < n; c += SAMPLE_THREADS) {
+            for (unsigned c = (tid >> 5) / parts * 32 + lane; c < n; c += SAMPLE_THREADS / parts) {
               const uint32_t x = key[c];
               if (x < bound) continue;
               const unsigned pos = atomicAdd(&s_ncand, 1u);
@@ -602,15 +610,25 @@ VOB_API int vob_sample(const float* logits, long ld, int R, int V, const float* 
   if (V <= 0) return VOB_BAD_ARGUMENT;
   const int smem = SAMPLE_CANDIDATES * 16;
   static bool configured = false;
+  static int rows_of[4] = {};      // rows that 1, 2, 4, 8 blocks each work on at once
   if (!configured) {
-    cudaError_t e = cudaFuncSetAttribute(sample_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
-    if (e != cudaSuccess) return (int)e;
+    for (auto kernel : {sample_kernel<false>, sample_kernel<true>}) {
+      cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+      if (e != cudaSuccess) return (int)e;
+    }
+    for (int i = 1; i < 4; ++i) rows_of[i] = resident_clusters(sample_kernel<false>, SAMPLE_THREADS, smem, 1u << i);
     configured = true;
   }
-  // blocks a row: as many (1, 2, 4, 8) as leave every block an SM, of at least four thousand tokens each
-  int blocks = 8;
-  while (blocks > 1 && ((long)R * blocks > sm_count() || V / blocks < 4 * SAMPLE_THREADS)) blocks /= 2;
-  return launch_kernel_cluster(sample_kernel, dim3((unsigned)(R * blocks)), SAMPLE_THREADS, smem, stream, (unsigned)blocks, logits, ld, V,
+  // Blocks a row: as many (8, 4, 2) as leave no row for a second round, of at least four thousand tokens each, else one.  Clusters lie inside a GPC,
+  // so those of 8 are 15 and not 18, those of 4 33 and not 37 (151,936 tokens, top-k 50: 16 rows by eight blocks 53 us, by four 33; 34 rows by four
+  // 47, by two 35; with top-p alone 252 and 209, 399 and 356).
+  int i = 3;
+  while (i > 0 && (R > rows_of[i] || V >> i < 4 * SAMPLE_THREADS)) --i;
+  const int blocks = 1 << i;
+  if (blocks == 1)
+    return launch_kernel(R > sm_count() ? sample_kernel<true> : sample_kernel<false>, dim3((unsigned)R), SAMPLE_THREADS, smem, stream, logits, ld, V,
+                         temperature, top_k, top_p, keys, out, blocks);
+  return launch_kernel_cluster(sample_kernel<false>, dim3((unsigned)(R * blocks)), SAMPLE_THREADS, smem, stream, (unsigned)blocks, logits, ld, V,
                                temperature, top_k, top_p, keys, out, blocks);
 }
 
