@@ -346,6 +346,7 @@ __device__ __forceinline__ int longest_first(const int* __restrict__ cu_q) {
   const int B = gridDim.z, lane = threadIdx.x & 31;
   if (B == 1 || B > 32) return blockIdx.z;
   const int mine = lane < B ? cu_q[lane + 1] - cu_q[lane] : -1;
+  if (__reduce_max_sync(0xffffffffu, mine) == __reduce_min_sync(0xffffffffu, lane < B ? mine : INT_MAX)) return blockIdx.z;      // decoding
   int rank = 0;
   for (int j = 0; j < B; ++j) {
     const int other = __shfl_sync(0xffffffffu, mine, j);
@@ -361,9 +362,12 @@ __device__ __forceinline__ int longest_first(const int* __restrict__ cu_q) {
 // unit vectors (laid out so that a thread finds its rows side by side), decay, beta and the block's slice of the values.
 // The two groups meet on named barriers: "full" when a buffer is ready, "empty" when its tokens have been walked.
 // AHEAD: a token's rows are asked for while the token before is worked on; without it a thread takes a quarter fewer registers and
-// three blocks share an SM, which is what many requests of one or few tokens wait for (their states come from memory).
+// three blocks share an SM, which is what many requests of one or few tokens wait for (their states come from memory).  With it two do,
+// also where the decay is one a row (left to itself the compiler takes 170 registers there, which is one block: a second
+// round from 149 blocks on.  One portion of 2,048 tokens, 32 heads of 128 x 128: 838 us, 1,438 with one; 333, 1,055 and 1,777, 16 heads:
+// 713 and 991; the loop before the read-outs went beside the exchange: 827 and 808).
 template <typename T, int LANES, int ROWS, bool CHD, bool AHEAD>
-__global__ void __launch_bounds__(DS_THREADS, ROWS != 16 ? 1 : (!AHEAD ? 3 : (CHD ? 1 : 2)))
+__global__ void __launch_bounds__(DS_THREADS, ROWS != 16 ? 1 : (AHEAD ? 2 : 3))
 delta_scan_kernel(const float* qkv, const T* ab, long ab_stride, int b_off, int a_off, const float* __restrict__ A_log,
                   const float* __restrict__ dt_bias, float* state, long state_stride, const int* __restrict__ cu_q,
                   const int* __restrict__ state_slots, float* raw, int heads, int kvh, int dim, int vdim, long num_slots,
@@ -825,7 +829,8 @@ static int launch_delta_scan(const float* qkv, const void* ab, long ab_stride, i
   const int rows = dim <= 128 ? 16 : 32;
   const int lanes = dim <= rows ? 1 : (dim <= 2 * rows ? 2 : (dim <= 4 * rows ? 4 : 8));
   // Without AHEAD where more blocks than two an SM have up to eight tokens a request on average (decoding): 64 requests of one token, 16
-  // heads of 128 x 128: 59 us, 75 with; of four: 83 and 95; 16 of sixteen: 47 and 44.
+  // heads of 128 x 128: 59 us, 75 with; of four: 83 and 95; 16 of sixteen: 47 and 44.  (Where fewer blocks have one token each it is the slower
+  // one, two requests, 16 heads, a decay a row, one launch behind the other: 5.1 us, 4.3 with.)
   const long blocks = (long)((vdim + DS_COMPUTE / lanes - 1) / (DS_COMPUTE / lanes)) * heads * B;
   const bool ahead = blocks <= 2 * sm_count() || T_all > 8 * (long)B;
 #define VOB_DS_LAUNCH(L, R, D, A)                                                                                          \
