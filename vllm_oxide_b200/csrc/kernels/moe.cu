@@ -60,20 +60,22 @@ constexpr int ROUTE_MOST = 8, ROUTE_OF_WARP = 4;      // tokens a block and a wa
 
 // A block takes TOKENS tokens, whose rows lie in shared memory as they are; eight warps take up to four of them.  A warp takes two
 // experts at a time: every element of a row that it reads serves both, and the experts' rows, which come from L2 or from memory, are on
-// their way many pieces at once.  (2,048 x 16 experts, 40 tokens: 12 us timed alone, 16 with an
-// expert at a time; 500: 13, 17; 1,333: 17, 20; 2,048: 27, 25; 4,096 x 16, 4,001 tokens: 64, 80.)
-template <int TOKENS> struct RouteShape {
+// their way many pieces at once.  (2,048 x 16 experts, 40 tokens: 12 us timed alone, 18 with an
+// expert at a time; 500: 14, 18; 1,333: 18, 20; 2,048: 20, 25; 4,096 x 16, 4,001 tokens: 53, 81.)
+// DENSE: four blocks of four tokens an SM instead of three, with 64 registers a thread; a round takes a little longer (2,048 x 16, 1,333 tokens
+// of bfloat16 18.4 us and 18.4; x 64 43 and 39).
+template <int TOKENS, bool DENSE> struct RouteShape {
   static constexpr int OWN = TOKENS < ROUTE_OF_WARP ? TOKENS : ROUTE_OF_WARP, GROUPS = TOKENS / OWN, THREADS = ROUTE_NT * GROUPS;
-  static constexpr int BLOCKS = TOKENS == 4 ? 3 : (TOKENS < 4 ? 2 : 1);      // an SM: with one fewer, 1,333 or 200 tokens take a second round
+  static constexpr int BLOCKS = DENSE ? 4 : (TOKENS == 4 ? 3 : (TOKENS < 4 ? 2 : 1));      // an SM
 };
 
-template <typename T, int TOKENS>
-__global__ void __launch_bounds__(RouteShape<TOKENS>::THREADS, RouteShape<TOKENS>::BLOCKS)
+template <typename T, int TOKENS, bool DENSE>
+__global__ void __launch_bounds__(RouteShape<TOKENS, DENSE>::THREADS, RouteShape<TOKENS, DENSE>::BLOCKS)
 moe_route_kernel(const T* h, const float* __restrict__ w_router, const float* __restrict__ router_bias,
                  const float* __restrict__ correction, const float* __restrict__ w_shared, float* shared_gate, int* ids, float* weights,
                  int W, int E, int top, int count, int keep, int sigmoid_scores, int group_top, int normalise, float weight_scale,
                  int num_tokens, int vec, int wide) {
-  constexpr int OWN = RouteShape<TOKENS>::OWN, NT = RouteShape<TOKENS>::THREADS, WARPS = ROUTE_NT / 32;
+  constexpr int OWN = RouteShape<TOKENS, DENSE>::OWN, NT = RouteShape<TOKENS, DENSE>::THREADS, WARPS = ROUTE_NT / 32;
   extern __shared__ __align__(16) float route_smem[];
   const int list = 2 * E + count + 1, logits = E + (w_shared ? 1 : 0);
   float* lists = route_smem;                        // per token: [E] scores, [E] choice scores, [count] group scores, [1] shared gate
@@ -663,30 +665,38 @@ VOB_API int vob_moe_route(const void* h, const float* w_router, const float* rou
   if ((w_shared == nullptr) != (shared_gate == nullptr)) return VOB_BAD_ARGUMENT;
   if (E <= 0 || top <= 0 || top > E || count <= 0 || E % count || keep <= 0 || keep > count || (long)(E / count) * keep < top)
     return VOB_BAD_ARGUMENT;
-  // as many tokens a block (1, 2, 4, 8) as leave every SM a block and as 96 KB hold; one where rows start on no boundary of four
-  // elements.  A token's arithmetic does not depend on how many share its block.
+  // as many tokens a block (1, 2, 4) as leave every SM a block and as 96 KB hold; one where rows start on no boundary of four elements.
+  // Eight where the router's rows are long and one round takes all tokens (4,096 x 16, 592 to 1,184 tokens: 21 to 22 us, 23 to 25 by four; 1,333,
+  // in two rounds: 35 and 25).  A token's arithmetic does not depend on how many share its block.
   const size_t size = dtype == VOB_BF16 ? 2 : 4;
   const int vec = W % 4 == 0 && (((uintptr_t)w_router | (uintptr_t)w_shared) % 16) == 0, wide = vec && (uintptr_t)h % (4 * size) == 0;
   auto bytes = [&](int tokens) { return (size_t)(tokens * (2 * E + count + 1) + 3) / 4 * 16 + (size_t)tokens * W * size; };
-  int tokens = vec ? (W >= 4096 ? ROUTE_MOST : ROUTE_OF_WARP) : 1;      // (at a width of 2,048, 1,333 tokens: 27 us with eight)
+  int tokens = vec ? ROUTE_OF_WARP : 1;
   while (tokens > 1 && (T < (long)tokens * sm_count() || bytes(tokens) > 96 * 1024)) tokens /= 2;
+  if (tokens == ROUTE_OF_WARP && dtype == VOB_BF16 && W >= 4096 && T <= (long)ROUTE_MOST * sm_count() && bytes(ROUTE_MOST) <= 96 * 1024)
+    tokens = ROUTE_MOST;
   const size_t smem = bytes(tokens);
+  // the dense form where that saves a round (rows of bfloat16, which fit its registers): 2,048 x 16, 2,048 tokens 20 us, 29 in two rounds;
+  // x 64 47 and 64; 4,096 x 16 29 and 39
+  auto rounds = [&](int an_sm) { return ((T + tokens - 1) / tokens + an_sm * sm_count() - 1) / (an_sm * sm_count()); };
+  const bool dense = tokens == ROUTE_OF_WARP && dtype == VOB_BF16 && 4 * (smem + 1024) <= 227 * 1024 && rounds(4) < rounds(3);
   if (smem > 200 * 1024) return VOB_UNSUPPORTED;
-#define VOB_ROUTE_N(TYPE, N)                                                                                             \
+#define VOB_ROUTE_N(TYPE, N, D)                                                                                          \
   do {                                                                                                                   \
     if (smem > 48 * 1024)                                                                                                \
-      cudaFuncSetAttribute(moe_route_kernel<TYPE, N>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);           \
-    return launch_kernel(moe_route_kernel<TYPE, N>, dim3((T + N - 1) / N), RouteShape<N>::THREADS, smem, stream, (const TYPE*)h, w_router, router_bias, \
-                         correction, w_shared, shared_gate, ids, weights, W, E, top, count, keep, sigmoid_scores, group_top, normalise,   \
-                         weight_scale, T, vec, wide);                                                                      \
+      cudaFuncSetAttribute(moe_route_kernel<TYPE, N, D>, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);        \
+    return launch_kernel(moe_route_kernel<TYPE, N, D>, dim3((T + N - 1) / N), (RouteShape<N, D>::THREADS), smem, stream, (const TYPE*)h, w_router, \
+                         router_bias, correction, w_shared, shared_gate, ids, weights, W, E, top, count, keep, sigmoid_scores, group_top, \
+                         normalise, weight_scale, T, vec, wide);                                                         \
   } while (0)
-#define VOB_ROUTE(TYPE)                    \
-  do {                                     \
-    if (tokens == 8) VOB_ROUTE_N(TYPE, 8); \
-    if (tokens == 4) VOB_ROUTE_N(TYPE, 4); \
-    if (tokens == 2) VOB_ROUTE_N(TYPE, 2); \
-    VOB_ROUTE_N(TYPE, 1);                  \
+#define VOB_ROUTE(TYPE)                           \
+  do {                                            \
+    if (tokens == 4) VOB_ROUTE_N(TYPE, 4, false); \
+    if (tokens == 2) VOB_ROUTE_N(TYPE, 2, false); \
+    VOB_ROUTE_N(TYPE, 1, false);                  \
   } while (0)
+  if (tokens == ROUTE_MOST) VOB_ROUTE_N(__nv_bfloat16, ROUTE_MOST, false);
+  if (dense) VOB_ROUTE_N(__nv_bfloat16, ROUTE_OF_WARP, true);
   if (dtype == VOB_F32) VOB_ROUTE(float);
   if (dtype == VOB_BF16) VOB_ROUTE(__nv_bfloat16);
 #undef VOB_ROUTE
