@@ -557,9 +557,11 @@ constexpr int DI_MERGE_FLOATS(int G) { return 2 * DEC_WARPS * 16 + DEC_WARPS * G
 constexpr int DI_DRAW_AHEAD = 2;                          // tiles before a pair's last at which the next pair is drawn
 constexpr int DI_QUEUE = 8;                               // entries; the producer is at most DT_STAGES + 1 pairs ahead
 // Pairs are given out with the longest requests first, so that the last to end are short ones: every block sorts up to DI_ORDERED
-// requests by their tiles (in 256 steps; equal ones stay in the batch's order, so every block finds the same), before the kernels ahead are done.
-// (224 requests of 40 to 1,152 keys, 8 x 2 heads of 128, and five portions: with the late start 136 us a layer, 143 without either.)
-constexpr int DI_ORDERED = 1024, DI_BUCKETS = 256;
+// requests by their tiles (in 256 steps; equal ones stay in the batch's order, so every block finds the same), before the kernels ahead are done:
+// all threads count, one warp places.  Up to DI_ORDERED_PAIRS pairs a block: with more of them the blocks end together anyway.  (Decoding alone, cold
+// L2, 8 x 2 heads of 128, 40 to 1,152 keys, 64, 128 and 224 requests: 49, 74 and 113 us, 55, 80 and 119 in the batch's order; 50 to 80 keys,
+// which are in order as they are, 224: 41 and 39; 500 and 1,000, not sorted: 225 and 395, 228 and 411 sorted.)
+constexpr int DI_ORDERED = 1024, DI_ORDERED_PAIRS = 8, DI_BUCKETS = 256;
 // (from seven heads a key head on the sums' buffers leave no room for it beside a second block)
 constexpr int DI_ORDER_BYTES(int G) { return G <= 6 ? DI_BUCKETS * 4 + DI_ORDERED * 2 : 0; }
 
@@ -583,23 +585,53 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
   uint64_t* full = reinterpret_cast<uint64_t*>(queue + DI_QUEUE);
   uint64_t* empty = full + DT_STAGES;
   volatile int* abort_flag = reinterpret_cast<volatile int*>(empty + DT_STAGES);
-  int* bucket_at = const_cast<int*>(reinterpret_cast<volatile int*>(abort_flag)) + 2;       // [DI_BUCKETS]
+  int* sorted = const_cast<int*>(reinterpret_cast<volatile int*>(abort_flag)) + 1;           // whether pairs are given out by `order`
+  int* bucket_at = sorted + 1;                                                              // [DI_BUCKETS]
   uint16_t* order = reinterpret_cast<uint16_t*>(bucket_at + DI_BUCKETS);                    // [num_requests], up to DI_ORDERED
-  const bool ordered = num_requests <= DI_ORDERED && DI_ORDER_BYTES(G) > 0;
+  const bool ordered = num_requests <= DI_ORDERED && num_requests * kvh <= DI_ORDERED_PAIRS * (int)gridDim.x && DI_ORDER_BYTES(G) > 0;
   pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  if (ordered && warp == 0) {
-    for (int i = lane; i < DI_BUCKETS; i += 32) bucket_at[i] = 0;
-    __syncwarp();
-    for (int pass = 0; pass < 2; ++pass) {           // how many a bucket has, then where each goes
-      for (int b0 = 0; b0 < num_requests; b0 += 32) {
-        const int b = b0 + lane;
-        int bucket = -1;
-        if (b < num_requests) {
-          const int pos = context_lens[b] - 1, start = first_key(pos, window, ep) & ~(box_keys - 1);
-          const int tiles = cu_q[b + 1] - cu_q[b] == 1 ? (pos + 1 - start + DEC_TILE - 1) / DEC_TILE : 0;
-          bucket = DI_BUCKETS - 1 - max(0, min(DI_BUCKETS - 1, tiles));
+  if (ordered) {
+    uint8_t* bucket_of = reinterpret_cast<uint8_t*>(wm);      // [num_requests], where the sums will lie
+    for (int i = threadIdx.x; i < DI_BUCKETS; i += DT_THREADS) bucket_at[i] = 0;
+    __syncthreads();
+#pragma unroll 4
+    for (int b = threadIdx.x; b < num_requests; b += DT_THREADS) {      // how many a bucket has
+      const int pos = context_lens[b] - 1, start = first_key(pos, window, ep) & ~(box_keys - 1);
+      const int tiles = cu_q[b + 1] - cu_q[b] == 1 ? (pos + 1 - start + DEC_TILE - 1) / DEC_TILE : 0;
+      const int bucket = DI_BUCKETS - 1 - max(0, min(DI_BUCKETS - 1, tiles));
+      bucket_of[b] = (uint8_t)bucket;
+      atomicAdd(&bucket_at[bucket], 1);
+    }
+    __syncthreads();
+    if (warp == 0) {
+      int mine[DI_BUCKETS / 32], sum = 0;
+#pragma unroll
+      for (int i = 0; i < DI_BUCKETS / 32; ++i) { mine[i] = sum; sum += bucket_at[lane * (DI_BUCKETS / 32) + i]; }
+      int before = sum;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int v = __shfl_up_sync(0xffffffffu, before, d);
+        if (lane >= d) before += v;
+      }
+      before -= sum;
+      // (lengths within two tiles of one another: any order does, and the batch's costs nothing)
+      int few = DI_BUCKETS, many = -1;
+#pragma unroll
+      for (int i = 0; i < DI_BUCKETS / 32; ++i)
+        if ((i + 1 < DI_BUCKETS / 32 ? mine[i + 1] : sum) > mine[i]) {
+          few = min(few, lane * (DI_BUCKETS / 32) + i);
+          many = lane * (DI_BUCKETS / 32) + i;
         }
+      const bool uneven = __reduce_max_sync(0xffffffffu, many) > __reduce_min_sync(0xffffffffu, few) + 1;
+      if (lane == 0) *sorted = uneven;
+      __syncwarp();
+#pragma unroll
+      for (int i = 0; i < DI_BUCKETS / 32; ++i) bucket_at[lane * (DI_BUCKETS / 32) + i] = before + mine[i];
+      __syncwarp();
+#pragma unroll 2
+      for (int b0 = 0; b0 < (uneven ? num_requests : 0); b0 += 32) {    // then where each goes
+        const int b = b0 + lane, bucket = b < num_requests ? bucket_of[b] : -1;
         const unsigned same = __match_any_sync(0xffffffffu, bucket);
         const int rank = __popc(same & ((1u << lane) - 1)), at = bucket >= 0 ? bucket_at[bucket] : 0;
         __syncwarp();
@@ -636,6 +668,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
   asm volatile("fence.mbarrier_init.release.cluster;\n" ::: "memory");
   asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
   __syncthreads();
+  const bool by_order = ordered && *sorted;
   const int num_items = num_requests * kvh;
 
   if (warp == DEC_WARPS) {
@@ -650,7 +683,7 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
       // yet draws after its tiles: the counter is this launch's only after the launches before it are done).
       int next = -1;
       bool drawn = false;
-      const int b = ordered ? order[item / kvh] : item / kvh, kh = item % kvh;
+      const int b = by_order ? order[item / kvh] : item / kvh, kh = item % kvh;
       const int t = cu_q[b];
       if (cu_q[b + 1] - t == 1) {                     // a decoding request (the others are the prefill kernel's)
         const int pos = context_lens[b] - 1;
