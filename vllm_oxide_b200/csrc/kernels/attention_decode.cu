@@ -981,10 +981,24 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
       if (e != cudaSuccess) return (int)e;
       tma_configured[late][form] = true;
     }
+  }
+#if VOB_HD == 192
+  // Clusters of splits that the GPU does not hold at once take a second round; with kept keys or a bias the cp.async kernel, whose blocks go
+  // anywhere, is then the faster one (24 requests of 600 keys, 4 heads, 3 splits: 28 us, 33 by this one), and in all other cases the
+  // slower one (8 of 2,000, 8 heads, 3 splits: 50 and 37; 40 of 600, 1 head, 4 splits: 24 and 21; 40 of 1,088, 8 heads, one split: 115 and 81).
+  if (by_tma && extras && num_splits > 1 && num_splits <= 8 && g_decode_cluster_merge && scratch) {
+    static int resident_of[2][2][9] = {};      // clusters that fit the GPU at once, plus one (0: not asked yet)
+    int& resident = resident_of[late][shared][num_splits];
+    if (!resident) resident = 1 + resident_clusters(kernel, DT_THREADS, tma_smem, (unsigned)num_splits);
+    by_tma = (long)kvh * num_requests < resident;
+  }
+#endif
+  if (by_tma) {
     const int box_keys = block_size % DEC_TILE == 0 ? DEC_TILE : RUN_KEYS;
     // one split and more (request, kv head) pairs than blocks fit the GPU: persistent blocks, the producer ahead across pairs (they
-    // walk one range of keys and know no bias)
-    if (num_splits == 1 && pairs_counter && !extras) {
+    // walk one range of keys, know no bias and bring a plane that is both keys and values in twice: 150, 296 and 600 requests of 700 to
+    // 2,100 keys, a latent of 256, 16 heads: 96, 125 and 217 us, 76, 82 and 150 by a block a pair)
+    if (num_splits == 1 && pairs_counter && !extras && !shared) {
       const int G = nh / kvh;
       const int items_smem = 1024 + DT_STAGES * DT_STAGE_BYTES + DI_MERGE_FLOATS(G) * 4 + DI_QUEUE * 16 + 2 * DT_STAGES * 8 + 32 + DI_ORDER_BYTES(G);
       auto items_kernel = late ? attention_decode_tma_items_kernel<true> : attention_decode_tma_items_kernel<false>;
