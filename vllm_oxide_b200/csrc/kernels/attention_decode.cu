@@ -637,24 +637,8 @@ attention_decode_tma_items_kernel(const __grid_constant__ CUtensorMap tmK, const
         __syncwarp();
         if (bucket >= 0) {
           if (rank == 0) bucket_at[bucket] = at + __popc(same);
-          if (pass) order[at + rank] = (uint16_t)b;
+          order[at + rank] = (uint16_t)b;
         }
-        __syncwarp();
-      }
-      if (pass == 0) {
-        int mine[DI_BUCKETS / 32], sum = 0;
-#pragma unroll
-        for (int i = 0; i < DI_BUCKETS / 32; ++i) { mine[i] = sum; sum += bucket_at[lane * (DI_BUCKETS / 32) + i]; }
-        int before = sum;
-#pragma unroll
-        for (int d = 1; d < 32; d <<= 1) {
-          const int v = __shfl_up_sync(0xffffffffu, before, d);
-          if (lane >= d) before += v;
-        }
-        before -= sum;
-        __syncwarp();
-#pragma unroll
-        for (int i = 0; i < DI_BUCKETS / 32; ++i) bucket_at[lane * (DI_BUCKETS / 32) + i] = before + mine[i];
         __syncwarp();
       }
     }
@@ -952,30 +936,27 @@ static int attention_decode_launch(const void* map_k, const void* map_v, const v
   int rc;
 #if VOB_HD % 64 == 0
   const int extras = ep.keep_first || ep.dist_bias;
-  // Heads of 192 left one block of this kernel on an SM when this was measured (since then two: DecodeShape), two of the cp.async kernel, which
-  // answers these calls where there are more blocks than SMs (24 requests of 600 keys, 4 heads, 3 splits: 21 us, 29 here; 40, 1 head, 4 splits: 23 and 30; 8 requests, 4
-  // splits, fit: 14 and 9).
-  const bool second_places = HD == 192 && extras && (long)num_splits * kvh * num_requests > sm_count() && (num_splits == 1 || scratch);
-  if (map_k && map_v && block_size % 16 == 0 && !second_places) {
-    // one plane for keys and values: a map of either, no head offset between them
-    const bool shared = HD >= 192 && kcache == vcache && ep.value_div == 1;
-    const bool dense = HD == 128 && extras && (long)num_splits * kvh * num_requests > 2 * sm_count();
-    const int form = extras + 2 * shared + 4 * dense;
-    static bool tma_configured[2][8] = {};
-    auto kernel = late ? attention_decode_tma_kernel<false, false, false, true> : attention_decode_tma_kernel<false, false, false, false>;
-    int tma_smem = DecodeShape<false, false, false>::SMEM;
+  // one plane for keys and values: a map of either, no head offset between them
+  const bool shared = HD >= 192 && kcache == vcache && ep.value_div == 1;
+  const bool dense = HD == 128 && extras && (long)num_splits * kvh * num_requests > 2 * sm_count();
+  const int form = extras + 2 * shared + 4 * dense;
+  auto kernel = late ? attention_decode_tma_kernel<false, false, false, true> : attention_decode_tma_kernel<false, false, false, false>;
+  int tma_smem = DecodeShape<false, false, false>::SMEM;
 #define VOB_FORM(X, S, D)                                                                                        \
   if (form == (X) + 2 * (S) + 4 * (D)) {                                                                         \
     kernel = late ? attention_decode_tma_kernel<X, S, D, true> : attention_decode_tma_kernel<X, S, D, false>;    \
     tma_smem = DecodeShape<X, S, D>::SMEM;                                                                       \
   }
-    VOB_FORM(true, false, false)
+  VOB_FORM(true, false, false)
 #if VOB_HD >= 192
-    VOB_FORM(false, true, false) VOB_FORM(true, true, false)
+  VOB_FORM(false, true, false) VOB_FORM(true, true, false)
 #elif VOB_HD == 128
-    VOB_FORM(true, false, true)
+  VOB_FORM(true, false, true)
 #endif
 #undef VOB_FORM
+  bool by_tma = map_k && map_v && block_size % 16 == 0;
+  if (by_tma) {
+    static bool tma_configured[2][8] = {};
     if (!tma_configured[late][form]) {
       cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, tma_smem);
       if (e != cudaSuccess) return (int)e;
