@@ -326,57 +326,57 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
         for (unsigned c = 0; c < n; ++c) reach += cand_key[c] >= mine;
       thr = block_max_u32((unsigned)tid < n && reach >= (unsigned)k ? mine : 0u, scratch);
     } else {
-    if (tid == 0) { s_prefix = 0; s_remaining_k = (unsigned)k; s_gather = 0; }
-    for (int pass = 0; pass < 4; ++pass) {
-      const int shift = 24 - 8 * pass;
-      if (tid < 256) hist[tid] = 0;
-      __syncthreads();
-      const uint32_t prefix = s_prefix;
-      const uint32_t mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
-      if (gathered) {
-        const unsigned ncand = s_ncand;
-        for (unsigned c = tid; c < ncand; c += SAMPLE_THREADS) {
-          const uint32_t key = cand_key[c];
-          if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        }
-      } else {
-        each_logit(l, V, 0, 1, [&](float x, int) {
-          const uint32_t key = ordered_key(x * inv_t);
-          if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
-        });
-      }
-      __syncthreads();
-      if (tid < 32) {
-        const unsigned need = s_remaining_k;
-        int b;
-        unsigned cum;
-        find_bin(hist, need, b, cum);
-        if (tid == 0) {
-          s_remaining_k = need - cum;
-          s_prefix = prefix | ((uint32_t)b << shift);
-          if (pass == 0 && !gathered && cum + hist[b] <= (unsigned)SAMPLE_CANDIDATES) { s_gather = 1; s_ncand = 0; }
-        }
-      }
-      __syncthreads();
-      if (pass == 0 && s_gather) {
-        const uint32_t first = s_prefix >> 24;
-        each_logit(l, V, 0, 1, [&](float x, int i) {
-          const uint32_t key = ordered_key(x * inv_t);
-          if ((key >> 24) >= first) {
-            const unsigned pos = atomicAdd(&s_ncand, 1u);
-            cand_key[pos] = key; cand_idx[pos] = (uint32_t)i;
-          }
-        });
-        gathered = true;
+      if (tid == 0) { s_prefix = 0; s_remaining_k = (unsigned)k; s_gather = 0; }
+      for (int pass = 0; pass < 4; ++pass) {
+        const int shift = 24 - 8 * pass;
+        if (tid < 256) hist[tid] = 0;
         __syncthreads();
+        const uint32_t prefix = s_prefix;
+        const uint32_t mask = pass == 0 ? 0u : (0xFFFFFFFFu << (shift + 8));
+        if (gathered) {
+          const unsigned ncand = s_ncand;
+          for (unsigned c = tid; c < ncand; c += SAMPLE_THREADS) {
+            const uint32_t key = cand_key[c];
+            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+          }
+        } else {
+          each_logit(l, V, 0, 1, [&](float x, int) {
+            const uint32_t key = ordered_key(x * inv_t);
+            if ((key & mask) == prefix) atomicAdd(&hist[(key >> shift) & 255u], 1u);
+          });
+        }
+        __syncthreads();
+        if (tid < 32) {
+          const unsigned need = s_remaining_k;
+          int b;
+          unsigned cum;
+          find_bin(hist, need, b, cum);
+          if (tid == 0) {
+            s_remaining_k = need - cum;
+            s_prefix = prefix | ((uint32_t)b << shift);
+            if (pass == 0 && !gathered && cum + hist[b] <= (unsigned)SAMPLE_CANDIDATES) { s_gather = 1; s_ncand = 0; }
+          }
+        }
+        __syncthreads();
+        if (pass == 0 && s_gather) {
+          const uint32_t first = s_prefix >> 24;
+          each_logit(l, V, 0, 1, [&](float x, int i) {
+            const uint32_t key = ordered_key(x * inv_t);
+            if ((key >> 24) >= first) {
+              const unsigned pos = atomicAdd(&s_ncand, 1u);
+              cand_key[pos] = key; cand_idx[pos] = (uint32_t)i;
+            }
+          });
+          gathered = true;
+          __syncthreads();
+        }
       }
-    }
-    thr = s_prefix;
+      thr = s_prefix;
     }
   }
 
   // the blocks that are still here share the row: all of them without a top-k, else the first alone
-  const int of = k >= 1 && k < V ? 1 : parts, now = rank;
+  const int of = k >= 1 && k < V ? 1 : parts;
   // ---- maximum of the scaled logits (always a survivor)
   unsigned long long best = 0;
   if (gathered) {
@@ -386,7 +386,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       best = cnd > best ? cnd : best;
     }
   } else {
-    each_logit(l, V, now, of, [&](float x, int i) {
+    each_logit(l, V, rank, of, [&](float x, int i) {
       const unsigned long long c = pack_candidate(x * inv_t, i);
       best = c > best ? c : best;
     });
@@ -405,7 +405,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
         z += m;
       }
     } else {
-      each_logit(l, V, now, of, [&](float raw, int) {
+      each_logit(l, V, rank, of, [&](float raw, int) {
         const float x = raw * inv_t;
         if (ordered_key(x) >= thr) z += fixed_mass(x, maxv);
       });
@@ -434,7 +434,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
     if (!gathered) {
       const unsigned long long floor_mass = (unsigned long long)((1.0 - (double)p) * (double)total / (double)V);
       if (floor_mass >= 1) {
-        each_logit(l, V, now, of, [&](float raw, int i) {
+        each_logit(l, V, rank, of, [&](float raw, int i) {
           const float x = raw * inv_t;
           const uint32_t key = ordered_key(x);
           if (key < thr) return;
@@ -509,7 +509,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
           if ((key & mask) == prefix) atomicAdd(&bins[(key >> shift) & 255u], cand_mass[i]);
         }
       } else {
-        each_logit_together(l, V, now, of, [&](float raw, int, bool there) {
+        each_logit_together(l, V, rank, of, [&](float raw, int, bool there) {
           const float x = there ? raw * inv_t : 0.f;
           const uint32_t key = ordered_key(x);
           const bool in = there && key >= thr && (key & mask) == prefix;
@@ -559,7 +559,7 @@ sample_kernel(const float* logits, long ld, int V, const float* __restrict__ tem
       best = cnd > best ? cnd : best;
     }
   } else
-  each_logit(l, V, now, drawing, [&](float raw, int i) {
+  each_logit(l, V, rank, drawing, [&](float raw, int i) {
     const float x = raw * inv_t;
     if (ordered_key(x) < thr) return;
     const float u = counter_uniform(key_row, (uint32_t)i);
